@@ -5,9 +5,9 @@ outward corner area normals B (geometry.cpp:40-234), exact volume
 Every expression keeps the reference's operands and association order, so the
 generated code is bit-for-bit equivalent to it when compiled without
 contraction.  The work is shared where that is exact:
-  * each cofactor combo is evaluated once per unordered node pair; the other
-    orientation is its exact negation (term-by-term negated sums round to the
-    negated value);
+  * each cofactor combo is evaluated once for all the node pairs it belongs to;
+    the other orientation, and the pairs whose terms are the negated ones, are
+    its exact negation (term-by-term negated sums round to the negated value);
   * the volume reuses the B-matrix products y_j * comb_ij of component 0.
 The volume's products and sums (and with them component 0 of B) go through
 FX_MUL / FX_ADD, which stay separately rounded in the fused-multiply-add build
@@ -39,6 +39,49 @@ def parse_tables():
     T = [[T[(p * 6 + t) * 4:(p * 6 + t + 1) * 4] for t in range(6)] for p in range(8)]
     VJ = [VJ[a * 6:(a + 1) * 6] for a in range(8)]
     return J, T, VI, VJ
+
+
+def combo_expr(I, terms):
+    """The combo's signed terms summed left to right, as the reference writes them."""
+    expr = ("-" if terms[0] < 0 else "") + "%s[%d]" % (I, abs(terms[0]) - 1)
+    for v_ in terms[1:]:
+        expr = "(%s %s %s[%d])" % (expr, "+" if v_ > 0 else "-", I, abs(v_) - 1)
+    return expr
+
+
+def emit_combos(w, I, pairs, T, indent="    "):
+    """Declares the combos the pairs need and returns pair index -> signed name.
+    A combo equal to an earlier one or to its term-by-term negation is that one
+    (the compiler does not see that (-a - b) + c + d is -((a + b) - c - d)), and
+    a four-term combo whose first two terms are a two-term combo starts from it:
+    12 + 16 additions per component instead of the 40 left of 48 when each pair
+    forms its own."""
+    seen, name_of = {}, {}
+    order = sorted(range(len(pairs)), key=lambda k: len([v for v in T[pairs[k][0]][pairs[k][1]] if v]))
+    for k in order:
+        p, t, j = pairs[k]
+        terms = tuple(v for v in T[p][t] if v)
+        neg = tuple(-v for v in terms)
+        if terms in seen:
+            name_of[k] = seen[terms]
+            continue
+        if neg in seen:
+            name_of[k] = "(-%s)" % seen[neg]
+            continue
+        head, neg_head = terms[:2], neg[:2]
+        expr = combo_expr(I, terms)
+        if len(terms) == 4 and (head in seen or neg_head in seen):
+            expr = seen[head] if head in seen else "(-%s)" % seen[neg_head]
+            for v_ in terms[2:]:
+                expr = "(%s %s %s[%d])" % (expr, "+" if v_ > 0 else "-", I, abs(v_) - 1)
+        w("%sconst double cm%d = %s;  // pair (%d,%d)" % (indent, k, expr, p, j))
+        seen[terms] = "cm%d" % k
+        name_of[k] = "cm%d" % k
+    return name_of
+
+
+def negated(name):
+    return name[2:-1] if name.startswith("(-") else "(-%s)" % name
 
 
 def main():
@@ -86,20 +129,12 @@ def main():
     vel = {0: "u", 1: "v", 2: "w"}
     for c, (O, I) in enumerate(comps):
         w("  {  // component %d: O = %s, I = %s" % (c, O, I))
-        for k, (p, t, j) in enumerate(pairs):
-            terms = [v for v in T[p][t] if v]
-            expr = ("-" if terms[0] < 0 else "") + "%s[%d]" % (I, abs(terms[0]) - 1)
-            for v_ in terms[1:]:
-                expr = "(%s %s %s[%d])" % (expr, "+" if v_ > 0 else "-", I, abs(v_) - 1)
-            w("    const double cm%d = %s;  // pair (%d,%d)" % (k, expr, p, j))
+        combo = emit_combos(w, I, pairs, T)
         # products
         for p in range(8):
             for t in range(6):
                 j = J[p][t]
-                if p < j:
-                    cm = "cm%d" % pair_of[(p, j)]
-                else:
-                    cm = "(-cm%d)" % pair_of[(j, p)]
+                cm = combo[pair_of[(p, j)]] if p < j else negated(combo[pair_of[(j, p)]])
                 if c == 0:
                     w("    const double pr%d_%d = FX_MUL(%s[%d], %s);" % (p, t, O, j, cm))
                 else:
@@ -137,12 +172,7 @@ def main():
     w("    const double* __restrict__ z) {")
     w("  const double twelth = 1. / 12.;")
     O, I = comps[0]
-    for k, (p_, t, j) in enumerate(pairs):
-        terms = [v for v in T[p_][t] if v]
-        expr = ("-" if terms[0] < 0 else "") + "%s[%d]" % (I, abs(terms[0]) - 1)
-        for v_ in terms[1:]:
-            expr = "(%s %s %s[%d])" % (expr, "+" if v_ > 0 else "-", I, abs(v_) - 1)
-        w("  const double cm%d = %s;" % (k, expr))
+    combo = emit_combos(w, I, pairs, T, "  ")
     used = set()
     for a in range(8):
         i = VI[a]
@@ -150,7 +180,7 @@ def main():
             used.add((i, J[i].index(jj)))
     for (p_, t) in sorted(used):
         j = J[p_][t]
-        cm = ("cm%d" % pair_of[(p_, j)]) if p_ < j else ("(-cm%d)" % pair_of[(j, p_)])
+        cm = combo[pair_of[(p_, j)]] if p_ < j else negated(combo[pair_of[(j, p_)]])
         w("  const double pr%d_%d = %s[%d] * %s;" % (p_, t, O, j, cm))
     for a in range(8):
         i = VI[a]
@@ -182,9 +212,7 @@ def main():
             w("    const double g%d = Bbar[%d] * twelth;" % (p_, p_ * 3 + c))
         for k, (p_, t, j) in enumerate(pairs):
             terms = [v for v in T[p_][t] if v]
-            expr = ("-" if terms[0] < 0 else "") + "%s[%d]" % (I, abs(terms[0]) - 1)
-            for v_ in terms[1:]:
-                expr = "(%s %s %s[%d])" % (expr, "+" if v_ > 0 else "-", I, abs(v_) - 1)
+            expr = combo_expr(I, terms)
             w("    {  // pair (%d,%d)" % (p_, j))
             w("      const double cm = %s;" % expr)
             w("      %s[%d] = fma(g%d, cm, %s[%d]);" % (bar[O], j, p_, bar[O], j))

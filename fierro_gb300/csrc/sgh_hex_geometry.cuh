@@ -19,30 +19,24 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     double& Sx, double& Sy, double& Sz) {
   const double twelth = 1. / 12.;
   {  // component 0: O = y, I = z
-    const double cm0 = (((-z[2] - z[3]) + z[4]) + z[5]);  // pair (0,1)
     const double cm1 = (z[1] - z[3]);  // pair (0,2)
-    const double cm2 = (((z[1] + z[2]) - z[4]) - z[7]);  // pair (0,3)
-    const double cm3 = (((-z[1] + z[3]) - z[5]) + z[7]);  // pair (0,4)
     const double cm4 = (-z[1] + z[4]);  // pair (0,5)
     const double cm5 = (z[3] - z[4]);  // pair (0,7)
-    const double cm6 = (((-z[0] - z[3]) + z[5]) + z[6]);  // pair (1,2)
     const double cm7 = (-z[0] + z[2]);  // pair (1,3)
     const double cm8 = (z[0] - z[5]);  // pair (1,4)
-    const double cm9 = (((z[0] - z[2]) + z[4]) - z[6]);  // pair (1,5)
     const double cm10 = (-z[2] + z[5]);  // pair (1,6)
-    const double cm11 = (((-z[0] - z[1]) + z[6]) + z[7]);  // pair (2,3)
     const double cm12 = (z[1] - z[6]);  // pair (2,5)
-    const double cm13 = (((z[1] - z[3]) + z[5]) - z[7]);  // pair (2,6)
     const double cm14 = (-z[3] + z[6]);  // pair (2,7)
     const double cm15 = (-z[0] + z[7]);  // pair (3,4)
     const double cm16 = (z[2] - z[7]);  // pair (3,6)
-    const double cm17 = (((-z[0] + z[2]) - z[4]) + z[6]);  // pair (3,7)
-    const double cm18 = (((-z[0] - z[1]) + z[6]) + z[7]);  // pair (4,5)
     const double cm19 = (-z[5] + z[7]);  // pair (4,6)
-    const double cm20 = (((z[0] + z[3]) - z[5]) - z[6]);  // pair (4,7)
-    const double cm21 = (((-z[1] - z[2]) + z[4]) + z[7]);  // pair (5,6)
     const double cm22 = (z[4] - z[6]);  // pair (5,7)
-    const double cm23 = (((-z[2] - z[3]) + z[4]) + z[5]);  // pair (6,7)
+    const double cm0 = (((-z[2] - z[3]) + z[4]) + z[5]);  // pair (0,1)
+    const double cm2 = (((z[1] + z[2]) - z[4]) - z[7]);  // pair (0,3)
+    const double cm3 = (((-cm1) - z[5]) + z[7]);  // pair (0,4)
+    const double cm6 = (((-z[0] - z[3]) + z[5]) + z[6]);  // pair (1,2)
+    const double cm9 = (((-cm7) + z[4]) - z[6]);  // pair (1,5)
+    const double cm11 = (((-z[0] - z[1]) + z[6]) + z[7]);  // pair (2,3)
     const double pr0_0 = FX_MUL(y[1], cm0);
     const double pr0_1 = FX_MUL(y[2], cm1);
     const double pr0_2 = FX_MUL(y[3], cm2);
@@ -59,38 +53,38 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     const double pr2_1 = FX_MUL(y[1], (-cm6));
     const double pr2_2 = FX_MUL(y[3], cm11);
     const double pr2_3 = FX_MUL(y[5], cm12);
-    const double pr2_4 = FX_MUL(y[6], cm13);
+    const double pr2_4 = FX_MUL(y[6], (-cm3));
     const double pr2_5 = FX_MUL(y[7], cm14);
     const double pr3_0 = FX_MUL(y[0], (-cm2));
     const double pr3_1 = FX_MUL(y[1], (-cm7));
     const double pr3_2 = FX_MUL(y[2], (-cm11));
     const double pr3_3 = FX_MUL(y[4], cm15);
     const double pr3_4 = FX_MUL(y[6], cm16);
-    const double pr3_5 = FX_MUL(y[7], cm17);
+    const double pr3_5 = FX_MUL(y[7], (-cm9));
     const double pr4_0 = FX_MUL(y[0], (-cm3));
     const double pr4_1 = FX_MUL(y[1], (-cm8));
     const double pr4_2 = FX_MUL(y[3], (-cm15));
-    const double pr4_3 = FX_MUL(y[5], cm18);
+    const double pr4_3 = FX_MUL(y[5], cm11);
     const double pr4_4 = FX_MUL(y[6], cm19);
-    const double pr4_5 = FX_MUL(y[7], cm20);
+    const double pr4_5 = FX_MUL(y[7], (-cm6));
     const double pr5_0 = FX_MUL(y[0], (-cm4));
     const double pr5_1 = FX_MUL(y[1], (-cm9));
     const double pr5_2 = FX_MUL(y[2], (-cm12));
-    const double pr5_3 = FX_MUL(y[4], (-cm18));
-    const double pr5_4 = FX_MUL(y[6], cm21);
+    const double pr5_3 = FX_MUL(y[4], (-cm11));
+    const double pr5_4 = FX_MUL(y[6], (-cm2));
     const double pr5_5 = FX_MUL(y[7], cm22);
     const double pr6_0 = FX_MUL(y[1], (-cm10));
-    const double pr6_1 = FX_MUL(y[2], (-cm13));
+    const double pr6_1 = FX_MUL(y[2], cm3);
     const double pr6_2 = FX_MUL(y[3], (-cm16));
     const double pr6_3 = FX_MUL(y[4], (-cm19));
-    const double pr6_4 = FX_MUL(y[5], (-cm21));
-    const double pr6_5 = FX_MUL(y[7], cm23);
+    const double pr6_4 = FX_MUL(y[5], cm2);
+    const double pr6_5 = FX_MUL(y[7], cm0);
     const double pr7_0 = FX_MUL(y[0], (-cm5));
     const double pr7_1 = FX_MUL(y[2], (-cm14));
-    const double pr7_2 = FX_MUL(y[3], (-cm17));
-    const double pr7_3 = FX_MUL(y[4], (-cm20));
+    const double pr7_2 = FX_MUL(y[3], cm9);
+    const double pr7_3 = FX_MUL(y[4], cm6);
     const double pr7_4 = FX_MUL(y[5], (-cm22));
-    const double pr7_5 = FX_MUL(y[6], (-cm23));
+    const double pr7_5 = FX_MUL(y[6], (-cm0));
     const double vi0 = FX_MUL(x[1], FX_ADD(FX_ADD(FX_ADD(FX_ADD(FX_ADD(pr1_2, pr1_3), pr1_0), pr1_5), pr1_4), pr1_1));
     const double vi1 = FX_MUL(x[7], FX_ADD(FX_ADD(FX_ADD(FX_ADD(FX_ADD(pr7_0, pr7_5), pr7_1), pr7_2), pr7_4), pr7_3));
     const double vi2 = FX_MUL(x[3], FX_ADD(FX_ADD(FX_ADD(FX_ADD(FX_ADD(pr3_1, pr3_5), pr3_4), pr3_2), pr3_3), pr3_0));
@@ -126,30 +120,24 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     Sx = Sx + u[7] * b7;
   }
   {  // component 1: O = z, I = x
-    const double cm0 = (((-x[2] - x[3]) + x[4]) + x[5]);  // pair (0,1)
     const double cm1 = (x[1] - x[3]);  // pair (0,2)
-    const double cm2 = (((x[1] + x[2]) - x[4]) - x[7]);  // pair (0,3)
-    const double cm3 = (((-x[1] + x[3]) - x[5]) + x[7]);  // pair (0,4)
     const double cm4 = (-x[1] + x[4]);  // pair (0,5)
     const double cm5 = (x[3] - x[4]);  // pair (0,7)
-    const double cm6 = (((-x[0] - x[3]) + x[5]) + x[6]);  // pair (1,2)
     const double cm7 = (-x[0] + x[2]);  // pair (1,3)
     const double cm8 = (x[0] - x[5]);  // pair (1,4)
-    const double cm9 = (((x[0] - x[2]) + x[4]) - x[6]);  // pair (1,5)
     const double cm10 = (-x[2] + x[5]);  // pair (1,6)
-    const double cm11 = (((-x[0] - x[1]) + x[6]) + x[7]);  // pair (2,3)
     const double cm12 = (x[1] - x[6]);  // pair (2,5)
-    const double cm13 = (((x[1] - x[3]) + x[5]) - x[7]);  // pair (2,6)
     const double cm14 = (-x[3] + x[6]);  // pair (2,7)
     const double cm15 = (-x[0] + x[7]);  // pair (3,4)
     const double cm16 = (x[2] - x[7]);  // pair (3,6)
-    const double cm17 = (((-x[0] + x[2]) - x[4]) + x[6]);  // pair (3,7)
-    const double cm18 = (((-x[0] - x[1]) + x[6]) + x[7]);  // pair (4,5)
     const double cm19 = (-x[5] + x[7]);  // pair (4,6)
-    const double cm20 = (((x[0] + x[3]) - x[5]) - x[6]);  // pair (4,7)
-    const double cm21 = (((-x[1] - x[2]) + x[4]) + x[7]);  // pair (5,6)
     const double cm22 = (x[4] - x[6]);  // pair (5,7)
-    const double cm23 = (((-x[2] - x[3]) + x[4]) + x[5]);  // pair (6,7)
+    const double cm0 = (((-x[2] - x[3]) + x[4]) + x[5]);  // pair (0,1)
+    const double cm2 = (((x[1] + x[2]) - x[4]) - x[7]);  // pair (0,3)
+    const double cm3 = (((-cm1) - x[5]) + x[7]);  // pair (0,4)
+    const double cm6 = (((-x[0] - x[3]) + x[5]) + x[6]);  // pair (1,2)
+    const double cm9 = (((-cm7) + x[4]) - x[6]);  // pair (1,5)
+    const double cm11 = (((-x[0] - x[1]) + x[6]) + x[7]);  // pair (2,3)
     const double pr0_0 = z[1] * cm0;
     const double pr0_1 = z[2] * cm1;
     const double pr0_2 = z[3] * cm2;
@@ -166,38 +154,38 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     const double pr2_1 = z[1] * (-cm6);
     const double pr2_2 = z[3] * cm11;
     const double pr2_3 = z[5] * cm12;
-    const double pr2_4 = z[6] * cm13;
+    const double pr2_4 = z[6] * (-cm3);
     const double pr2_5 = z[7] * cm14;
     const double pr3_0 = z[0] * (-cm2);
     const double pr3_1 = z[1] * (-cm7);
     const double pr3_2 = z[2] * (-cm11);
     const double pr3_3 = z[4] * cm15;
     const double pr3_4 = z[6] * cm16;
-    const double pr3_5 = z[7] * cm17;
+    const double pr3_5 = z[7] * (-cm9);
     const double pr4_0 = z[0] * (-cm3);
     const double pr4_1 = z[1] * (-cm8);
     const double pr4_2 = z[3] * (-cm15);
-    const double pr4_3 = z[5] * cm18;
+    const double pr4_3 = z[5] * cm11;
     const double pr4_4 = z[6] * cm19;
-    const double pr4_5 = z[7] * cm20;
+    const double pr4_5 = z[7] * (-cm6);
     const double pr5_0 = z[0] * (-cm4);
     const double pr5_1 = z[1] * (-cm9);
     const double pr5_2 = z[2] * (-cm12);
-    const double pr5_3 = z[4] * (-cm18);
-    const double pr5_4 = z[6] * cm21;
+    const double pr5_3 = z[4] * (-cm11);
+    const double pr5_4 = z[6] * (-cm2);
     const double pr5_5 = z[7] * cm22;
     const double pr6_0 = z[1] * (-cm10);
-    const double pr6_1 = z[2] * (-cm13);
+    const double pr6_1 = z[2] * cm3;
     const double pr6_2 = z[3] * (-cm16);
     const double pr6_3 = z[4] * (-cm19);
-    const double pr6_4 = z[5] * (-cm21);
-    const double pr6_5 = z[7] * cm23;
+    const double pr6_4 = z[5] * cm2;
+    const double pr6_5 = z[7] * cm0;
     const double pr7_0 = z[0] * (-cm5);
     const double pr7_1 = z[2] * (-cm14);
-    const double pr7_2 = z[3] * (-cm17);
-    const double pr7_3 = z[4] * (-cm20);
+    const double pr7_2 = z[3] * cm9;
+    const double pr7_3 = z[4] * cm6;
     const double pr7_4 = z[5] * (-cm22);
-    const double pr7_5 = z[6] * (-cm23);
+    const double pr7_5 = z[6] * (-cm0);
     const double b0 = (((((pr0_0 + pr0_1) + pr0_2) + pr0_3) + pr0_4) + pr0_5) * twelth;
     bmat[(size_t)1 * ne + e] = b0;
     Sy = v[0] * b0;
@@ -224,30 +212,24 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     Sy = Sy + v[7] * b7;
   }
   {  // component 2: O = x, I = y
-    const double cm0 = (((-y[2] - y[3]) + y[4]) + y[5]);  // pair (0,1)
     const double cm1 = (y[1] - y[3]);  // pair (0,2)
-    const double cm2 = (((y[1] + y[2]) - y[4]) - y[7]);  // pair (0,3)
-    const double cm3 = (((-y[1] + y[3]) - y[5]) + y[7]);  // pair (0,4)
     const double cm4 = (-y[1] + y[4]);  // pair (0,5)
     const double cm5 = (y[3] - y[4]);  // pair (0,7)
-    const double cm6 = (((-y[0] - y[3]) + y[5]) + y[6]);  // pair (1,2)
     const double cm7 = (-y[0] + y[2]);  // pair (1,3)
     const double cm8 = (y[0] - y[5]);  // pair (1,4)
-    const double cm9 = (((y[0] - y[2]) + y[4]) - y[6]);  // pair (1,5)
     const double cm10 = (-y[2] + y[5]);  // pair (1,6)
-    const double cm11 = (((-y[0] - y[1]) + y[6]) + y[7]);  // pair (2,3)
     const double cm12 = (y[1] - y[6]);  // pair (2,5)
-    const double cm13 = (((y[1] - y[3]) + y[5]) - y[7]);  // pair (2,6)
     const double cm14 = (-y[3] + y[6]);  // pair (2,7)
     const double cm15 = (-y[0] + y[7]);  // pair (3,4)
     const double cm16 = (y[2] - y[7]);  // pair (3,6)
-    const double cm17 = (((-y[0] + y[2]) - y[4]) + y[6]);  // pair (3,7)
-    const double cm18 = (((-y[0] - y[1]) + y[6]) + y[7]);  // pair (4,5)
     const double cm19 = (-y[5] + y[7]);  // pair (4,6)
-    const double cm20 = (((y[0] + y[3]) - y[5]) - y[6]);  // pair (4,7)
-    const double cm21 = (((-y[1] - y[2]) + y[4]) + y[7]);  // pair (5,6)
     const double cm22 = (y[4] - y[6]);  // pair (5,7)
-    const double cm23 = (((-y[2] - y[3]) + y[4]) + y[5]);  // pair (6,7)
+    const double cm0 = (((-y[2] - y[3]) + y[4]) + y[5]);  // pair (0,1)
+    const double cm2 = (((y[1] + y[2]) - y[4]) - y[7]);  // pair (0,3)
+    const double cm3 = (((-cm1) - y[5]) + y[7]);  // pair (0,4)
+    const double cm6 = (((-y[0] - y[3]) + y[5]) + y[6]);  // pair (1,2)
+    const double cm9 = (((-cm7) + y[4]) - y[6]);  // pair (1,5)
+    const double cm11 = (((-y[0] - y[1]) + y[6]) + y[7]);  // pair (2,3)
     const double pr0_0 = x[1] * cm0;
     const double pr0_1 = x[2] * cm1;
     const double pr0_2 = x[3] * cm2;
@@ -264,38 +246,38 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     const double pr2_1 = x[1] * (-cm6);
     const double pr2_2 = x[3] * cm11;
     const double pr2_3 = x[5] * cm12;
-    const double pr2_4 = x[6] * cm13;
+    const double pr2_4 = x[6] * (-cm3);
     const double pr2_5 = x[7] * cm14;
     const double pr3_0 = x[0] * (-cm2);
     const double pr3_1 = x[1] * (-cm7);
     const double pr3_2 = x[2] * (-cm11);
     const double pr3_3 = x[4] * cm15;
     const double pr3_4 = x[6] * cm16;
-    const double pr3_5 = x[7] * cm17;
+    const double pr3_5 = x[7] * (-cm9);
     const double pr4_0 = x[0] * (-cm3);
     const double pr4_1 = x[1] * (-cm8);
     const double pr4_2 = x[3] * (-cm15);
-    const double pr4_3 = x[5] * cm18;
+    const double pr4_3 = x[5] * cm11;
     const double pr4_4 = x[6] * cm19;
-    const double pr4_5 = x[7] * cm20;
+    const double pr4_5 = x[7] * (-cm6);
     const double pr5_0 = x[0] * (-cm4);
     const double pr5_1 = x[1] * (-cm9);
     const double pr5_2 = x[2] * (-cm12);
-    const double pr5_3 = x[4] * (-cm18);
-    const double pr5_4 = x[6] * cm21;
+    const double pr5_3 = x[4] * (-cm11);
+    const double pr5_4 = x[6] * (-cm2);
     const double pr5_5 = x[7] * cm22;
     const double pr6_0 = x[1] * (-cm10);
-    const double pr6_1 = x[2] * (-cm13);
+    const double pr6_1 = x[2] * cm3;
     const double pr6_2 = x[3] * (-cm16);
     const double pr6_3 = x[4] * (-cm19);
-    const double pr6_4 = x[5] * (-cm21);
-    const double pr6_5 = x[7] * cm23;
+    const double pr6_4 = x[5] * cm2;
+    const double pr6_5 = x[7] * cm0;
     const double pr7_0 = x[0] * (-cm5);
     const double pr7_1 = x[2] * (-cm14);
-    const double pr7_2 = x[3] * (-cm17);
-    const double pr7_3 = x[4] * (-cm20);
+    const double pr7_2 = x[3] * cm9;
+    const double pr7_3 = x[4] * cm6;
     const double pr7_4 = x[5] * (-cm22);
-    const double pr7_5 = x[6] * (-cm23);
+    const double pr7_5 = x[6] * (-cm0);
     const double b0 = (((((pr0_0 + pr0_1) + pr0_2) + pr0_3) + pr0_4) + pr0_5) * twelth;
     bmat[(size_t)2 * ne + e] = b0;
     Sz = w[0] * b0;
@@ -328,30 +310,24 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
 __device__ __forceinline__ double hex_volume(const double* __restrict__ x, const double* __restrict__ y,
     const double* __restrict__ z) {
   const double twelth = 1. / 12.;
-  const double cm0 = (((-z[2] - z[3]) + z[4]) + z[5]);
-  const double cm1 = (z[1] - z[3]);
-  const double cm2 = (((z[1] + z[2]) - z[4]) - z[7]);
-  const double cm3 = (((-z[1] + z[3]) - z[5]) + z[7]);
-  const double cm4 = (-z[1] + z[4]);
-  const double cm5 = (z[3] - z[4]);
-  const double cm6 = (((-z[0] - z[3]) + z[5]) + z[6]);
-  const double cm7 = (-z[0] + z[2]);
-  const double cm8 = (z[0] - z[5]);
-  const double cm9 = (((z[0] - z[2]) + z[4]) - z[6]);
-  const double cm10 = (-z[2] + z[5]);
-  const double cm11 = (((-z[0] - z[1]) + z[6]) + z[7]);
-  const double cm12 = (z[1] - z[6]);
-  const double cm13 = (((z[1] - z[3]) + z[5]) - z[7]);
-  const double cm14 = (-z[3] + z[6]);
-  const double cm15 = (-z[0] + z[7]);
-  const double cm16 = (z[2] - z[7]);
-  const double cm17 = (((-z[0] + z[2]) - z[4]) + z[6]);
-  const double cm18 = (((-z[0] - z[1]) + z[6]) + z[7]);
-  const double cm19 = (-z[5] + z[7]);
-  const double cm20 = (((z[0] + z[3]) - z[5]) - z[6]);
-  const double cm21 = (((-z[1] - z[2]) + z[4]) + z[7]);
-  const double cm22 = (z[4] - z[6]);
-  const double cm23 = (((-z[2] - z[3]) + z[4]) + z[5]);
+  const double cm1 = (z[1] - z[3]);  // pair (0,2)
+  const double cm4 = (-z[1] + z[4]);  // pair (0,5)
+  const double cm5 = (z[3] - z[4]);  // pair (0,7)
+  const double cm7 = (-z[0] + z[2]);  // pair (1,3)
+  const double cm8 = (z[0] - z[5]);  // pair (1,4)
+  const double cm10 = (-z[2] + z[5]);  // pair (1,6)
+  const double cm12 = (z[1] - z[6]);  // pair (2,5)
+  const double cm14 = (-z[3] + z[6]);  // pair (2,7)
+  const double cm15 = (-z[0] + z[7]);  // pair (3,4)
+  const double cm16 = (z[2] - z[7]);  // pair (3,6)
+  const double cm19 = (-z[5] + z[7]);  // pair (4,6)
+  const double cm22 = (z[4] - z[6]);  // pair (5,7)
+  const double cm0 = (((-z[2] - z[3]) + z[4]) + z[5]);  // pair (0,1)
+  const double cm2 = (((z[1] + z[2]) - z[4]) - z[7]);  // pair (0,3)
+  const double cm3 = (((-cm1) - z[5]) + z[7]);  // pair (0,4)
+  const double cm6 = (((-z[0] - z[3]) + z[5]) + z[6]);  // pair (1,2)
+  const double cm9 = (((-cm7) + z[4]) - z[6]);  // pair (1,5)
+  const double cm11 = (((-z[0] - z[1]) + z[6]) + z[7]);  // pair (2,3)
   const double pr0_0 = y[1] * cm0;
   const double pr0_1 = y[2] * cm1;
   const double pr0_2 = y[3] * cm2;
@@ -368,38 +344,38 @@ __device__ __forceinline__ double hex_volume(const double* __restrict__ x, const
   const double pr2_1 = y[1] * (-cm6);
   const double pr2_2 = y[3] * cm11;
   const double pr2_3 = y[5] * cm12;
-  const double pr2_4 = y[6] * cm13;
+  const double pr2_4 = y[6] * (-cm3);
   const double pr2_5 = y[7] * cm14;
   const double pr3_0 = y[0] * (-cm2);
   const double pr3_1 = y[1] * (-cm7);
   const double pr3_2 = y[2] * (-cm11);
   const double pr3_3 = y[4] * cm15;
   const double pr3_4 = y[6] * cm16;
-  const double pr3_5 = y[7] * cm17;
+  const double pr3_5 = y[7] * (-cm9);
   const double pr4_0 = y[0] * (-cm3);
   const double pr4_1 = y[1] * (-cm8);
   const double pr4_2 = y[3] * (-cm15);
-  const double pr4_3 = y[5] * cm18;
+  const double pr4_3 = y[5] * cm11;
   const double pr4_4 = y[6] * cm19;
-  const double pr4_5 = y[7] * cm20;
+  const double pr4_5 = y[7] * (-cm6);
   const double pr5_0 = y[0] * (-cm4);
   const double pr5_1 = y[1] * (-cm9);
   const double pr5_2 = y[2] * (-cm12);
-  const double pr5_3 = y[4] * (-cm18);
-  const double pr5_4 = y[6] * cm21;
+  const double pr5_3 = y[4] * (-cm11);
+  const double pr5_4 = y[6] * (-cm2);
   const double pr5_5 = y[7] * cm22;
   const double pr6_0 = y[1] * (-cm10);
-  const double pr6_1 = y[2] * (-cm13);
+  const double pr6_1 = y[2] * cm3;
   const double pr6_2 = y[3] * (-cm16);
   const double pr6_3 = y[4] * (-cm19);
-  const double pr6_4 = y[5] * (-cm21);
-  const double pr6_5 = y[7] * cm23;
+  const double pr6_4 = y[5] * cm2;
+  const double pr6_5 = y[7] * cm0;
   const double pr7_0 = y[0] * (-cm5);
   const double pr7_1 = y[2] * (-cm14);
-  const double pr7_2 = y[3] * (-cm17);
-  const double pr7_3 = y[4] * (-cm20);
+  const double pr7_2 = y[3] * cm9;
+  const double pr7_3 = y[4] * cm6;
   const double pr7_4 = y[5] * (-cm22);
-  const double pr7_5 = y[6] * (-cm23);
+  const double pr7_5 = y[6] * (-cm0);
   const double vi0 = x[1] * (((((pr1_2 + pr1_3) + pr1_0) + pr1_5) + pr1_4) + pr1_1);
   const double vi1 = x[7] * (((((pr7_0 + pr7_5) + pr7_1) + pr7_2) + pr7_4) + pr7_3);
   const double vi2 = x[3] * (((((pr3_1 + pr3_5) + pr3_4) + pr3_2) + pr3_3) + pr3_0);
