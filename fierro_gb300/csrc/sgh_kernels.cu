@@ -12,10 +12,13 @@
 //       (the IEEE quotient's bits) by Newton iterations from single-precision
 //       seeds, mostly on the FP32 and integer pipes (mode_sqrt, mode_cbrt,
 //       mode_div, mode_rcp in sgh_common.cuh) -- except where the
-//       reference's sums cancel (the hex volume, the element power, the Riemann
-//       velocity), which stay separately rounded (FX_MUL / FX_ADD) so this mode
-//       keeps within 1e-12 of the reference after one cycle and 1e-9 after a
-//       full run.
+//       reference's sums cancel by a factor of the mesh size (the hex volume,
+//       with it B's first component, and the energy update), which stay
+//       separately rounded (FX_MUL / FX_ADD) so this mode keeps within 1e-12
+//       of the reference after one cycle and 1e-9 after a full run.  (Also
+//       contracting those sums, or leaving B's factor 1/12 to its readers, 4 %
+//       faster, moves the rounding noise of velocities at rest past the tests'
+//       bounds.)
 //
 // One cycle is 2 + 3*rk_num_stages launches:
 //   k_dt                    CFL minimum over the last stage's per-block partials,
@@ -98,6 +101,15 @@ __device__ __forceinline__ double ld_pl(const double* p) {
 #include "sgh_cfl.cuh"
 #include "sgh_user_mat.cuh"
 
+// a + b c: fused in the FMA mode, the reference's product and sum in the exact mode.
+__device__ __forceinline__ double mul_add(double a, double b, double c) {
+#if FIERRO_FMA
+  return fma(b, c, a);
+#else
+  return a + b * c;
+#endif
+}
+
 // Velocity gradient (momentum.cpp:59-144): L(i,j) = (sum_l v_i(l) B(l,j)) / vol,
 // B the outward corner normals in rows [lid*3+dim][ne], summed over l in order.
 __device__ __forceinline__ void velocity_gradient(const double (&u)[8], const double (&v)[8], const double (&w)[8],
@@ -169,21 +181,25 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
   double mu[8];
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
   const double q1c = qa * sspd;
+#if FIERRO_FMA
+  const double den_q1c = den * q1c, den_qb = den * qb;  // den (q1c + qb |d|) as one fma per corner
+#endif
 #pragma unroll
   for (int l = 0; l < 8; ++l) {
     const double d0 = vu[l] - vs0, d1 = vv[l] - vs1, d2 = vw[l] - vs2;
     const double mag_vel = mode_sqrt(d0 * d0 + d1 * d1 + d2 * d2);
+#if FIERRO_FMA
+    const double muc = fma(den_qb, mag_vel, den_q1c);
+#else
     const double muc = den * (q1c + qb * mag_vel);
+#endif
     const double b0 = a.bmat[(size_t)(l * 3 + 0) * ne + e];
     const double b1 = a.bmat[(size_t)(l * 3 + 1) * ne + e];
     const double b2 = a.bmat[(size_t)(l * 3 + 2) * ne + e];
     const double mu_term = muc * mode_sqrt(b0 * b0 + b1 * b1 + b2 * b2);
-    // the Riemann velocity's sums stay separately rounded in both modes: the
-    // force's (v* - v) and then the element power cancel, and a contracted v*
-    // would move a cold element's energy by ~1e-12 relative after one cycle
-    s0 = FX_ADD(s0, FX_MUL(mu_term, vu[l]));
-    s1 = FX_ADD(s1, FX_MUL(mu_term, vv[l]));
-    s2 = FX_ADD(s2, FX_MUL(mu_term, vw[l]));
+    s0 = mul_add(s0, mu_term, vu[l]);
+    s1 = mul_add(s1, mu_term, vv[l]);
+    s2 = mul_add(s2, mu_term, vw[l]);
     s3 = s3 + mu_term;
     mu[l] = mu_term;
   }
@@ -406,10 +422,10 @@ __device__ __forceinline__ void node_update(const NodeArgs& a, const int n) {
 #if FIERRO_FMA
   // the reciprocal of the node's mass, formed once per uploaded state (the
   // same IEEE division, so the same bits as forming it here every stage)
-  const double rm = a.node_rm ? a.node_rm[n] : 1.0 / a.node_mass[n];
-  double u1 = u0 + adt * f0 * rm;
-  double v1 = v0 + adt * f1 * rm;
-  double w1 = w0 + adt * f2 * rm;
+  const double adt_rm = adt * (a.node_rm ? a.node_rm[n] : 1.0 / a.node_mass[n]);
+  double u1 = fma(adt_rm, f0, u0);
+  double v1 = fma(adt_rm, f1, v0);
+  double w1 = fma(adt_rm, f2, w0);
 #else
   const Divisor m = divisor(a.node_mass[n]);  // correctly rounded quotients, one reciprocal seed
   double u1 = u0 + quot(adt * f0, m);
@@ -482,15 +498,13 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
     }
     double sie1 = 0.0;
     if (KIND != 2) {
-      // energy (energy_sgh.cpp:16-52): power = sum_c F_c . (v1 + v0)/2, lid-major,
-      // separately rounded in both modes: where a cold element's heating nearly
-      // cancels its energy, a contracted sum would move sie by far more than an ulp
+      // energy (energy_sgh.cpp:16-52): power = sum_c F_c . (v1 + v0)/2, lid-major
       double power = 0.0;
 #pragma unroll
       for (int l = 0; l < 8; ++l) {
-        power = FX_ADD(power, FX_MUL(ld_pl<COH>(a.force + (size_t)(l * 3 + 0) * ne + e), ld_ro<COH>(a.hx + nid[l])));
-        power = FX_ADD(power, FX_MUL(ld_pl<COH>(a.force + (size_t)(l * 3 + 1) * ne + e), ld_ro<COH>(a.hy + nid[l])));
-        power = FX_ADD(power, FX_MUL(ld_pl<COH>(a.force + (size_t)(l * 3 + 2) * ne + e), ld_ro<COH>(a.hz + nid[l])));
+        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 0) * ne + e), ld_ro<COH>(a.hx + nid[l]));
+        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 1) * ne + e), ld_ro<COH>(a.hy + nid[l]));
+        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 2) * ne + e), ld_ro<COH>(a.hz + nid[l]));
       }
       const double adt = a.rk_alpha * ctrl->dt;
       sie1 = a.sie0[e] - FX_MUL(mode_div(adt, a.mass[e]), power);  // not fused: sie1 may cancel sie0
