@@ -46,28 +46,59 @@ namespace FIERRO_RZ_IMPL {
 constexpr int kRzBlock = 128;
 constexpr int kRzNodeBlock = 256;
 
-// get_bmatrix2D (geometry.cpp:315-365): outward corner normals B[l][dim].
-__device__ __forceinline__ void rz_bmatrix(const double (&x)[4], const double (&y)[4], double (&B)[4][2]) {
-  B[0][0] = -0.5 * (y[3] - y[1]);
-  B[1][0] = -0.5 * (y[0] - y[2]);
-  B[2][0] = -0.5 * (y[1] - y[3]);
-  B[3][0] = -0.5 * (y[2] - y[0]);
-  B[0][1] = -0.5 * (x[1] - x[3]);
-  B[1][1] = -0.5 * (x[2] - x[0]);
-  B[2][1] = -0.5 * (x[3] - x[1]);
-  B[3][1] = -0.5 * (x[0] - x[2]);
+// The differences a quad's normals, area, volume and edge lengths are made of,
+// each formed once: a sum or square of the opposite difference is its exact
+// negation, which the compiler does not see.
+struct RzDiffs {
+  double x02, x13, y02, y13;                      // diagonals
+  double x03, x23, x21, x01, y03, y23, y21, y01;  // edges
+};
+__device__ __forceinline__ RzDiffs rz_diffs(const double (&x)[4], const double (&y)[4]) {
+  RzDiffs d;
+  d.x02 = x[0] - x[2];
+  d.x13 = x[1] - x[3];
+  d.y02 = y[0] - y[2];
+  d.y13 = y[1] - y[3];
+  d.x03 = x[0] - x[3];
+  d.x23 = x[2] - x[3];
+  d.x21 = x[2] - x[1];
+  d.x01 = x[0] - x[1];
+  d.y03 = y[0] - y[3];
+  d.y23 = y[2] - y[3];
+  d.y21 = y[2] - y[1];
+  d.y01 = y[0] - y[1];
+  return d;
+}
+
+// get_bmatrix2D (geometry.cpp:315-365): outward corner normals B[l][dim];
+// opposite corners' are opposite.
+__device__ __forceinline__ void rz_bmatrix(const RzDiffs& d, double (&B)[4][2]) {
+  B[0][0] = 0.5 * d.y13;
+  B[1][0] = -0.5 * d.y02;
+  B[2][0] = -B[0][0];
+  B[3][0] = -B[1][0];
+  B[0][1] = -0.5 * d.x13;
+  B[1][1] = 0.5 * d.x02;
+  B[2][1] = -B[0][1];
+  B[3][1] = -B[1][1];
 }
 
 // get_area_quad (geometry.cpp:438-466)
-__device__ __forceinline__ double rz_area(const double (&x)[4], const double (&y)[4]) {
-  return 0.5 * ((x[0] - x[2]) * (y[1] - y[3]) + (x[3] - x[1]) * (y[0] - y[2]));
+__device__ __forceinline__ double rz_area(const RzDiffs& d) { return 0.5 * (d.x02 * d.y13 + (-d.x13) * d.y02); }
+
+// v / 6, correctly rounded (the IEEE quotient in both modes): a quotient one
+// ulp off at most and one remainder step through the rounded reciprocal
+// (Markstein's theorem), 3 FP64 operations instead of a general division.
+__device__ __forceinline__ double sixth(double v) {
+  if (!plain_range(__double_as_longlong(v))) return lib_div(v, 6.0);
+  const double r = 1.0 / 6.0, q = v * r;
+  return fma(fma(-6.0, q, v), r, q);
 }
 
 // get_vol_quad (geometry.cpp:369-434): volume per radian of the revolved quad.
-__device__ __forceinline__ double rz_vol(const double (&x)[4], const double (&y)[4]) {
-  return ((y[2] + y[3] + y[0]) * ((y[2] - y[3]) * (x[0] - x[3]) - (y[0] - y[3]) * (x[2] - x[3])) +
-          (y[0] + y[1] + y[2]) * ((y[0] - y[1]) * (x[2] - x[1]) - (y[2] - y[1]) * (x[0] - x[1]))) /
-         6.0;
+__device__ __forceinline__ double rz_vol(const double (&y)[4], const RzDiffs& d) {
+  return sixth((y[2] + y[3] + y[0]) * (d.y23 * d.x03 - d.y03 * d.x23) +
+               (y[0] + y[1] + y[2]) * (d.y01 * d.x21 - d.y21 * d.x01));
 }
 
 // heron (geometry.cpp:470-500)
@@ -110,26 +141,35 @@ __device__ __forceinline__ void rz_corner_areas(const double (&x)[4], const doub
 // computed factors carry an absolute error of about 9 eps s (sides and s to a few
 // ulps each); so T > 3 sqrt(eps) s^2 ~ 3.2e-8 s^2 keeps every computed factor
 // positive.  With s <= P / 2 for the L1 perimeter P, |cross| = 2T > 1e-4 P^2 is
-// sufficient by more than three orders of magnitude, and its own rounding (a few
-// eps P^2) does not matter.  True for all four centroid triangles (and NaN-free
-// coordinates) means the corner areas need not be formed; otherwise they are,
-// as the reference does.
-__device__ __forceinline__ bool rz_corner_areas_finite(const double (&x)[4], const double (&y)[4]) {
-  double rc = 0.0, zc = 0.0;
-#pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    rc = rc + 0.25 * y[l];
-    zc = zc + 0.25 * x[l];
-  }
+// sufficient by more than three orders of magnitude.  That margin lets the test
+// run in single precision (6 FP64 operations for the centroid's offset instead
+// of 68): with the diagonals a = x2 - x0, b = x3 - x1 and m = x1 + x3 - x0 - x2
+// the corners lie at (-a/2 - m/4, -b/2 + m/4, a/2 - m/4, b/2 + m/4) from the
+// centroid, and rounding a, b and m to 24 bits moves a cross product by under
+// 1e-6 P^2.  Quads too small (P < 1e-13) or large for float fail it.
+// True for all four centroid triangles (and finite coordinates) means the corner
+// areas need not be formed; otherwise they are, as the reference does.
+__device__ __forceinline__ float f32_signed(double d) {
+  const long long b = __double_as_longlong(d);
+  const int e = (int)((b >> 52) & 0x7FF) - 1023 + 127;
+  const unsigned m = (unsigned)((b >> 29) & 0x7FFFFF), s = (unsigned)(b >> 32) & 0x80000000u;
+  return __uint_as_float(s | (e <= 0 ? 0u : e >= 255 ? 0x7F800000u : ((unsigned)e << 23) | m));
+}
+__device__ __forceinline__ bool rz_corner_areas_finite(const RzDiffs& d) {
+  const float ax = 0.5f * f32_signed(-d.x02), bx = 0.5f * f32_signed(-d.x13);
+  const float ay = 0.5f * f32_signed(-d.y02), by = 0.5f * f32_signed(-d.y13);
+  const float mx = 0.25f * f32_signed(-d.x01 - d.x23), my = 0.25f * f32_signed(-d.y01 - d.y23);
+  const float px[4] = {-ax - mx, -bx + mx, ax - mx, bx + mx};
+  const float py[4] = {-ay - my, -by + my, ay - my, by + my};
   bool ok = true;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int j = (i + 1) & 3;
-    const double d1x = x[i] - zc, d1y = y[i] - rc, d2x = x[j] - zc, d2y = y[j] - rc;
-    const double ex = x[j] - x[i], ey = y[j] - y[i];
-    const double cross = d1x * d2y - d1y * d2x;
-    const double P = fabs(d1x) + fabs(d1y) + fabs(d2x) + fabs(d2y) + fabs(ex) + fabs(ey);
-    ok = ok && (fabs(cross) > 1e-4 * P * P);
+    const float cross = px[i] * py[j] - py[i] * px[j];
+    const float P = fabsf(px[i]) + fabsf(py[i]) + fabsf(px[j]) + fabsf(py[j]) + fabsf(px[j] - px[i]) +
+                    fabsf(py[j] - py[i]);
+    const float far = 1e-4f * P * P;
+    ok = ok && (fabsf(cross) > far) && far > 1e-30f;
   }
   return ok;
 }
@@ -163,11 +203,12 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     u[l] = __ldg(a.u + nid[l]);
     v[l] = __ldg(a.v + nid[l]);
   }
+  const RzDiffs df = rz_diffs(x, y);
   double B[4][2], ca[4] = {0.0, 0.0, 0.0, 0.0};
-  rz_bmatrix(x, y, B);
-  const double area = rz_area(x, y);
+  rz_bmatrix(df, B);
+  const double area = rz_area(df);
   const double den = a.den[e], pres = a.pres[e], sspd = a.sspd[e], vol = a.vol[e], div = a.div[e];
-  const bool hoop_zero = !STRENGTH && isfinite(pres) && rz_corner_areas_finite(x, y);
+  const bool hoop_zero = !STRENGTH && isfinite(pres) && rz_corner_areas_finite(df);
   if (!hoop_zero) rz_corner_areas(x, y, ca);
   const int mat = a.mat[e];
   const double* q = a.qtab + 4 * mat;
@@ -191,7 +232,9 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     vs0 = fma(0.25, u[l], vs0);
     vs1 = fma(0.25, v[l], vs1);
   }
-  // MARS impedances (:520-636); |inward normal| = |B|
+  // MARS impedances (:520-636); |inward normal| = |B|, the same at opposite corners
+  const double bn[2] = {mode_sqrt(B[0][0] * B[0][0] + B[0][1] * B[0][1]),
+                        mode_sqrt(B[1][0] * B[1][0] + B[1][1] * B[1][1])};
   double mu[4];
   double s0 = 0.0, s1 = 0.0, s3 = 0.0;
   const double q1c = qa * sspd;
@@ -200,7 +243,7 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     const double d0 = u[l] - vs0, d1 = v[l] - vs1;
     const double mag_vel = mode_sqrt(d0 * d0 + d1 * d1);
     const double muc = den * (q1c + qb * mag_vel);
-    const double mu_term = muc * mode_sqrt(B[l][0] * B[l][0] + B[l][1] * B[l][1]);
+    const double mu_term = muc * bn[l & 1];
     s0 = s0 + mu_term * u[l];
     s1 = s1 + mu_term * v[l];
     s3 = s3 + mu_term;
@@ -256,15 +299,20 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     const double a0 = -B[l][0], a1 = -B[l][1];
     const double vl[2] = {u[l], v[l]};
     double f[2];
+    if (hoop_zero) {
+      // finite normals and no shear: the products with tau's zeros are zeros, and so
+      // are the hoop terms; adding those would only turn a -0.0 force into +0.0,
+      // which is done on the bits
+      f[0] = a0 * t[0] + pm * (vs[0] - vl[0]);
+      f[1] = a1 * t[4] + pm * (vs[1] - vl[1]);
 #pragma unroll
-    for (int d = 0; d < 2; ++d) f[d] = a0 * t[d] + a1 * t[3 + d] + pm * (vs[d] - vl[d]);
-    const double r = y[l];
-    if (r > 1e-14) {
-      if (hoop_zero) {
-        // the terms' exact value (+0.0 turns a -0.0 force into +0.0, as adding them does)
-        f[0] = f[0] + 0.0;
-        f[1] = f[1] + 0.0;
-      } else {
+      for (int d = 0; d < 2; ++d)
+        if ((__double_as_longlong(f[d]) & kAbsMask) == 0) f[d] = 0.0;
+    } else {
+#pragma unroll
+      for (int d = 0; d < 2; ++d) f[d] = a0 * t[d] + a1 * t[3 + d] + pm * (vs[d] - vl[d]);
+      const double r = y[l];
+      if (r > 1e-14) {
         f[0] = f[0] + t[3] * ca[l] / r;
         f[1] = f[1] + (t[4] - t[8]) * ca[l] / r;
       }
@@ -343,7 +391,7 @@ __global__ void __launch_bounds__(kRzNodeBlock) k_node_rz(const RzNodeArgs a) {
   a.x1[n] = x1;
   a.y1[n] = y1;
   double mn = 0.0;
-  if (y1 > a.tiny) mn = a.node_ext[n] / y1;
+  if (y1 > a.tiny) mn = mode_div(a.node_ext[n], y1);
   a.node_mass[n] = mn;
 }
 
@@ -397,11 +445,12 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
       sie1 = a.sie0[e] - mode_div(adt, a.mass[e]) * power;
       a.sie1[e] = sie1;
     }
-    const double vol = (KIND == 2) ? a.vol[e] : rz_vol(x, y);
+    const RzDiffs df = rz_diffs(x, y);
+    const double vol = (KIND == 2) ? a.vol[e] : rz_vol(y, df);
     // divergence for the next stage (momentum.cpp:298-378)
     double B[4][2];
-    rz_bmatrix(x, y, B);
-    const double area = rz_area(x, y);
+    rz_bmatrix(df, B);
+    const double area = rz_area(df);
     const double inverse_area = mode_rcp(area);
     const double mean_radius = mode_div(vol, area);
     const double elem_vel_r = 0.25 * (v[0] + v[1] + v[2] + v[3]);
@@ -430,17 +479,15 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     if (KIND != 0) {
       // CFL step (time_integration.cpp:189-228): the six node-pair distances; the
       // minimum of the square roots is the square root of the minimum
-      double d2 = 0.0;
-      bool first = true;
+      const double dx[6] = {df.x01, df.x02, df.x03, df.x21, df.x13, df.x23};
+      const double dy[6] = {df.y01, df.y02, df.y03, df.y21, df.y13, df.y23};
+      long long kd = 0x7FFFFFFFFFFFFFFFLL;  // squares are >= 0: their bits order as they do
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = i + 1; j <= 3; ++j) {
-          const double dx = x[i] - x[j], dy = y[i] - y[j];
-          const double s = dx * dx + dy * dy;
-          d2 = first ? s : fmin(s, d2);
-          first = false;
-        }
+      for (int i = 0; i < 6; ++i) {
+        const long long k = __double_as_longlong(dx[i] * dx[i] + dy[i] * dy[i]) & kAbsMask;
+        kd = k < kd ? k : kd;
+      }
+      const double d2 = __longlong_as_double(kd);
       const double dist_min = mode_sqrt(d2);
       const double dt_l = mode_div(a.dt_cfl * dist_min, sspd + a.fuzz);
       dkey = isnan(dt_l) ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);
