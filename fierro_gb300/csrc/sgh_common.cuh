@@ -66,6 +66,21 @@ constexpr long long kAbsMask = 0x7FFFFFFFFFFFFFFFLL;
 constexpr long long kMantMask = 0x000FFFFFFFFFFFFFLL;
 constexpr long long kHardBand = 1LL << 32;  // 2^-20 relative, on the bits
 
+// d < 0 and isfinite(d) on the bits: a comparison of doubles takes an FP64 issue
+// slot, these run on the integer pipes.
+__device__ __forceinline__ bool is_negative(double d) {
+  const long long b = __double_as_longlong(d);
+  return b < 0 && (unsigned long long)((b & kAbsMask) - 1) < 0x7FF0000000000000ULL;  // not -0, not NaN
+}
+__device__ __forceinline__ bool is_finite(double d) { return (__double2hiint(d) & 0x7FF00000) != 0x7FF00000; }
+// max(0, r) of a number r that is not NaN, and min(1, v), on the bits.
+__device__ __forceinline__ double at_least_0(double r) { return __double_as_longlong(r) < 0 ? 0.0 : r; }
+__device__ __forceinline__ double at_most_1(double v) {
+  const long long b = __double_as_longlong(v);
+  if (b < 0) return fmin(1.0, v);
+  return b > 0x3FF0000000000000LL ? 1.0 : v;  // NaN too, as fmin has it
+}
+
 // Single-precision image of a positive double within float range (truncated).
 __device__ __forceinline__ float f32_image(double d) {
   const long long b = __double_as_longlong(d);
@@ -264,10 +279,14 @@ __device__ __forceinline__ double quot(double a, const Divisor& d) {
 #endif
 #endif
 }
-// A single quotient or reciprocal: the Newton form in the FMA mode; the
+// A single quotient by the Newton form in both modes: the force passes and the
+// quad kernels, whose registers leave room for it (exact mode, 768^2 quads:
+// k_force_rz 256 -> 250 us, k_elem_rz 157 -> 155; 144^3: k_force 2615 -> 2601).
+__device__ __forceinline__ double newton_div(double a, double b) { return quot(a, divisor(b)); }
+// A single quotient or reciprocal elsewhere: the Newton form in the FMA mode; the
 // library's division in the exact mode, where the remainder test makes the
-// Newton form no cheaper unless several quotients share the divisor's seed
-// (measured: the exact element pass 1.4 % faster with the library's).
+// Newton form no cheaper unless several quotients share the divisor's seed (the
+// exact hex element pass: 3184 us at 144^3 with the library's, 3242 without).
 #if FIERRO_FMA
 __device__ __forceinline__ double mode_div(double a, double b) { return quot(a, divisor(b)); }
 #else

@@ -164,7 +164,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
   const int mat = a.mat[e];
   const double* q = a.qtab + 4 * mat;
   const unsigned br = BR == 2 ? (unsigned)a.br_flags[e] : 0u;
-  const bool compress = BR == 2 ? (br & FIERRO_BR_COMPRESS) != 0 : div < 0;
+  const bool compress = BR == 2 ? (br & FIERRO_BR_COMPRESS) != 0 : is_negative(div);
   const double qa = compress ? q[0] : q[1];  // q1 or q1ex
   const double qb = compress ? q[2] : q[3];  // q2 or q2ex
 
@@ -232,25 +232,25 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
   }
   double r_min = 1.0;
   if (k1 > k0) {
-    const double dsel = okey_decode(D > 0 ? kmin : kmax);
-    const bool regular = isfinite(D) && D != 0.0 && isfinite(dsel);
+    const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
+    const bool regular = is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel);
     if (regular) {
-      const double r_face = mode_div(0.9 * (dsel + small), D);
+      const double r_face = newton_div(0.9 * (dsel + small), D);
       r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
     } else {
       for (int k = k0; k < k1; ++k) {
-        const double r_face = mode_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + small), D);
+        const double r_face = newton_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + small), D);
         r_min = fmin(r_face, r_min);
       }
     }
   }
-  double phi = 1.0 - fmax(0.0, r_min);  // pow(phi, 1.0) == phi
+  double phi = 1.0 - at_least_0(r_min);  // pow(phi, 1.0) == phi
   // Mach-number detector (:318-328)
   const double c_length = pow_third(vol);
   // |div|: on the frozen trajectory, the sign recorded with the compression bit
   const double adiv = BR == 2 ? (compress ? -div : div) : fabs(div);
-  const double araw = mode_div(20.0 * (c_length * adiv), sspd + a.fuzz);
-  const double alpha = BR == 2 ? ((br & FIERRO_BR_MACH_CLAMP) ? 1.0 : araw) : fmin(1.0, araw);
+  const double araw = newton_div(20.0 * (c_length * adiv), sspd + a.fuzz);
+  const double alpha = BR == 2 ? ((br & FIERRO_BR_MACH_CLAMP) ? 1.0 : araw) : at_most_1(araw);
   if (BR == 1) {
     // the limiter's case, and the neighbour that set r_min on the r_face branch
     unsigned lim = FIERRO_LIM_NONE;
@@ -282,7 +282,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     } else if (lim == FIERRO_LIM_FULL) {
       phi = 1.0;
     } else if (lim == FIERRO_LIM_FACE && a.br_sel[e] >= 0) {
-      phi = 1.0 - mode_div(0.9 * (__ldg(a.div + a.br_sel[e]) + small), D);
+      phi = 1.0 - newton_div(0.9 * (__ldg(a.div + a.br_sel[e]) + small), D);
     }  // FIERRO_LIM_IRREGULAR: as evaluated above
   }
   if (TAPE) {
@@ -548,8 +548,8 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
       a.den[e] = den;
       a.pres[e] = pres;
       a.sspd[e] = sspd;
-      if (!(vol > 0.0) || !isfinite(vol)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_VOLUME);
-      if (!isfinite(sie1) || !isfinite(pres)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_STATE);
+      if (__double_as_longlong(vol) <= 0 || !is_finite(vol)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_VOLUME);
+      if (!is_finite(sie1) || !is_finite(pres)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_STATE);
     } else {
       sspd = a.sspd[e];
     }
@@ -569,7 +569,8 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
                                        &s_xyz[16][threadIdx.x], kElemBlock);
       const double dist_min = mode_sqrt(d2min);
       const double dt_l = mode_div(dt_cfl * dist_min, sspd + a.fuzz);
-      dkey = isnan(dt_l) ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);
+      const long long db = __double_as_longlong(dt_l);
+      dkey = (db & kAbsMask) > 0x7FF0000000000000LL ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);  // NaN: no bound
     }
   }
   if (KIND != 0) {

@@ -208,11 +208,11 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
   rz_bmatrix(df, B);
   const double area = rz_area(df);
   const double den = a.den[e], pres = a.pres[e], sspd = a.sspd[e], vol = a.vol[e], div = a.div[e];
-  const bool hoop_zero = !STRENGTH && isfinite(pres) && rz_corner_areas_finite(df);
+  const bool hoop_zero = !STRENGTH && is_finite(pres) && rz_corner_areas_finite(df);
   if (!hoop_zero) rz_corner_areas(x, y, ca);
   const int mat = a.mat[e];
   const double* q = a.qtab + 4 * mat;
-  const bool compress = div < 0;
+  const bool compress = is_negative(div);
   const double qa = compress ? q[0] : q[1];
   const double qb = compress ? q[2] : q[3];
   // Cauchy stress (:480-493): tau(i,j) = stress(i,j), tau(i,i) -= p
@@ -275,21 +275,21 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
   }
   double r_min = 1.0;
   if (k1 > k0) {
-    const double dsel = okey_decode(D > 0 ? kmin : kmax);
-    if (isfinite(D) && D != 0.0 && isfinite(dsel)) {
-      const double r_face = mode_div(0.9 * (dsel + small), D);
+    const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
+    if (is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel)) {
+      const double r_face = newton_div(0.9 * (dsel + small), D);
       r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
     } else {
       for (int k = k0; k < k1; ++k) {
-        const double r_face = mode_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + small), D);
+        const double r_face = newton_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + small), D);
         r_min = fmin(r_face, r_min);
       }
     }
   }
-  double phi = 1.0 - fmax(0.0, r_min);
+  double phi = 1.0 - at_least_0(r_min);
   // Mach-number detector with the characteristic length sqrt(area) (:692-700)
   const double c_length = mode_sqrt(area);
-  const double alpha = fmin(1.0, mode_div(20.0 * (c_length * fabs(div)), sspd + a.fuzz));
+  const double alpha = at_most_1(newton_div(20.0 * (c_length * fabs(div)), sspd + a.fuzz));
   phi = alpha * phi;
   // corner forces with the inward normals -B, then the hoop-stress terms (:718-755)
   const double vs[2] = {vstar0, vstar1};
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kRzNodeBlock) k_node_rz(const RzNodeArgs a) {
   a.x1[n] = x1;
   a.y1[n] = y1;
   double mn = 0.0;
-  if (y1 > a.tiny) mn = mode_div(a.node_ext[n], y1);
+  if (y1 > a.tiny) mn = newton_div(a.node_ext[n], y1);
   a.node_mass[n] = mn;
 }
 
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
         power = power + a.force[(size_t)(l * 2 + 1) * ne + e] * r * __ldg(a.hy + nid[l]);
       }
       const double adt = a.rk_alpha * ctrl->dt;
-      sie1 = a.sie0[e] - mode_div(adt, a.mass[e]) * power;
+      sie1 = a.sie0[e] - newton_div(adt, a.mass[e]) * power;
       a.sie1[e] = sie1;
     }
     const RzDiffs df = rz_diffs(x, y);
@@ -451,19 +451,20 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     double B[4][2];
     rz_bmatrix(df, B);
     const double area = rz_area(df);
-    const double inverse_area = mode_rcp(area);
-    const double mean_radius = mode_div(vol, area);
+    const Divisor da = divisor(area);  // two quotients, one reciprocal seed
+    const double inverse_area = quot(1.0, da);
+    const double mean_radius = quot(vol, da);
     const double elem_vel_r = 0.25 * (v[0] + v[1] + v[2] + v[3]);
     double div = 0.0;
     div = div + (u[0] * B[0][0] + u[1] * B[1][0] + u[2] * B[2][0] + u[3] * B[3][0]) * inverse_area;
     div = div + ((v[0] * B[0][1] + v[1] * B[1][1] + v[2] * B[2][1] + v[3] * B[3][1]) * inverse_area +
-                 mode_div(elem_vel_r, mean_radius));
+                 newton_div(elem_vel_r, mean_radius));
     a.div[e] = div;
     double sspd;
     if (KIND != 2) {
       a.vol[e] = vol;
       // update_state2D (properties.cpp:140, eos.cpp:12-46)
-      const double den = mode_div(a.mass[e], vol);
+      const double den = newton_div(a.mass[e], vol);
       const double gamma = a.gamma[e], csmin = a.csmin[e];
       const double pres = (gamma - 1.0) * sie1 * den;
       sspd = mode_sqrt(gamma * (gamma - 1.0) * sie1);
@@ -471,8 +472,8 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
       a.den[e] = den;
       a.pres[e] = pres;
       a.sspd[e] = sspd;
-      if (!(vol > 0.0) || !isfinite(vol)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_VOLUME);
-      if (!isfinite(sie1) || !isfinite(pres)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_STATE);
+      if (__double_as_longlong(vol) <= 0 || !is_finite(vol)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_VOLUME);
+      if (!is_finite(sie1) || !is_finite(pres)) atomicOr(&ctrl->status, FIERRO_STATUS_BAD_STATE);
     } else {
       sspd = a.sspd[e];
     }
@@ -489,8 +490,9 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
       }
       const double d2 = __longlong_as_double(kd);
       const double dist_min = mode_sqrt(d2);
-      const double dt_l = mode_div(a.dt_cfl * dist_min, sspd + a.fuzz);
-      dkey = isnan(dt_l) ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);
+      const double dt_l = newton_div(a.dt_cfl * dist_min, sspd + a.fuzz);
+      const long long db = __double_as_longlong(dt_l);
+      dkey = (db & kAbsMask) > 0x7FF0000000000000LL ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);  // NaN: no bound
     }
   }
   if (KIND != 0) {
