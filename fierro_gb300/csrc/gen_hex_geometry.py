@@ -119,6 +119,23 @@ def main():
     w("#define FX_ADD(a, b) ((a) + (b))")
     w("#endif")
     w("")
+    w("// a + b c and a b + c d: fused in the FMA build (which product is the fused one is")
+    w("// part of the result), the reference's products and sum in the exact build.")
+    w("__device__ __forceinline__ double mul_add(double a, double b, double c) {")
+    w("#if FIERRO_FMA")
+    w("  return fma(b, c, a);")
+    w("#else")
+    w("  return a + b * c;")
+    w("#endif")
+    w("}")
+    w("__device__ __forceinline__ double mul_mul(double a, double b, double c, double d) {")
+    w("#if FIERRO_FMA")
+    w("  return fma(a, b, __dmul_rn(c, d));")
+    w("#else")
+    w("  return a * b + c * d;")
+    w("#endif")
+    w("}")
+    w("")
     w("// In: x,y,z,u,v,w[8] (node lids 0..7).  Out: vol; bmat rows lid*3+dim at")
     w("// bmat[row*ne + e]; Sx,Sy,Sz = sum_p u_p B(p,0), v_p B(p,1), w_p B(p,2) (p order).")
     w("__device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const double* __restrict__ y,")
@@ -131,6 +148,7 @@ def main():
         w("  {  // component %d: O = %s, I = %s" % (c, O, I))
         combo = emit_combos(w, I, pairs, T)
         # products
+        prod = {}
         for p in range(8):
             for t in range(6):
                 j = J[p][t]
@@ -138,7 +156,7 @@ def main():
                 if c == 0:
                     w("    const double pr%d_%d = FX_MUL(%s[%d], %s);" % (p, t, O, j, cm))
                 else:
-                    w("    const double pr%d_%d = %s[%d] * %s;" % (p, t, O, j, cm))
+                    prod[(p, t)] = "%s[%d], %s" % (O, j, cm)
         if c == 0:
             # volume: sum_a x[VI[a]] * (sum_b products in VJ order)
             for a in range(8):
@@ -154,15 +172,20 @@ def main():
             w("    vol = FX_MUL(%s, twelth);" % expr)
         S = "S" + "xyz"[c]
         for p in range(8):
-            expr = "pr%d_0" % p
-            for t in range(1, 6):
-                expr = "(%s + pr%d_%d)" % (expr, p, t)
+            if c == 0:
+                expr = "pr%d_0" % p
+                for t in range(1, 6):
+                    expr = "(%s + pr%d_%d)" % (expr, p, t)
+            else:
+                expr = "mul_mul(%s, %s)" % (prod[(p, 0)], prod[(p, 1)])
+                for t in range(2, 6):
+                    expr = "mul_add(%s, %s)" % (expr, prod[(p, t)])
             w("    const double b%d = %s * twelth;" % (p, expr))
             w("    bmat[(size_t)%d * ne + e] = b%d;" % (p * 3 + c, p))
-            if p == 0:
-                w("    %s = %s[0] * b0;" % (S, vel[c]))
-            else:
-                w("    %s = %s + %s[%d] * b%d;" % (S, S, vel[c], p, p))
+            if p == 1:
+                w("    %s = mul_mul(%s[0], b0, %s[1], b1);" % (S, vel[c], vel[c]))
+            elif p > 1:
+                w("    %s = mul_add(%s, %s[%d], b%d);" % (S, S, vel[c], p, p))
         w("  }")
     w("}")
     w("")

@@ -316,6 +316,7 @@ int replay_segment(fierro_sgh* h, AdjState* a, int g, int n) {
       na.hz = sn.hz;
       na.ctrl = a->ctrl;
       na.rk_alpha = alpha;
+      na.lanes = h->lanes_node;
       na.block = h->blk_node;
       h->ks->node(na, st);
       ElemArgs ea{};
@@ -347,6 +348,7 @@ int replay_segment(fierro_sgh* h, AdjState* a, int g, int n) {
       ea.rk_alpha = alpha;
       ea.dt_cfl = h->lp.dt_cfl;
       ea.fuzz = h->lp.fuzz;
+      ea.lanes = h->lanes_elem;
       ea.block = h->blk_elem;
       h->ks->elem(ea, s == S - 1 ? 1 : 0, st);
     }

@@ -85,6 +85,7 @@ ForceArgs force_args(fierro_sgh* h, int rb, int q) {
   a.ctrl = h->d_ctrl;
   a.fuzz = h->lp.fuzz;
   a.small = h->lp.small;
+  a.lanes = h->lanes_force;
   a.block = h->blk_force;
   return a;
 }
@@ -116,6 +117,7 @@ NodeArgs node_args(fierro_sgh* h, int c, double alpha) {
   a.hz = h->d_h[2];
   a.ctrl = h->d_ctrl;
   a.rk_alpha = alpha;
+  a.lanes = h->lanes_node;
   a.block = h->blk_node;
   return a;
 }
@@ -150,6 +152,7 @@ ElemArgs elem_args(fierro_sgh* h, int cur_bin, int c, double alpha, int div_out)
   a.rk_alpha = alpha;
   a.dt_cfl = h->lp.dt_cfl;
   a.fuzz = h->lp.fuzz;
+  a.lanes = h->lanes_elem;
   a.block = h->blk_elem;
   return a;
 }
@@ -397,7 +400,11 @@ static int create_impl(fierro_sgh* h, const fierro_mesh* mesh, const fierro_mate
   h->blk_elem = small_mesh_block(ne, kElemBlock);
   h->blk_force = small_mesh_block(ne, kForceBlock);
   h->blk_node = small_mesh_block(nn, kNodeBlock);
-  h->ncfl = (int)((ne + h->blk_elem - 1) / h->blk_elem);
+  h->lanes_force = (long long)ne <= kLanesForce && !h->strength;
+  h->lanes_node = (long long)nn <= kLanesNode;
+  h->lanes_elem = (long long)ne <= kLanesElem && !h->has_hyper;
+  const size_t tile = h->lanes_elem ? kLaneTile : h->blk_elem;
+  h->ncfl = (int)((ne + tile - 1) / tile);
   TRY(dalloc(h, &h->d_cfl, (size_t)h->ncfl));
   TRY(dalloc(h, &h->d_ctrl, 1));
   TRY(dalloc(h, &h->d_node_ext2int, nn));
@@ -979,7 +986,12 @@ struct CkptHeader {
 struct Block {
   void* ptr;
   size_t bytes;
+  bool cfl = false;  // the CFL partials: in the file one per element block, also of a lane handle
 };
+
+// The CFL partials a file holds, and how many of a handle's fall on each.
+int64_t ckpt_ncfl(const fierro_sgh* h) { return h->lanes_elem ? (h->ne + h->blk_elem - 1) / h->blk_elem : h->ncfl; }
+int64_t ckpt_cfl_group(const fierro_sgh* h) { return h->lanes_elem ? h->blk_elem / kLaneTile : 1; }
 
 uint64_t fnv1a(uint64_t h, const void* p, size_t n) {
   const unsigned char* c = static_cast<const unsigned char*>(p);
@@ -1032,7 +1044,7 @@ std::vector<Block> ckpt_blocks(fierro_sgh* h) {
   b.push_back({h->d_mat, ne * sizeof(int)});
   b.push_back({h->d_node_mass, nn * d8});
   b.push_back({h->d_force, ne * (h->dims == 2 ? 8 : 24) * d8});
-  b.push_back({h->d_cfl, (size_t)h->ncfl * sizeof(long long)});
+  b.push_back({h->d_cfl, (size_t)ckpt_ncfl(h) * sizeof(long long), true});
   b.push_back({h->d_ctrl, sizeof(Ctrl)});
   if (h->dims == 2) b.push_back({h->d_node_ext, nn * d8});
   else b.push_back({h->d_bmat, ne * 24 * d8});
@@ -1058,7 +1070,7 @@ CkptHeader ckpt_header(fierro_sgh* h) {
   hd.strength = (h->strength ? 1 : 0) | (h->has_hyper ? 2 : 0);
   hd.topo_hash = (int64_t)topo_hash(h);
   hd.base = h->base;
-  hd.ncfl = h->ncfl;
+  hd.ncfl = ckpt_ncfl(h);
   return hd;
 }
 
@@ -1080,11 +1092,17 @@ extern "C" int fierro_sgh_checkpoint(fierro_sgh* h, const char* path) {
   std::vector<char> buf;
   for (const Block& b : ckpt_blocks(h)) {
     if (!ok) break;
-    buf.resize(std::max<size_t>(b.bytes, 1));
-    cudaError_t err = cudaMemcpy(buf.data(), b.ptr, b.bytes, cudaMemcpyDeviceToHost);
+    const size_t held = b.cfl ? (size_t)h->ncfl * sizeof(long long) : b.bytes;
+    buf.resize(std::max<size_t>(held, 1));
+    cudaError_t err = cudaMemcpy(buf.data(), b.ptr, held, cudaMemcpyDeviceToHost);
     if (err != cudaSuccess) {
       std::fclose(f);
       return set_error(FIERRO_ECUDA, "checkpoint: %s", cudaGetErrorString(err));
+    }
+    if (b.cfl && err == cudaSuccess) {
+      long long* k = reinterpret_cast<long long*>(buf.data());
+      const int64_t g = ckpt_cfl_group(h), n = ckpt_ncfl(h);
+      for (int64_t i = 0; i < n; ++i) k[i] = *std::min_element(k + i * g, k + std::min<int64_t>((i + 1) * g, h->ncfl));
     }
     ok = std::fwrite(buf.data(), 1, b.bytes, f) == b.bytes;
   }
@@ -1147,7 +1165,13 @@ extern "C" int fierro_sgh_restart(fierro_sgh* h, const char* path) {
       std::fclose(f);
       return set_error(FIERRO_EINVAL, "restart: %s is truncated", path);
     }
-    cudaError_t err = cudaMemcpy(b.ptr, buf.data(), b.bytes, cudaMemcpyHostToDevice);
+    if (b.cfl) {
+      const int64_t g = ckpt_cfl_group(h);
+      buf.resize((size_t)h->ncfl * sizeof(long long));
+      long long* k = reinterpret_cast<long long*>(buf.data());
+      for (int64_t i = h->ncfl - 1; i >= 0; --i) k[i] = k[i / g];
+    }
+    cudaError_t err = cudaMemcpy(b.ptr, buf.data(), b.cfl ? buf.size() : b.bytes, cudaMemcpyHostToDevice);
     if (err != cudaSuccess) {
       std::fclose(f);
       return set_error(FIERRO_ECUDA, "restart: %s", cudaGetErrorString(err));

@@ -63,6 +63,13 @@ __device__ __forceinline__ double key_decode(long long k) {
   return __longlong_as_double(k ^ ((k >> 63) & 0x7FFFFFFFFFFFFFFFLL));
 }
 
+// The square of the bound T above: pairs estimated at or below it can be the minimum.
+__device__ __forceinline__ float screen_limit(float e2min, float M) {
+  const float E = 4.0e-6f * M;
+  const float T = (sqrtf(e2min) + E) * (1.0f + 3.814697265625e-06f) + E;  // 2^-18
+  return T * T * (1.0f + 9.5367431640625e-07f);                           // 2^-20
+}
+
 // x, y, z: the element's node coordinates in registers; sx, sy, sz: the same
 // values in per-thread memory (shared or local), indexed [lid * stride].
 __device__ __forceinline__ double min_d2(const double* x, const double* y, const double* z,
@@ -88,9 +95,7 @@ __device__ __forceinline__ double min_d2(const double* x, const double* y, const
       e2[i] = (dx * dx + dy * dy) + dz * dz;
       e2min = fminf(e2min, e2[i]);
     }
-    const float E = 4.0e-6f * M;
-    const float T = (sqrtf(e2min) + E) * (1.0f + 3.814697265625e-06f) + E;  // 2^-18
-    const float T2 = T * T * (1.0f + 9.5367431640625e-07f);                 // 2^-20
+    const float T2 = screen_limit(e2min, M);
     unsigned mask = 0;
 #pragma unroll
     for (int i = 0; i < 28; ++i) mask |= (e2[i] <= T2 ? 1u : 0u) << i;

@@ -81,6 +81,7 @@ struct ForceArgs {
   const double* sie0;  // cycle-start energy (the reference passes elem_sie bin 0)
   double rk_alpha;
   int copy_stress;     // stage 0: elements without a hypo model carry stress_cur over
+  int lanes;           // eight lanes per element (small gas-only meshes, sgh_lanes.cuh)
   int block;           // threads per block (0: kForceBlock)
   int grid;            // batch only: blocks of a persistent grid (0: one block per tile)
 };
@@ -115,6 +116,7 @@ struct NodeArgs {
   const Ctrl* ctrl;
   const int* inst;  // batch only: instance of each node
   double rk_alpha;
+  int lanes;        // one component per thread (small meshes)
   int block;        // threads per block (0: kNodeBlock)
   int grid;         // batch only: blocks of a persistent grid (0: one block per node tile)
 };
@@ -146,6 +148,7 @@ struct ElemArgs {
   const double* stress0;  // cycle-start stress(0)
   double* stress1;        // stress(1), updated in place
   double* statev;         // [nsv][ne]
+  int lanes;              // eight lanes per element, one CFL partial per kLaneTile elements (small meshes)
   int block;              // threads per block, one CFL partial per tile of that many elements (0: kElemBlock;
                           // a batch's block divides kElemBlock)
   int grid;               // batch only: blocks of a persistent grid looping over the tiles (0: one per tile)
@@ -229,6 +232,19 @@ inline int small_mesh_block(long long n, int bs) {
   while (bs > 32 && (n + bs - 1) / bs < kMinBlocks) bs >>= 1;
   return bs;
 }
+
+// Meshes of at most this many elements (nodes) run the lane passes of
+// sgh_lanes.cuh.  A lane pass does about twice the work in an eighth-long chain:
+// it wins until the chip's sub-partitions hold several of its warps each.  Per
+// launch (events, us), one thread per element against eight lanes:
+//                 12^3         20^3         22^3         24^3         32^3
+//   force exact   26.6 / 12.4  26.7 / 22.6  26.7 / 26.9  26.8 / 34.8  42.5 / 68.6
+//   force FMA     20.6 / 10.3  21.4 / 16.6  22.1 / 18.8  22.3 / 24.5  30.6 / 45.0
+//   elem exact    24.5 / 12.2  24.7 / 22.7  24.6 / 28.5  24.8 / 35.0  49.2 / 71.8
+//   elem FMA      20.4 / 10.4  20.5 / 18.7  20.5 / 22.4  20.6 / 27.0  37.0 / 53.9
+//   node exact    10.3 /  8.3  10.4 /  8.4  10.3 /  8.4  10.4 /  9.0  12.3 / 12.3
+constexpr long long kLanesForce = 10500, kLanesElem = 9000, kLanesNode = 30000;
+constexpr int kLaneTile = 4;  // elements per warp of a lane pass
 
 const KernelSet& kernels_exact();
 const KernelSet& kernels_fma();

@@ -67,6 +67,7 @@ struct fierro_sgh {
   int ncfl = 0;  // CFL partials: one per element block
   // threads per block of the element, force and node kernels (small_mesh_block)
   int blk_elem = fierro::kElemBlock, blk_force = fierro::kForceBlock, blk_node = fierro::kNodeBlock;
+  bool lanes_force = false, lanes_node = false, lanes_elem = false;  // small meshes: sgh_lanes.cuh
   fierro::Ctrl* d_ctrl = nullptr;
   double *d_energy_part = nullptr, *d_energy_out = nullptr;
   // pinned double buffer for permuted transfers

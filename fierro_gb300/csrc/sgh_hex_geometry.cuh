@@ -11,6 +11,23 @@
 #define FX_ADD(a, b) ((a) + (b))
 #endif
 
+// a + b c and a b + c d: fused in the FMA build (which product is the fused one is
+// part of the result), the reference's products and sum in the exact build.
+__device__ __forceinline__ double mul_add(double a, double b, double c) {
+#if FIERRO_FMA
+  return fma(b, c, a);
+#else
+  return a + b * c;
+#endif
+}
+__device__ __forceinline__ double mul_mul(double a, double b, double c, double d) {
+#if FIERRO_FMA
+  return fma(a, b, __dmul_rn(c, d));
+#else
+  return a * b + c * d;
+#endif
+}
+
 // In: x,y,z,u,v,w[8] (node lids 0..7).  Out: vol; bmat rows lid*3+dim at
 // bmat[row*ne + e]; Sx,Sy,Sz = sum_p u_p B(p,0), v_p B(p,1), w_p B(p,2) (p order).
 __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const double* __restrict__ y,
@@ -96,28 +113,27 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     vol = FX_MUL(FX_ADD(FX_ADD(FX_ADD(FX_ADD(FX_ADD(FX_ADD(FX_ADD(vi0, vi1), vi2), vi3), vi4), vi5), vi6), vi7), twelth);
     const double b0 = (((((pr0_0 + pr0_1) + pr0_2) + pr0_3) + pr0_4) + pr0_5) * twelth;
     bmat[(size_t)0 * ne + e] = b0;
-    Sx = u[0] * b0;
     const double b1 = (((((pr1_0 + pr1_1) + pr1_2) + pr1_3) + pr1_4) + pr1_5) * twelth;
     bmat[(size_t)3 * ne + e] = b1;
-    Sx = Sx + u[1] * b1;
+    Sx = mul_mul(u[0], b0, u[1], b1);
     const double b2 = (((((pr2_0 + pr2_1) + pr2_2) + pr2_3) + pr2_4) + pr2_5) * twelth;
     bmat[(size_t)6 * ne + e] = b2;
-    Sx = Sx + u[2] * b2;
+    Sx = mul_add(Sx, u[2], b2);
     const double b3 = (((((pr3_0 + pr3_1) + pr3_2) + pr3_3) + pr3_4) + pr3_5) * twelth;
     bmat[(size_t)9 * ne + e] = b3;
-    Sx = Sx + u[3] * b3;
+    Sx = mul_add(Sx, u[3], b3);
     const double b4 = (((((pr4_0 + pr4_1) + pr4_2) + pr4_3) + pr4_4) + pr4_5) * twelth;
     bmat[(size_t)12 * ne + e] = b4;
-    Sx = Sx + u[4] * b4;
+    Sx = mul_add(Sx, u[4], b4);
     const double b5 = (((((pr5_0 + pr5_1) + pr5_2) + pr5_3) + pr5_4) + pr5_5) * twelth;
     bmat[(size_t)15 * ne + e] = b5;
-    Sx = Sx + u[5] * b5;
+    Sx = mul_add(Sx, u[5], b5);
     const double b6 = (((((pr6_0 + pr6_1) + pr6_2) + pr6_3) + pr6_4) + pr6_5) * twelth;
     bmat[(size_t)18 * ne + e] = b6;
-    Sx = Sx + u[6] * b6;
+    Sx = mul_add(Sx, u[6], b6);
     const double b7 = (((((pr7_0 + pr7_1) + pr7_2) + pr7_3) + pr7_4) + pr7_5) * twelth;
     bmat[(size_t)21 * ne + e] = b7;
-    Sx = Sx + u[7] * b7;
+    Sx = mul_add(Sx, u[7], b7);
   }
   {  // component 1: O = z, I = x
     const double cm1 = (x[1] - x[3]);  // pair (0,2)
@@ -138,78 +154,29 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     const double cm6 = (((-x[0] - x[3]) + x[5]) + x[6]);  // pair (1,2)
     const double cm9 = (((-cm7) + x[4]) - x[6]);  // pair (1,5)
     const double cm11 = (((-x[0] - x[1]) + x[6]) + x[7]);  // pair (2,3)
-    const double pr0_0 = z[1] * cm0;
-    const double pr0_1 = z[2] * cm1;
-    const double pr0_2 = z[3] * cm2;
-    const double pr0_3 = z[4] * cm3;
-    const double pr0_4 = z[5] * cm4;
-    const double pr0_5 = z[7] * cm5;
-    const double pr1_0 = z[0] * (-cm0);
-    const double pr1_1 = z[2] * cm6;
-    const double pr1_2 = z[3] * cm7;
-    const double pr1_3 = z[4] * cm8;
-    const double pr1_4 = z[5] * cm9;
-    const double pr1_5 = z[6] * cm10;
-    const double pr2_0 = z[0] * (-cm1);
-    const double pr2_1 = z[1] * (-cm6);
-    const double pr2_2 = z[3] * cm11;
-    const double pr2_3 = z[5] * cm12;
-    const double pr2_4 = z[6] * (-cm3);
-    const double pr2_5 = z[7] * cm14;
-    const double pr3_0 = z[0] * (-cm2);
-    const double pr3_1 = z[1] * (-cm7);
-    const double pr3_2 = z[2] * (-cm11);
-    const double pr3_3 = z[4] * cm15;
-    const double pr3_4 = z[6] * cm16;
-    const double pr3_5 = z[7] * (-cm9);
-    const double pr4_0 = z[0] * (-cm3);
-    const double pr4_1 = z[1] * (-cm8);
-    const double pr4_2 = z[3] * (-cm15);
-    const double pr4_3 = z[5] * cm11;
-    const double pr4_4 = z[6] * cm19;
-    const double pr4_5 = z[7] * (-cm6);
-    const double pr5_0 = z[0] * (-cm4);
-    const double pr5_1 = z[1] * (-cm9);
-    const double pr5_2 = z[2] * (-cm12);
-    const double pr5_3 = z[4] * (-cm11);
-    const double pr5_4 = z[6] * (-cm2);
-    const double pr5_5 = z[7] * cm22;
-    const double pr6_0 = z[1] * (-cm10);
-    const double pr6_1 = z[2] * cm3;
-    const double pr6_2 = z[3] * (-cm16);
-    const double pr6_3 = z[4] * (-cm19);
-    const double pr6_4 = z[5] * cm2;
-    const double pr6_5 = z[7] * cm0;
-    const double pr7_0 = z[0] * (-cm5);
-    const double pr7_1 = z[2] * (-cm14);
-    const double pr7_2 = z[3] * cm9;
-    const double pr7_3 = z[4] * cm6;
-    const double pr7_4 = z[5] * (-cm22);
-    const double pr7_5 = z[6] * (-cm0);
-    const double b0 = (((((pr0_0 + pr0_1) + pr0_2) + pr0_3) + pr0_4) + pr0_5) * twelth;
+    const double b0 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[1], cm0, z[2], cm1), z[3], cm2), z[4], cm3), z[5], cm4), z[7], cm5) * twelth;
     bmat[(size_t)1 * ne + e] = b0;
-    Sy = v[0] * b0;
-    const double b1 = (((((pr1_0 + pr1_1) + pr1_2) + pr1_3) + pr1_4) + pr1_5) * twelth;
+    const double b1 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[0], (-cm0), z[2], cm6), z[3], cm7), z[4], cm8), z[5], cm9), z[6], cm10) * twelth;
     bmat[(size_t)4 * ne + e] = b1;
-    Sy = Sy + v[1] * b1;
-    const double b2 = (((((pr2_0 + pr2_1) + pr2_2) + pr2_3) + pr2_4) + pr2_5) * twelth;
+    Sy = mul_mul(v[0], b0, v[1], b1);
+    const double b2 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[0], (-cm1), z[1], (-cm6)), z[3], cm11), z[5], cm12), z[6], (-cm3)), z[7], cm14) * twelth;
     bmat[(size_t)7 * ne + e] = b2;
-    Sy = Sy + v[2] * b2;
-    const double b3 = (((((pr3_0 + pr3_1) + pr3_2) + pr3_3) + pr3_4) + pr3_5) * twelth;
+    Sy = mul_add(Sy, v[2], b2);
+    const double b3 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[0], (-cm2), z[1], (-cm7)), z[2], (-cm11)), z[4], cm15), z[6], cm16), z[7], (-cm9)) * twelth;
     bmat[(size_t)10 * ne + e] = b3;
-    Sy = Sy + v[3] * b3;
-    const double b4 = (((((pr4_0 + pr4_1) + pr4_2) + pr4_3) + pr4_4) + pr4_5) * twelth;
+    Sy = mul_add(Sy, v[3], b3);
+    const double b4 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[0], (-cm3), z[1], (-cm8)), z[3], (-cm15)), z[5], cm11), z[6], cm19), z[7], (-cm6)) * twelth;
     bmat[(size_t)13 * ne + e] = b4;
-    Sy = Sy + v[4] * b4;
-    const double b5 = (((((pr5_0 + pr5_1) + pr5_2) + pr5_3) + pr5_4) + pr5_5) * twelth;
+    Sy = mul_add(Sy, v[4], b4);
+    const double b5 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[0], (-cm4), z[1], (-cm9)), z[2], (-cm12)), z[4], (-cm11)), z[6], (-cm2)), z[7], cm22) * twelth;
     bmat[(size_t)16 * ne + e] = b5;
-    Sy = Sy + v[5] * b5;
-    const double b6 = (((((pr6_0 + pr6_1) + pr6_2) + pr6_3) + pr6_4) + pr6_5) * twelth;
+    Sy = mul_add(Sy, v[5], b5);
+    const double b6 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[1], (-cm10), z[2], cm3), z[3], (-cm16)), z[4], (-cm19)), z[5], cm2), z[7], cm0) * twelth;
     bmat[(size_t)19 * ne + e] = b6;
-    Sy = Sy + v[6] * b6;
-    const double b7 = (((((pr7_0 + pr7_1) + pr7_2) + pr7_3) + pr7_4) + pr7_5) * twelth;
+    Sy = mul_add(Sy, v[6], b6);
+    const double b7 = mul_add(mul_add(mul_add(mul_add(mul_mul(z[0], (-cm5), z[2], (-cm14)), z[3], cm9), z[4], cm6), z[5], (-cm22)), z[6], (-cm0)) * twelth;
     bmat[(size_t)22 * ne + e] = b7;
-    Sy = Sy + v[7] * b7;
+    Sy = mul_add(Sy, v[7], b7);
   }
   {  // component 2: O = x, I = y
     const double cm1 = (y[1] - y[3]);  // pair (0,2)
@@ -230,78 +197,29 @@ __device__ __forceinline__ void hex_geometry(const double* __restrict__ x, const
     const double cm6 = (((-y[0] - y[3]) + y[5]) + y[6]);  // pair (1,2)
     const double cm9 = (((-cm7) + y[4]) - y[6]);  // pair (1,5)
     const double cm11 = (((-y[0] - y[1]) + y[6]) + y[7]);  // pair (2,3)
-    const double pr0_0 = x[1] * cm0;
-    const double pr0_1 = x[2] * cm1;
-    const double pr0_2 = x[3] * cm2;
-    const double pr0_3 = x[4] * cm3;
-    const double pr0_4 = x[5] * cm4;
-    const double pr0_5 = x[7] * cm5;
-    const double pr1_0 = x[0] * (-cm0);
-    const double pr1_1 = x[2] * cm6;
-    const double pr1_2 = x[3] * cm7;
-    const double pr1_3 = x[4] * cm8;
-    const double pr1_4 = x[5] * cm9;
-    const double pr1_5 = x[6] * cm10;
-    const double pr2_0 = x[0] * (-cm1);
-    const double pr2_1 = x[1] * (-cm6);
-    const double pr2_2 = x[3] * cm11;
-    const double pr2_3 = x[5] * cm12;
-    const double pr2_4 = x[6] * (-cm3);
-    const double pr2_5 = x[7] * cm14;
-    const double pr3_0 = x[0] * (-cm2);
-    const double pr3_1 = x[1] * (-cm7);
-    const double pr3_2 = x[2] * (-cm11);
-    const double pr3_3 = x[4] * cm15;
-    const double pr3_4 = x[6] * cm16;
-    const double pr3_5 = x[7] * (-cm9);
-    const double pr4_0 = x[0] * (-cm3);
-    const double pr4_1 = x[1] * (-cm8);
-    const double pr4_2 = x[3] * (-cm15);
-    const double pr4_3 = x[5] * cm11;
-    const double pr4_4 = x[6] * cm19;
-    const double pr4_5 = x[7] * (-cm6);
-    const double pr5_0 = x[0] * (-cm4);
-    const double pr5_1 = x[1] * (-cm9);
-    const double pr5_2 = x[2] * (-cm12);
-    const double pr5_3 = x[4] * (-cm11);
-    const double pr5_4 = x[6] * (-cm2);
-    const double pr5_5 = x[7] * cm22;
-    const double pr6_0 = x[1] * (-cm10);
-    const double pr6_1 = x[2] * cm3;
-    const double pr6_2 = x[3] * (-cm16);
-    const double pr6_3 = x[4] * (-cm19);
-    const double pr6_4 = x[5] * cm2;
-    const double pr6_5 = x[7] * cm0;
-    const double pr7_0 = x[0] * (-cm5);
-    const double pr7_1 = x[2] * (-cm14);
-    const double pr7_2 = x[3] * cm9;
-    const double pr7_3 = x[4] * cm6;
-    const double pr7_4 = x[5] * (-cm22);
-    const double pr7_5 = x[6] * (-cm0);
-    const double b0 = (((((pr0_0 + pr0_1) + pr0_2) + pr0_3) + pr0_4) + pr0_5) * twelth;
+    const double b0 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[1], cm0, x[2], cm1), x[3], cm2), x[4], cm3), x[5], cm4), x[7], cm5) * twelth;
     bmat[(size_t)2 * ne + e] = b0;
-    Sz = w[0] * b0;
-    const double b1 = (((((pr1_0 + pr1_1) + pr1_2) + pr1_3) + pr1_4) + pr1_5) * twelth;
+    const double b1 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[0], (-cm0), x[2], cm6), x[3], cm7), x[4], cm8), x[5], cm9), x[6], cm10) * twelth;
     bmat[(size_t)5 * ne + e] = b1;
-    Sz = Sz + w[1] * b1;
-    const double b2 = (((((pr2_0 + pr2_1) + pr2_2) + pr2_3) + pr2_4) + pr2_5) * twelth;
+    Sz = mul_mul(w[0], b0, w[1], b1);
+    const double b2 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[0], (-cm1), x[1], (-cm6)), x[3], cm11), x[5], cm12), x[6], (-cm3)), x[7], cm14) * twelth;
     bmat[(size_t)8 * ne + e] = b2;
-    Sz = Sz + w[2] * b2;
-    const double b3 = (((((pr3_0 + pr3_1) + pr3_2) + pr3_3) + pr3_4) + pr3_5) * twelth;
+    Sz = mul_add(Sz, w[2], b2);
+    const double b3 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[0], (-cm2), x[1], (-cm7)), x[2], (-cm11)), x[4], cm15), x[6], cm16), x[7], (-cm9)) * twelth;
     bmat[(size_t)11 * ne + e] = b3;
-    Sz = Sz + w[3] * b3;
-    const double b4 = (((((pr4_0 + pr4_1) + pr4_2) + pr4_3) + pr4_4) + pr4_5) * twelth;
+    Sz = mul_add(Sz, w[3], b3);
+    const double b4 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[0], (-cm3), x[1], (-cm8)), x[3], (-cm15)), x[5], cm11), x[6], cm19), x[7], (-cm6)) * twelth;
     bmat[(size_t)14 * ne + e] = b4;
-    Sz = Sz + w[4] * b4;
-    const double b5 = (((((pr5_0 + pr5_1) + pr5_2) + pr5_3) + pr5_4) + pr5_5) * twelth;
+    Sz = mul_add(Sz, w[4], b4);
+    const double b5 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[0], (-cm4), x[1], (-cm9)), x[2], (-cm12)), x[4], (-cm11)), x[6], (-cm2)), x[7], cm22) * twelth;
     bmat[(size_t)17 * ne + e] = b5;
-    Sz = Sz + w[5] * b5;
-    const double b6 = (((((pr6_0 + pr6_1) + pr6_2) + pr6_3) + pr6_4) + pr6_5) * twelth;
+    Sz = mul_add(Sz, w[5], b5);
+    const double b6 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[1], (-cm10), x[2], cm3), x[3], (-cm16)), x[4], (-cm19)), x[5], cm2), x[7], cm0) * twelth;
     bmat[(size_t)20 * ne + e] = b6;
-    Sz = Sz + w[6] * b6;
-    const double b7 = (((((pr7_0 + pr7_1) + pr7_2) + pr7_3) + pr7_4) + pr7_5) * twelth;
+    Sz = mul_add(Sz, w[6], b6);
+    const double b7 = mul_add(mul_add(mul_add(mul_add(mul_mul(x[0], (-cm5), x[2], (-cm14)), x[3], cm9), x[4], cm6), x[5], (-cm22)), x[6], (-cm0)) * twelth;
     bmat[(size_t)23 * ne + e] = b7;
-    Sz = Sz + w[7] * b7;
+    Sz = mul_add(Sz, w[7], b7);
   }
 }
 

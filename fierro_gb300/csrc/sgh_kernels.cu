@@ -45,6 +45,7 @@
 #include <cstdint>
 
 #include "sgh_device.h"
+#include "sgh_hex.h"
 
 #ifndef FIERRO_FMA
 #error "compile with -DFIERRO_FMA=0 or -DFIERRO_FMA=1"
@@ -101,15 +102,6 @@ __device__ __forceinline__ double ld_pl(const double* p) {
 #include "sgh_cfl.cuh"
 #include "sgh_user_mat.cuh"
 
-// a + b c: fused in the FMA mode, the reference's product and sum in the exact mode.
-__device__ __forceinline__ double mul_add(double a, double b, double c) {
-#if FIERRO_FMA
-  return fma(b, c, a);
-#else
-  return a + b * c;
-#endif
-}
-
 // Velocity gradient (momentum.cpp:59-144): L(i,j) = (sum_l v_i(l) B(l,j)) / vol,
 // B the outward corner normals in rows [lid*3+dim][ne], summed over l in order.
 __device__ __forceinline__ void velocity_gradient(const double (&u)[8], const double (&v)[8], const double (&w)[8],
@@ -130,6 +122,80 @@ __device__ __forceinline__ void velocity_gradient(const double (&u)[8], const do
     L[3 + j] = sv * inverse_vol;
     L[6 + j] = sw * inverse_vol;
   }
+}
+
+// ---------------------------------------------------------------------------
+// The scalar steps the one-thread-per-element passes and the lane passes
+// (sgh_lanes.cuh) share; what the FMA mode fuses is written out, as the two must
+// round alike.
+// a^2 + b^2 + c^2, left to right
+__device__ __forceinline__ double sum_sq(double a, double b, double c) {
+  return mul_add(mul_mul(a, a, b, b), c, c);
+}
+// MARS impedance (force_sgh.cpp:176-255): mu = den (q1 c + q2 |v - v_avg|) |B|
+struct Impedance {
+  double lin, quad, den;
+};
+__device__ __forceinline__ Impedance impedance(double den, double sspd, double qa, double qb) {
+  const double q1c = qa * sspd;
+#if FIERRO_FMA
+  return Impedance{den * q1c, den * qb, den};  // den (q1c + qb |d|) as one fma per corner
+#else
+  return Impedance{q1c, qb, den};
+#endif
+}
+__device__ __forceinline__ double corner_impedance(const Impedance& z, double d0, double d1, double d2, double b0,
+                                                   double b1, double b2) {
+  const double mag_vel = mode_sqrt(sum_sq(d0, d1, d2));
+#if FIERRO_FMA
+  const double muc = fma(z.quad, mag_vel, z.lin);
+#else
+  const double muc = z.den * (z.lin + z.quad * mag_vel);
+#endif
+  return muc * mode_sqrt(sum_sq(b0, b1, b2));
+}
+// Shock detector (force_sgh.cpp:287-315): r_face = 0.9 (div_nb + small) / (div + small)
+// is monotone in div_nb (non-decreasing for div + small > 0, non-increasing for < 0),
+// so the minimum over neighbours is attained at the smallest (resp. largest)
+// neighbour divergence (keys kmin, kmax) and needs one division instead of one
+// per neighbour.
+__device__ __forceinline__ double limiter_min(const ForceArgs& a, double div, int k0, int k1, long long kmin,
+                                              long long kmax) {
+  const double D = div + a.small;
+  double r_min = 1.0;
+  if (k1 > k0) {
+    const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
+    const bool regular = is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel);
+    if (regular) {
+      const double r_face = newton_div(0.9 * (dsel + a.small), D);
+      r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
+    } else {
+      for (int k = k0; k < k1; ++k) {
+        const double r_face = newton_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + a.small), D);
+        r_min = fmin(r_face, r_min);
+      }
+    }
+  }
+  return r_min;
+}
+// Mach-number detector (force_sgh.cpp:318-328)
+__device__ __forceinline__ double mach_switch(double vol, double div, double sspd, double fuzz) {
+  return at_most_1(newton_div(20.0 * (pow_third(vol) * fabs(div)), sspd + fuzz));
+}
+// Divergence from the velocity sums (momentum.cpp:265-286)
+__device__ __forceinline__ double divergence(double Sx, double Sy, double Sz, double vol) {
+  const double inverse_vol = mode_rcp(vol);
+  double div = 0.0;
+  div = mul_add(div, Sx, inverse_vol);
+  div = mul_add(div, Sy, inverse_vol);
+  div = mul_add(div, Sz, inverse_vol);
+  return div;
+}
+// Order key of the element CFL step dt_cfl * min distance / (c + fuzz)
+// (time_integration.cpp:124-131); a NaN bounds nothing.
+__device__ __forceinline__ long long cfl_key(double d2min, double sspd, double dt_cfl, double fuzz) {
+  const double dt_l = mode_div(dt_cfl * mode_sqrt(d2min), sspd + fuzz);
+  return (__double_as_longlong(dt_l) & kAbsMask) > 0x7FF0000000000000LL ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);
 }
 
 // ---------------------------------------------------------------------------
@@ -180,23 +246,13 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
   // MARS impedances (:176-255)
   double mu[8];
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  const double q1c = qa * sspd;
-#if FIERRO_FMA
-  const double den_q1c = den * q1c, den_qb = den * qb;  // den (q1c + qb |d|) as one fma per corner
-#endif
+  const Impedance z = impedance(den, sspd, qa, qb);
 #pragma unroll
   for (int l = 0; l < 8; ++l) {
-    const double d0 = vu[l] - vs0, d1 = vv[l] - vs1, d2 = vw[l] - vs2;
-    const double mag_vel = mode_sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-#if FIERRO_FMA
-    const double muc = fma(den_qb, mag_vel, den_q1c);
-#else
-    const double muc = den * (q1c + qb * mag_vel);
-#endif
     const double b0 = a.bmat[(size_t)(l * 3 + 0) * ne + e];
     const double b1 = a.bmat[(size_t)(l * 3 + 1) * ne + e];
     const double b2 = a.bmat[(size_t)(l * 3 + 2) * ne + e];
-    const double mu_term = muc * mode_sqrt(b0 * b0 + b1 * b1 + b2 * b2);
+    const double mu_term = corner_impedance(z, vu[l] - vs0, vv[l] - vs1, vw[l] - vs2, b0, b1, b2);
     s0 = mul_add(s0, mu_term, vu[l]);
     s1 = mul_add(s1, mu_term, vv[l]);
     s2 = mul_add(s2, mu_term, vw[l]);
@@ -217,10 +273,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     vstar2 = quot(s2, ds3);
 #endif
   }
-  // shock detector (:287-315): r_face = 0.9 (div_nb + small) / (div + small) is
-  // monotone in div_nb (non-decreasing for div + small > 0, non-increasing for < 0),
-  // so the minimum over neighbours is attained at the smallest (resp. largest)
-  // neighbour divergence and needs one division instead of one per neighbour.
+  // shock detector (:287-315)
   const double small = a.small;
   const double D = div + small;
   const int k0 = a.eie_start[e], k1 = a.eie_start[e + 1];
@@ -230,20 +283,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     kmin = key < kmin ? key : kmin;
     kmax = key > kmax ? key : kmax;
   }
-  double r_min = 1.0;
-  if (k1 > k0) {
-    const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
-    const bool regular = is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel);
-    if (regular) {
-      const double r_face = newton_div(0.9 * (dsel + small), D);
-      r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
-    } else {
-      for (int k = k0; k < k1; ++k) {
-        const double r_face = newton_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + small), D);
-        r_min = fmin(r_face, r_min);
-      }
-    }
-  }
+  const double r_min = limiter_min(a, div, k0, k1, kmin, kmax);
   double phi = 1.0 - at_least_0(r_min);  // pow(phi, 1.0) == phi
   // Mach-number detector (:318-328)
   const double c_length = pow_third(vol);
@@ -324,9 +364,9 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
       const double b0 = a.bmat[(size_t)(l * 3 + 0) * ne + e];
       const double b1 = a.bmat[(size_t)(l * 3 + 1) * ne + e];
       const double b2 = a.bmat[(size_t)(l * 3 + 2) * ne + e];
-      a.force[(size_t)(l * 3 + 0) * ne + e] = b0 * pres + pm * (vstar0 - vu[l]);
-      a.force[(size_t)(l * 3 + 1) * ne + e] = b1 * pres + pm * (vstar1 - vv[l]);
-      a.force[(size_t)(l * 3 + 2) * ne + e] = b2 * pres + pm * (vstar2 - vw[l]);
+      a.force[(size_t)(l * 3 + 0) * ne + e] = mul_mul(b0, pres, pm, vstar0 - vu[l]);
+      a.force[(size_t)(l * 3 + 1) * ne + e] = mul_mul(b1, pres, pm, vstar1 - vv[l]);
+      a.force[(size_t)(l * 3 + 2) * ne + e] = mul_mul(b2, pres, pm, vstar2 - vw[l]);
     }
   } else {
     // Cauchy stress tau = stress(1) - p I (:128-140), then the corner forces with
@@ -443,9 +483,9 @@ __device__ __forceinline__ void node_update(const NodeArgs& a, const int n) {
   a.hx[n] = hu;
   a.hy[n] = hv;
   a.hz[n] = hw;
-  a.x1[n] = a.x0[n] + adt * hu;
-  a.y1[n] = a.y0[n] + adt * hv;
-  a.z1[n] = a.z0[n] + adt * hw;
+  a.x1[n] = mul_add(a.x0[n], adt, hu);
+  a.y1[n] = mul_add(a.y0[n], adt, hv);
+  a.z1[n] = mul_add(a.z0[n], adt, hw);
 }
 
 // One thread per node; a batch may run as a persistent grid striding over the nodes.
@@ -515,11 +555,7 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
     // the priming pass keeps the uploaded volume, as get_divergence reads elem_vol
     const double vol = (KIND == 2) ? a.vol[e] : vol_geo;
     // divergence for the next stage (momentum.cpp:265-286), with this geometry
-    const double inverse_vol = mode_rcp(vol);
-    double div = 0.0;
-    div = div + Sx * inverse_vol;
-    div = div + Sy * inverse_vol;
-    div = div + Sz * inverse_vol;
+    const double div = divergence(Sx, Sy, Sz, vol);
     a.div[e] = div;
     double sspd;
     if (KIND != 2) {
@@ -554,8 +590,8 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
       sspd = a.sspd[e];
     }
     if (KIND != 0) {
-      // element CFL step dt_cfl * min distance / (c + fuzz) (time_integration.cpp:124-131);
-      // min of the square roots == square root of the min (sqrt is monotone, exact).
+      // element CFL step: min of the square roots == square root of the min (sqrt is
+      // monotone, exact).
       // The coordinates go to this thread's column of shared memory for the exact
       // re-evaluation of the screened pairs (no other thread reads them).
       __shared__ double s_xyz[24][kElemBlock];
@@ -567,10 +603,7 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
       }
       const double d2min = cfl::min_d2(x, y, z, &s_xyz[0][threadIdx.x], &s_xyz[8][threadIdx.x],
                                        &s_xyz[16][threadIdx.x], kElemBlock);
-      const double dist_min = mode_sqrt(d2min);
-      const double dt_l = mode_div(dt_cfl * dist_min, sspd + a.fuzz);
-      const long long db = __double_as_longlong(dt_l);
-      dkey = (db & kAbsMask) > 0x7FF0000000000000LL ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);  // NaN: no bound
+      dkey = cfl_key(d2min, sspd, dt_cfl, a.fuzz);
     }
   }
   if (KIND != 0) {
@@ -593,6 +626,8 @@ __global__ void FIERRO_ELEM_BOUNDS k_elem(const ElemArgs a) {
     elem_tile<KIND, false, STRENGTH>(a, blockIdx.x);
   }
 }
+
+#include "sgh_lanes.cuh"
 
 // ---------------------------------------------------------------------------
 // A batch's RK stage in one cooperative launch: the force pass, a grid barrier,
@@ -773,7 +808,8 @@ static unsigned grid_or(int grid, unsigned blocks) {
 static void launch_force(const ForceArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);
   const unsigned g = blocks_for(a.ne, bs);
-  if (a.inst) k_force<true, false, false><<<grid_or(a.grid, g), bs, 0, s>>>(a);
+  if (a.lanes) k_force_lanes<<<blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, 0, s>>>(a);
+  else if (a.inst) k_force<true, false, false><<<grid_or(a.grid, g), bs, 0, s>>>(a);
   else if (a.stress_out) k_force<false, false, true><<<g, bs, 0, s>>>(a);
   else k_force<false, false, false><<<g, bs, 0, s>>>(a);
 }
@@ -788,7 +824,10 @@ static void launch_force_branch(const ForceArgs& a, int mode, cudaStream_t s) {
 }
 static void launch_node(const NodeArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kNodeBlock);
-  if (a.inst) k_node<true><<<grid_or(a.grid, blocks_for(a.nn, bs)), bs, 0, s>>>(a);
+  if (a.lanes) {
+    const int b = small_mesh_block(3LL * a.nn, kNodeBlock);
+    k_node_lanes<<<dim3(blocks_for(a.nn, b), 3), b, 0, s>>>(a);
+  } else if (a.inst) k_node<true><<<grid_or(a.grid, blocks_for(a.nn, bs)), bs, 0, s>>>(a);
   else k_node<false><<<blocks_for(a.nn, bs), bs, 0, s>>>(a);
 }
 template <bool B, bool S>
@@ -800,10 +839,18 @@ static void launch_elem_t(const ElemArgs& a, int kind, cudaStream_t s) {
   else k_elem<2, B, false><<<g, bs, 0, s>>>(a);
 }
 static void launch_elem(const ElemArgs& a, int kind, cudaStream_t s) {
+  if (a.lanes) {
+    const unsigned g = blocks_for(8LL * a.ne, kLaneBlock);
+    if (kind == 0) k_elem_lanes<0><<<g, kLaneBlock, 0, s>>>(a);
+    else if (kind == 1) k_elem_lanes<1><<<g, kLaneBlock, 0, s>>>(a);
+    else k_elem_lanes<2><<<g, kLaneBlock, 0, s>>>(a);
+    return;
+  }
   if (a.inst) launch_elem_t<true, false>(a, kind, s);
   else if (a.stress1) launch_elem_t<false, true>(a, kind, s);
   else launch_elem_t<false, false>(a, kind, s);
 }
+static_assert(kLaneTile == kGroups, "one CFL partial per warp of the lane passes");
 static void launch_dt(const DtArgs& a, cudaStream_t s) {
   if (a.part_start) k_dt_batch<<<a.ninst, 256, 0, s>>>(a);
   else k_dt<<<1, 1024, 0, s>>>(a);

@@ -1,0 +1,448 @@
+// The force, node and element passes of small meshes: eight lanes per element
+// (one per corner), one thread per node component.  Included in sgh_kernels.cu's
+// implementation namespace; the results are those of the one-thread-per-element
+// passes bit for bit, in both modes.
+//
+// Bound: a warp issues one FP64 instruction every ~65 clocks (GB300 has half an
+// FP64 lane per clock and sub-partition, whatever the number of active lanes), so
+// with at most one warp per sub-partition (608) a pass takes as long as one
+// thread's chain: 465 instructions for an element's exact force, 15 us, however
+// few elements there are.  Eight lanes cut the chain to the ~95 instructions one
+// corner and the ordered sums take, at twice the total work, which such a mesh
+// does not fill the chip with: a 12^3 cycle 106 -> 50 us exact, 84 -> 43 us FMA,
+// 8^3 105 -> 48 us.  Sums whose order is part of the result run in one
+// lane over the corners' products in shared memory (different lanes summing
+// different quantities in the same instructions); everything else is per corner.
+#pragma once
+
+// ---------------------------------------------------------------------------
+// The hex cofactor tables (sgh_hex.h), rearranged per lane.  two[m] = (i, j): the
+// combo I[i] - I[j]; four[m]: signed 1-based terms summed left to right; a lane's
+// row: for each of its six products the O node (3 bits), the combo (5 bits: 0-11
+// two-term, 12-17 four-term) and its sign (1 bit); vol: the volume's order of the
+// six products (3 bits each) and the node's place in the volume's sum (3 bits).
+struct LaneTables {
+  unsigned long long two[2], four[2], row[8];
+  unsigned vol[8];
+};
+constexpr LaneTables make_lane_tables() {
+  LaneTables r{};
+  signed char uniq[18][4] = {};
+  int n2 = 0, n4 = 0;
+  for (int pass = 0; pass < 2; ++pass)
+    for (int p = 0; p < 8; ++p)
+      for (int t = 0; t < 6; ++t) {
+        const signed char* T = hex::TERMS[p][t];
+        const bool is4 = T[2] != 0;
+        if (is4 != (pass == 1) || hex::J[p][t] < p) continue;
+        bool known = false;
+        const int lo = is4 ? 12 : 0, hi = is4 ? 12 + n4 : n2;
+        for (int k = lo; k < hi; ++k) {
+          bool same = true, neg = true;
+          for (int q = 0; q < 4; ++q) {
+            if (uniq[k][q] != T[q]) same = false;
+            if (uniq[k][q] != -T[q]) neg = false;
+          }
+          if (same || neg) known = true;
+        }
+        if (known) continue;
+        const int at = is4 ? 12 + n4++ : n2++;
+        for (int q = 0; q < 4; ++q) uniq[at][q] = T[q];
+      }
+  for (int k = 0; k < 12; ++k) {
+    const int i = (uniq[k][0] > 0 ? uniq[k][0] : uniq[k][1]) - 1, j = -(uniq[k][0] > 0 ? uniq[k][1] : uniq[k][0]) - 1;
+    r.two[k / 10] |= (unsigned long long)(i | (j << 3)) << (6 * (k % 10));
+  }
+  for (int k = 0; k < 6; ++k) {
+    unsigned long long w = 0;
+    for (int q = 0; q < 4; ++q) {
+      const int v = uniq[12 + k][q];
+      w |= (unsigned long long)(((v > 0 ? v : -v) - 1) | (v < 0 ? 8 : 0)) << (4 * q);
+    }
+    r.four[k / 4] |= w << (16 * (k % 4));
+  }
+  for (int p = 0; p < 8; ++p) {
+    for (int t = 0; t < 6; ++t) {
+      const signed char* T = hex::TERMS[p][t];
+      const int lo = T[2] != 0 ? 12 : 0, hi = T[2] != 0 ? 18 : 12;
+      for (int k = lo; k < hi; ++k) {
+        bool same = true, neg = true;
+        for (int q = 0; q < 4; ++q) {
+          if (uniq[k][q] != T[q]) same = false;
+          if (uniq[k][q] != -T[q]) neg = false;
+        }
+        // a two-term combo is kept as (positive) - (negative): -a + b is b - a
+        if (same || neg) r.row[p] |= (unsigned long long)(hex::J[p][t] | (k << 3) | (neg ? 256 : 0)) << (9 * t);
+      }
+    }
+    for (int a = 0; a < 8; ++a)
+      if (hex::VI[a] == p) {
+        for (int b = 0; b < 6; ++b) r.vol[p] |= (unsigned)hex::slot(p, hex::VJ[a][b]) << (3 * b);
+        r.vol[p] |= (unsigned)a << 18;
+      }
+  }
+  return r;
+}
+constexpr LaneTables kLane = make_lane_tables();
+
+// One of eight constants by lane, by selects (no memory access).
+__device__ __forceinline__ unsigned long long by_lane(int l, unsigned long long a, unsigned long long b,
+                                                      unsigned long long c, unsigned long long d, unsigned long long e,
+                                                      unsigned long long f, unsigned long long g,
+                                                      unsigned long long h) {
+  const unsigned long long ab = l & 1 ? b : a, cd = l & 1 ? d : c, ef = l & 1 ? f : e, gh = l & 1 ? h : g;
+  const unsigned long long lo = l & 2 ? cd : ab, hi = l & 2 ? gh : ef;
+  return l & 4 ? hi : lo;
+}
+__device__ __forceinline__ double flip(double v, unsigned neg) {
+  return __hiloint2double(__double2hiint(v) ^ (int)(neg << 31), __double2loint(v));
+}
+// Value of the first lane of each group of eight, or of its lane `src`.
+__device__ __forceinline__ double from_lane(double v, int src) { return __shfl_sync(0xFFFFFFFFu, v, src, 8); }
+__device__ __forceinline__ long long group_min(long long k) {
+  for (int o = 4; o > 0; o >>= 1) {
+    const long long t = __shfl_xor_sync(0xFFFFFFFFu, k, o);
+    k = t < k ? t : k;
+  }
+  return k;
+}
+
+constexpr int kLaneBlock = 64;               // threads: two warps, eight elements
+constexpr int kLaneWarps = kLaneBlock / 32;
+constexpr int kGroups = 4;                   // elements per warp
+
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
+  // per element: the corners' velocities and impedance terms, rows u, v, w, mu
+  __shared__ double s_v[kLaneWarps][kGroups][4][9];
+  if (!a.ctrl->active) return;
+  const int t = blockIdx.x * kLaneBlock + threadIdx.x;
+  const int lane = threadIdx.x & 31, l = lane & 7, ne = a.ne;
+  if ((t & ~31) >= 8 * ne) return;  // whole warps past the end
+  const bool live = (t >> 3) < ne;
+  const int e = live ? t >> 3 : ne - 1;
+  double(*sv)[9] = s_v[threadIdx.x >> 5][lane >> 3];
+  const int n = __ldg(a.nie + 8 * (size_t)e + l);
+  const double vu = __ldg(a.u + n), vv = __ldg(a.v + n), vw = __ldg(a.w + n);
+  const double b0 = a.bmat[(size_t)(l * 3 + 0) * ne + e];
+  const double b1 = a.bmat[(size_t)(l * 3 + 1) * ne + e];
+  const double b2 = a.bmat[(size_t)(l * 3 + 2) * ne + e];
+  const double den = a.den[e], pres = a.pres[e], sspd = a.sspd[e], vol = a.vol[e], div = a.div[e];
+  const double* q = a.qtab + 4 * a.mat[e];
+  const bool compress = is_negative(div);
+  const double qa = compress ? q[0] : q[1], qb = compress ? q[2] : q[3];
+  // the limiter's neighbours, eight at a time
+  const int k0 = a.eie_start[e], k1 = a.eie_start[e + 1];
+  long long kmin = 0x7FFFFFFFFFFFFFFFLL, kmax = (long long)0x8000000000000000ULL;
+  for (int k = k0 + l; k < k1; k += 8) {
+    const long long key = okey(__ldg(a.div + __ldg(a.eie + k)));
+    kmin = key < kmin ? key : kmin;
+    kmax = key > kmax ? key : kmax;
+  }
+  __syncwarp();
+  kmin = group_min(kmin);
+  kmax = ~group_min(~kmax);
+  sv[0][l] = vu;
+  sv[1][l] = vv;
+  sv[2][l] = vw;
+  __syncwarp();
+  // lane r sums component r (lane 3: mu); the others repeat lane 3
+  const int r = l < 3 ? l : 3, c = l < 3 ? l : 2;
+  double vs = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) vs = fma(0.125, sv[c][k], vs);
+  const double vs0 = from_lane(vs, 0), vs1 = from_lane(vs, 1), vs2 = from_lane(vs, 2);
+  const Impedance z = impedance(den, sspd, qa, qb);
+  const double mu = corner_impedance(z, vu - vs0, vv - vs1, vw - vs2, b0, b1, b2);
+  __syncwarp();
+#if FIERRO_FMA
+  sv[3][l] = mu;
+  __syncwarp();
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = fma(sv[3][k], l < 3 ? sv[c][k] : 1.0, s);
+#else
+  sv[0][l] = mu * vu;
+  sv[1][l] = mu * vv;
+  sv[2][l] = mu * vw;
+  sv[3][l] = mu;
+  __syncwarp();
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = s + sv[r][k];
+#endif
+  const double s3 = from_lane(s, 3);
+  double vstar = 0.0;
+  if (s3 > a.fuzz) {
+#if FIERRO_FMA
+    vstar = s * mode_rcp(s3);
+#else
+    vstar = quot(s, divisor(s3));
+#endif
+  }
+  __syncwarp();
+  const double vstar0 = from_lane(vstar, 0), vstar1 = from_lane(vstar, 1), vstar2 = from_lane(vstar, 2);
+  const double r_min = limiter_min(a, div, k0, k1, kmin, kmax);
+  const double phi = mach_switch(vol, div, sspd, a.fuzz) * (1.0 - at_least_0(r_min));
+  const double pm = phi * mu;
+  if (!live) return;
+  a.force[(size_t)(l * 3 + 0) * ne + e] = mul_mul(b0, pres, pm, vstar0 - vu);
+  a.force[(size_t)(l * 3 + 1) * ne + e] = mul_mul(b1, pres, pm, vstar1 - vv);
+  a.force[(size_t)(l * 3 + 2) * ne + e] = mul_mul(b2, pres, pm, vstar2 - vw);
+}
+
+// ---------------------------------------------------------------------------
+// One component of one node per thread (blockIdx.y the component).
+__global__ void __launch_bounds__(kNodeBlock) k_node_lanes(const NodeArgs a) {
+  if (!a.ctrl->active) return;
+  const int n = blockIdx.x * blockDim.x + threadIdx.x, d = blockIdx.y;
+  if (n >= a.nn) return;
+  const size_t ne = (size_t)a.ne;
+  const int c0 = a.cin_start[n], c1 = a.cin_start[n + 1];
+  double f = 0.0;
+  for (int base = c0; base < c1; base += 8) {
+    double g[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int cid = base + k < c1 ? __ldg(a.cin + base + k) : 0;
+      g[k] = base + k < c1 ? __ldg(a.force + (size_t)((cid & 7) * 3 + d) * ne + (cid >> 3)) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (base + k < c1) f = f + g[k];
+  }
+  const double adt = a.rk_alpha * a.ctrl->dt;
+  const double v0 = (d == 0 ? a.u0 : d == 1 ? a.v0 : a.w0)[n];
+#if FIERRO_FMA
+  const double adt_rm = adt * (a.node_rm ? a.node_rm[n] : 1.0 / a.node_mass[n]);
+  double v1 = fma(adt_rm, f, v0);
+#else
+  double v1 = v0 + quot(adt * f, divisor(a.node_mass[n]));
+#endif
+  if (a.bc_mask[n] & (1u << d)) v1 = 0.0;
+  const double h = (v1 + v0) * 0.5;
+  (d == 0 ? a.u1 : d == 1 ? a.v1 : a.w1)[n] = v1;
+  (d == 0 ? a.hx : d == 1 ? a.hy : a.hz)[n] = h;
+  (d == 0 ? a.x1 : d == 1 ? a.y1 : a.z1)[n] = mul_add((d == 0 ? a.x0 : d == 1 ? a.y0 : a.z0)[n], adt, h);
+}
+
+// ---------------------------------------------------------------------------
+// Element update (KIND as in elem_tile), one CFL partial per warp.  Shared memory
+// per element, doubles: coordinates x, y, z by node; the 18 combos of each
+// component; the ordered sums' terms -- power (24), the velocity sums (8 each),
+// the volume (8) -- as products (exact) or factor pairs (FMA).
+constexpr int kChain = 24 + 4 * 8;
+struct LaneElem {
+  double x[3][8];
+  double combo[3][18];
+  double pr[8][7];  // a lane's products of the first component
+  double p[kChain];
+#if FIERRO_FMA
+  double q[kChain];
+#endif
+  float f[3][8];
+  double pad;
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kLaneBlock) k_elem_lanes(const ElemArgs a) {
+  __shared__ LaneElem s_e[kLaneWarps][kGroups];
+  if (KIND != 2 && !a.ctrl->active) return;
+  const int t = blockIdx.x * kLaneBlock + threadIdx.x;
+  const int lane = threadIdx.x & 31, l = lane & 7, ne = a.ne;
+  if ((t & ~31) >= 8 * ne) return;
+  const bool live = (t >> 3) < ne;
+  const int e = live ? t >> 3 : ne - 1;
+  LaneElem& s = s_e[threadIdx.x >> 5][lane >> 3];
+  const int n = __ldg(a.nie + 8 * (size_t)e + l);
+  const double x[3] = {__ldg(a.x + n), __ldg(a.y + n), __ldg(a.z + n)};
+  const double v[3] = {__ldg(a.u + n), __ldg(a.v + n), __ldg(a.w + n)};
+  double fc[3] = {0.0, 0.0, 0.0}, h[3] = {0.0, 0.0, 0.0};
+  if (KIND != 2) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) fc[d] = a.force[(size_t)(l * 3 + d) * ne + e];
+    h[0] = __ldg(a.hx + n);
+    h[1] = __ldg(a.hy + n);
+    h[2] = __ldg(a.hz + n);
+  }
+  const double mass = KIND != 2 ? a.mass[e] : 0.0, sie0 = KIND != 2 ? a.sie0[e] : 0.0;
+  const double gamma = KIND != 2 ? a.gamma[e] : 0.0, csmin = KIND != 2 ? a.csmin[e] : 0.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) s.x[d][l] = x[d];
+  __syncwarp();
+  // the combos: 36 two-term and 18 four-term ones over eight lanes
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const int task = l + 8 * i;
+    if (task < 36) {
+      const int c = task / 12, m = task - 12 * c;
+      const double* I = s.x[c == 0 ? 2 : c - 1];
+      const unsigned w = (unsigned)(m < 10 ? kLane.two[0] >> (6 * m) : kLane.two[1] >> (6 * (m - 10)));
+      s.combo[c][m] = I[w & 7] - I[(w >> 3) & 7];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int task = l + 8 * i;
+    if (task < 18) {
+      const int c = task / 6, m = task - 6 * c;
+      const double* I = s.x[c == 0 ? 2 : c - 1];
+      const unsigned w = (unsigned)(m < 4 ? kLane.four[0] >> (16 * m) : kLane.four[1] >> (16 * (m - 4)));
+      double v4 = flip(I[w & 7], (w >> 3) & 1);
+#pragma unroll
+      for (int k = 1; k < 4; ++k) v4 = v4 + flip(I[(w >> (4 * k)) & 7], (w >> (4 * k + 3)) & 1);
+      s.combo[c][12 + m] = v4;
+    }
+  }
+  __syncwarp();
+  // this corner's normals
+  const double twelth = 1. / 12.;
+  const unsigned long long row = by_lane(l, kLane.row[0], kLane.row[1], kLane.row[2], kLane.row[3], kLane.row[4],
+                                         kLane.row[5], kLane.row[6], kLane.row[7]);
+  const unsigned vorder = (unsigned)by_lane(l, kLane.vol[0], kLane.vol[1], kLane.vol[2], kLane.vol[3], kLane.vol[4],
+                                            kLane.vol[5], kLane.vol[6], kLane.vol[7]);
+  double b[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double* O = s.x[c == 2 ? 0 : c + 1];
+    double o[6], cm[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const unsigned w = (unsigned)(row >> (9 * k));
+      o[k] = O[w & 7];
+      cm[k] = flip(s.combo[c][(w >> 3) & 31], (w >> 8) & 1);
+    }
+    double sum;
+    if (c == 0) {
+      double pr[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s.pr[l][k] = pr[k] = FX_MUL(o[k], cm[k]);
+      sum = ((((pr[0] + pr[1]) + pr[2]) + pr[3]) + pr[4]) + pr[5];
+      double sv = s.pr[l][vorder & 7];
+#pragma unroll
+      for (int k = 1; k < 6; ++k) sv = FX_ADD(sv, s.pr[l][(vorder >> (3 * k)) & 7]);
+      const int at = 48 + (int)(vorder >> 18);
+      s.p[at] = FX_MUL(x[0], sv);
+#if FIERRO_FMA
+      s.q[at] = 1.0;
+#endif
+    } else {
+      sum = mul_mul(o[0], cm[0], o[1], cm[1]);
+#pragma unroll
+      for (int k = 2; k < 6; ++k) sum = mul_add(sum, o[k], cm[k]);
+    }
+    b[c] = sum * twelth;
+    if (live) a.bmat[(size_t)(l * 3 + c) * ne + e] = b[c];
+    // terms of the velocity sums and the power, in the sums' order (the fused sums
+    // begin with the second corner's product, as mul_mul does)
+#if FIERRO_FMA
+    const int at = 24 + 8 * c + (l < 2 ? 1 - l : l);
+    s.p[at] = v[c];
+    s.q[at] = b[c];
+    s.p[3 * l + c] = fc[c];
+    s.q[3 * l + c] = h[c];
+#else
+    s.p[24 + 8 * c + l] = v[c] * b[c];
+    s.p[3 * l + c] = fc[c] * h[c];
+#endif
+  }
+  __syncwarp();
+  // lanes 0-2: the velocity sums; 3: the volume; 4: the power (24 terms); the rest repeat the volume
+  double acc = 0.0;
+  const int at = l < 3 ? 24 + 8 * l : l == 4 ? 0 : 48;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+#if FIERRO_FMA
+    acc = fma(s.p[at + k], s.q[at + k], acc);
+#else
+    acc = acc + s.p[at + k];
+#endif
+  }
+  if (KIND != 2) {
+    double pw = acc;
+#pragma unroll
+    for (int k = 8; k < 24; ++k) {
+#if FIERRO_FMA
+      pw = fma(s.p[k], s.q[k], pw);
+#else
+      pw = pw + s.p[k];
+#endif
+    }
+    if (l == 4) acc = pw;
+  }
+  const double Sx = from_lane(acc, 0), Sy = from_lane(acc, 1), Sz = from_lane(acc, 2);
+  const double vol_geo = FX_MUL(from_lane(acc, 3), twelth);
+  const double power = from_lane(acc, 4);
+  const double vol = (KIND == 2) ? a.vol[e] : vol_geo;
+  const double div = divergence(Sx, Sy, Sz, vol);
+  double sspd;
+  const bool writer = live && l == 0;
+  if (KIND != 2) {
+    const double adt = a.rk_alpha * a.ctrl->dt;
+    const double sie1 = sie0 - FX_MUL(mode_div(adt, mass), power);
+    const double den = mode_div(mass, vol);
+    const double pres = (gamma - 1.0) * sie1 * den;
+    sspd = mode_sqrt(gamma * (gamma - 1.0) * sie1);
+    if (sspd < csmin) sspd = csmin;
+    if (writer) {
+      a.sie1[e] = sie1;
+      a.vol[e] = vol;
+      a.den[e] = den;
+      a.pres[e] = pres;
+      a.sspd[e] = sspd;
+      if (__double_as_longlong(vol) <= 0 || !is_finite(vol)) atomicOr(&a.ctrl->status, FIERRO_STATUS_BAD_VOLUME);
+      if (!is_finite(sie1) || !is_finite(pres)) atomicOr(&a.ctrl->status, FIERRO_STATUS_BAD_STATE);
+    }
+  } else {
+    sspd = a.sspd[e];
+  }
+  if (writer) a.div[e] = div;
+  if (KIND != 0) {
+    // the CFL length: each lane screens every eighth of the 28 pairs in single
+    // precision (sgh_cfl.cuh's bound) and evaluates the ones left in FP64
+    bool ok = true;
+    float M = 0.0f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float im = cfl::image(x[d], ok);
+      s.f[d][l] = im;
+      M = fmaxf(M, fabsf(im));
+    }
+    __syncwarp();
+    for (int o = 4; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, o));
+    const unsigned bad = __ballot_sync(0xFFFFFFFFu, !ok) >> (lane & 24) & 0xFFu;
+    const bool screen = bad == 0 && M >= 9.5367431640625e-07f;
+    float e2[4], e2min = 3.0e38f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = l + 8 * i;
+      const int pa = cfl::pair_a(k < 28 ? k : l), pb = cfl::pair_b(k < 28 ? k : l);
+      const float dx = s.f[0][pb] - s.f[0][pa], dy = s.f[1][pb] - s.f[1][pa], dz = s.f[2][pb] - s.f[2][pa];
+      e2[i] = (dx * dx + dy * dy) + dz * dz;
+      e2min = fminf(e2min, e2[i]);
+    }
+    for (int o = 4; o > 0; o >>= 1) e2min = fminf(e2min, __shfl_xor_sync(0xFFFFFFFFu, e2min, o));
+    const float T2 = cfl::screen_limit(e2min, M);
+    unsigned mask = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (l + 8 * i < 28 && (!screen || e2[i] <= T2)) mask |= 1u << i;
+    long long kd = 0x7FFFFFFFFFFFFFFFLL;
+    while (mask) {
+      const int k = l + 8 * (__ffs((int)mask) - 1);
+      mask &= mask - 1;
+      const long long key = cfl::key_of(cfl::exact_d2(s.x[0], s.x[1], s.x[2], cfl::pair_a(k), cfl::pair_b(k)));
+      kd = key < kd ? key : kd;
+    }
+    __syncwarp();
+    kd = group_min(kd);
+    long long dkey = 0x7FFFFFFFFFFFFFFFLL;
+    if (live) dkey = cfl_key(cfl::key_decode(kd), sspd, a.dt_cfl, a.fuzz);
+    __syncwarp();
+    for (int o = 16; o > 4; o >>= 1) {
+      const long long tk = __shfl_xor_sync(0xFFFFFFFFu, dkey, o);
+      dkey = tk < dkey ? tk : dkey;
+    }
+    if (lane == 0) a.cfl_part[t >> 5] = dkey;
+  }
+}

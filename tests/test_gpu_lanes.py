@@ -1,0 +1,71 @@
+"""The lane passes of small meshes (sgh_lanes.cuh): bit for bit the
+one-thread-per-element passes, which a batch of one instance runs, in both
+modes, at element counts around a warp's four, around the sizes where the
+force, element and node passes change over, and on a checkpoint between them."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# 1, 3, 4, 5, 27, 315 elements; 9000 | 9009 (element pass), 10500 | 10520 (force
+# pass), 27 x 30 x 33 elements on 29,512 nodes and 29 x 31 x 31 on 30,720 (node pass)
+SHAPES = [(1, 1, 1), (3, 1, 1), (2, 2, 1), (5, 1, 1), (3, 3, 3), (7, 9, 5), (20, 18, 25), (21, 13, 33), (20, 21, 25),
+          (20, 2, 263), (27, 30, 33), (29, 31, 31)]
+
+
+def _deck(shape, cycles=12):
+    from fierro_gb300 import mesh, problems
+    m = mesh.box_mesh(*shape, length=(1.0, 1.1, 0.9), jitter=0.15, seed=sum(shape), permute=True)
+    p = problems.noh(max(shape), mesh=m, cycles=cycles)
+    p.materials[0].q2ex = 0.4
+    p.fills[0].sie = 0.02
+    return p
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("mode", [0, 1])
+def test_lanes_equal_the_batch(lib_built, shape, mode):
+    from fierro_gb300 import sgh
+    p = _deck(shape)
+    st = sgh.setup(p)
+    with sgh.Batch([p], fp_mode=mode) as b:
+        b.set_state(0, st)
+        b.run(12)
+        want, wt = b.get_state(0), b.time(0)
+    with sgh.SGHSolver(p, fp_mode=mode) as s:
+        s.set_state(st)
+        s.run(12)
+        got, gt = s.get_state(), s.time()
+    assert (gt[0], gt[1], gt[3]) == wt
+    for k in ("node_coords", "node_vel", "elem_den", "elem_pres", "elem_sspd", "elem_sie", "elem_vol", "elem_div",
+              "corner_force"):
+        assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("shape", [(5, 1, 1), (7, 9, 5), (21, 13, 33)])
+def test_checkpoint_of_a_lane_handle(lib_built, tmp_path, shape):
+    """The file holds one CFL partial per element block, as it always has, and a
+    restart from it takes the same time steps."""
+    import struct
+
+    from fierro_gb300 import sgh
+    p = _deck(shape)
+    path = str(tmp_path / "a.ckpt")
+    with sgh.SGHSolver(p) as a:
+        a.set_state(sgh.setup(p))
+        a.run(5)
+        a.checkpoint(path)
+        a.run(7)
+        want, wt = a.get_state(), a.time()
+    ne, block = p.mesh.num_elems, 128
+    while block > 32 and -(-ne // block) < 304:
+        block //= 2
+    head = struct.unpack_from("<8sII10q", open(path, "rb").read(), 0)
+    assert head[3:5] == (p.mesh.num_nodes, ne) and head[-1] == -(-ne // block)
+    with sgh.SGHSolver(p) as b:
+        b.restart(path)
+        b.run(7)
+        got, gt = b.get_state(), b.time()
+    assert gt == wt
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
