@@ -85,18 +85,17 @@ namespace FIERRO_IMPL {
 
 constexpr int kNodeGather = FIERRO_NODE_GATHER;
 
-// Loads of values an earlier phase of the same launch wrote (the batch's fused
-// stage kernel, COH): from L2 (ld.global.cg), never from a line another phase
-// left in this SM's L1.  Otherwise the read-only path (__ldg) or a plain load.
-template <bool COH>
-__device__ __forceinline__ double ld_ro(const double* p) {
-  return COH ? __ldcg(p) : __ldg(p);
-}
+// Loads of state.  Values an earlier phase of the same launch wrote (the batch's
+// fused stage kernel, COH): from L2 (ld.global.cg), never from a line another
+// phase left in this SM's L1.  Otherwise a plain load; the read-only path
+// (__ldg) is for the mesh's index lists alone, as a launch may begin before the
+// launch that writes its inputs has ended (sgh_launch.cuh).
 template <bool COH>
 __device__ __forceinline__ double ld_pl(const double* p) {
   return COH ? __ldcg(p) : *p;
 }
 
+#include "sgh_launch.cuh"
 #include "sgh_common.cuh"
 #include "sgh_hex_geometry.cuh"
 #include "sgh_cfl.cuh"
@@ -171,7 +170,7 @@ __device__ __forceinline__ double limiter_min(const ForceArgs& a, double div, in
       r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
     } else {
       for (int k = k0; k < k1; ++k) {
-        const double r_face = newton_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + a.small), D);
+        const double r_face = newton_div(0.9 * (a.div[__ldg(a.eie + k)] + a.small), D);
         r_min = fmin(r_face, r_min);
       }
     }
@@ -222,9 +221,9 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
   double vu[8], vv[8], vw[8];
 #pragma unroll
   for (int l = 0; l < 8; ++l) {
-    vu[l] = __ldg(a.u + nid[l]);
-    vv[l] = __ldg(a.v + nid[l]);
-    vw[l] = __ldg(a.w + nid[l]);
+    vu[l] = a.u[nid[l]];
+    vv[l] = a.v[nid[l]];
+    vw[l] = a.w[nid[l]];
   }
   const double den = a.den[e], pres = a.pres[e], sspd = a.sspd[e], vol = a.vol[e], div = a.div[e];
   const int mat = a.mat[e];
@@ -279,7 +278,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
   const int k0 = a.eie_start[e], k1 = a.eie_start[e + 1];
   long long kmin = 0x7FFFFFFFFFFFFFFFLL, kmax = (long long)0x8000000000000000ULL;
   for (int k = k0; k < k1; ++k) {
-    const long long key = okey(__ldg(a.div + __ldg(a.eie + k)));
+    const long long key = okey(a.div[__ldg(a.eie + k)]);
     kmin = key < kmin ? key : kmin;
     kmax = key > kmax ? key : kmax;
   }
@@ -303,7 +302,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
       const long long ksel = D > 0 ? kmin : kmax;
       for (int k = k0; k < k1; ++k) {
         const int nb = __ldg(a.eie + k);
-        if (okey(__ldg(a.div + nb)) == ksel) {
+        if (okey(a.div[nb]) == ksel) {
           sel = nb;
           break;
         }
@@ -322,7 +321,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     } else if (lim == FIERRO_LIM_FULL) {
       phi = 1.0;
     } else if (lim == FIERRO_LIM_FACE && a.br_sel[e] >= 0) {
-      phi = 1.0 - newton_div(0.9 * (__ldg(a.div + a.br_sel[e]) + small), D);
+      phi = 1.0 - newton_div(0.9 * (a.div[a.br_sel[e]] + small), D);
     }  // FIERRO_LIM_IRREGULAR: as evaluated above
   }
   if (TAPE) {
@@ -347,7 +346,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     if (k1 > k0 && isfinite(D) && D != 0.0 && isfinite(okey_decode(ksel)) && r_min < 1.0 && r_min > 0.0) {
       for (int k = k0; k < k1; ++k) {
         const int nb = __ldg(a.eie + k);
-        if (okey(__ldg(a.div + nb)) == ksel) {
+        if (okey(a.div[nb]) == ksel) {
           sel = nb;
           break;
         }
@@ -414,6 +413,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
 // that strides over the elements.
 template <bool BATCH, bool TAPE, bool STRENGTH, int BR = 0>
 __global__ void FIERRO_FORCE_BOUNDS k_force(const ForceArgs a) {
+  previous_launch_done();
   if (BATCH) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.ne; e += gridDim.x * blockDim.x)
       force_elem<true, TAPE, STRENGTH, BR>(a, e);
@@ -447,7 +447,7 @@ __device__ __forceinline__ void node_update(const NodeArgs& a, const int n) {
     for (int k = 0; k < kNodeGather; ++k) {
       const int e = cid[k] >> 3, l = cid[k] & 7;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) g[k][d] = k < cnt ? ld_ro<COH>(a.force + (size_t)(l * 3 + d) * ne + e) : 0.0;
+      for (int d = 0; d < 3; ++d) g[k][d] = k < cnt ? ld_pl<COH>(a.force + (size_t)(l * 3 + d) * ne + e) : 0.0;
     }
 #pragma unroll
     for (int k = 0; k < kNodeGather; ++k)
@@ -491,6 +491,7 @@ __device__ __forceinline__ void node_update(const NodeArgs& a, const int n) {
 // One thread per node; a batch may run as a persistent grid striding over the nodes.
 template <bool BATCH>
 __global__ void __launch_bounds__(kNodeBlock) k_node(const NodeArgs a) {
+  previous_launch_done();
   if (BATCH) {
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < a.nn; n += gridDim.x * blockDim.x)
       node_update<true>(a, n);
@@ -529,12 +530,12 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
     double x[8], y[8], z[8], u[8], v[8], w[8];
 #pragma unroll
     for (int l = 0; l < 8; ++l) {
-      x[l] = ld_ro<COH>(a.x + nid[l]);
-      y[l] = ld_ro<COH>(a.y + nid[l]);
-      z[l] = ld_ro<COH>(a.z + nid[l]);
-      u[l] = ld_ro<COH>(a.u + nid[l]);
-      v[l] = ld_ro<COH>(a.v + nid[l]);
-      w[l] = ld_ro<COH>(a.w + nid[l]);
+      x[l] = ld_pl<COH>(a.x + nid[l]);
+      y[l] = ld_pl<COH>(a.y + nid[l]);
+      z[l] = ld_pl<COH>(a.z + nid[l]);
+      u[l] = ld_pl<COH>(a.u + nid[l]);
+      v[l] = ld_pl<COH>(a.v + nid[l]);
+      w[l] = ld_pl<COH>(a.w + nid[l]);
     }
     double sie1 = 0.0;
     if (KIND != 2) {
@@ -542,9 +543,9 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
       double power = 0.0;
 #pragma unroll
       for (int l = 0; l < 8; ++l) {
-        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 0) * ne + e), ld_ro<COH>(a.hx + nid[l]));
-        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 1) * ne + e), ld_ro<COH>(a.hy + nid[l]));
-        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 2) * ne + e), ld_ro<COH>(a.hz + nid[l]));
+        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 0) * ne + e), ld_pl<COH>(a.hx + nid[l]));
+        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 1) * ne + e), ld_pl<COH>(a.hy + nid[l]));
+        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 2) * ne + e), ld_pl<COH>(a.hz + nid[l]));
       }
       const double adt = a.rk_alpha * ctrl->dt;
       sie1 = a.sie0[e] - FX_MUL(mode_div(adt, a.mass[e]), power);  // not fused: sie1 may cancel sie0
@@ -616,6 +617,7 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
 // tiles (a barrier between tiles, as the CFL reduction reuses shared memory).
 template <int KIND, bool BATCH, bool STRENGTH>
 __global__ void FIERRO_ELEM_BOUNDS k_elem(const ElemArgs a) {
+  previous_launch_done();
   if (BATCH) {
     const int ntiles = (a.ne + blockDim.x - 1) / blockDim.x;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -706,6 +708,7 @@ __device__ __forceinline__ void dt_update(Ctrl* c, long long k, const LoopParams
 }
 
 __global__ void __launch_bounds__(1024) k_dt(const DtArgs a) {
+  previous_launch_done();
   long long k = 0x7FFFFFFFFFFFFFFFLL;
   for (int i = threadIdx.x; i < a.nparts; i += blockDim.x) {
     const long long t = a.cfl_part[i];
@@ -718,6 +721,7 @@ __global__ void __launch_bounds__(1024) k_dt(const DtArgs a) {
 // One block per instance: instance i's CFL partials are cfl_part[part_start[i] ..
 // part_start[i+1]).
 __global__ void __launch_bounds__(256) k_dt_batch(const DtArgs a) {
+  previous_launch_done();
   const int i = blockIdx.x;
   long long k = 0x7FFFFFFFFFFFFFFFLL;
   for (int j = a.part_start[i] + threadIdx.x; j < a.part_start[i + 1]; j += blockDim.x) {
@@ -745,9 +749,13 @@ __device__ __forceinline__ void end_update(Ctrl* c, const LoopParams& lp) {
   c->active = 0;
 }
 
-__global__ void k_end(Ctrl* c, const LoopParams lp) { end_update(c, lp); }
+__global__ void k_end(Ctrl* c, const LoopParams lp) {
+  previous_launch_done();
+  end_update(c, lp);
+}
 
 __global__ void k_end_batch(Ctrl* c, const LoopParams* lps, int ninst) {
+  previous_launch_done();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < ninst) end_update(c + i, lps[i]);
 }
@@ -808,42 +816,42 @@ static unsigned grid_or(int grid, unsigned blocks) {
 static void launch_force(const ForceArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);
   const unsigned g = blocks_for(a.ne, bs);
-  if (a.lanes) k_force_lanes<<<blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, 0, s>>>(a);
-  else if (a.inst) k_force<true, false, false><<<grid_or(a.grid, g), bs, 0, s>>>(a);
-  else if (a.stress_out) k_force<false, false, true><<<g, bs, 0, s>>>(a);
-  else k_force<false, false, false><<<g, bs, 0, s>>>(a);
+  if (a.lanes) launch(k_force_lanes, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
+  else if (a.inst) launch(k_force<true, false, false>, grid_or(a.grid, g), bs, s, a);
+  else if (a.stress_out) launch(k_force<false, false, true>, g, bs, s, a);
+  else launch(k_force<false, false, false>, g, bs, s, a);
 }
 static void launch_force_tape(const ForceArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);
-  k_force<false, true, false><<<blocks_for(a.ne, bs), bs, 0, s>>>(a);
+  launch(k_force<false, true, false>, blocks_for(a.ne, bs), bs, s, a);
 }
 static void launch_force_branch(const ForceArgs& a, int mode, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);
-  if (mode == 1) k_force<false, false, false, 1><<<blocks_for(a.ne, bs), bs, 0, s>>>(a);
-  else k_force<false, false, false, 2><<<blocks_for(a.ne, bs), bs, 0, s>>>(a);
+  if (mode == 1) launch(k_force<false, false, false, 1>, blocks_for(a.ne, bs), bs, s, a);
+  else launch(k_force<false, false, false, 2>, blocks_for(a.ne, bs), bs, s, a);
 }
 static void launch_node(const NodeArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kNodeBlock);
   if (a.lanes) {
     const int b = small_mesh_block(3LL * a.nn, kNodeBlock);
-    k_node_lanes<<<dim3(blocks_for(a.nn, b), 3), b, 0, s>>>(a);
-  } else if (a.inst) k_node<true><<<grid_or(a.grid, blocks_for(a.nn, bs)), bs, 0, s>>>(a);
-  else k_node<false><<<blocks_for(a.nn, bs), bs, 0, s>>>(a);
+    launch(k_node_lanes, dim3(blocks_for(a.nn, b), 3), b, s, a);
+  } else if (a.inst) launch(k_node<true>, grid_or(a.grid, blocks_for(a.nn, bs)), bs, s, a);
+  else launch(k_node<false>, blocks_for(a.nn, bs), bs, s, a);
 }
 template <bool B, bool S>
 static void launch_elem_t(const ElemArgs& a, int kind, cudaStream_t s) {
   const int bs = block_or(a.block, kElemBlock);
   const unsigned g = B ? grid_or(a.grid, blocks_for(a.ne, bs)) : blocks_for(a.ne, bs);
-  if (kind == 0) k_elem<0, B, S><<<g, bs, 0, s>>>(a);
-  else if (kind == 1) k_elem<1, B, S><<<g, bs, 0, s>>>(a);
-  else k_elem<2, B, false><<<g, bs, 0, s>>>(a);
+  if (kind == 0) launch(k_elem<0, B, S>, g, bs, s, a);
+  else if (kind == 1) launch(k_elem<1, B, S>, g, bs, s, a);
+  else launch(k_elem<2, B, false>, g, bs, s, a);
 }
 static void launch_elem(const ElemArgs& a, int kind, cudaStream_t s) {
   if (a.lanes) {
     const unsigned g = blocks_for(8LL * a.ne, kLaneBlock);
-    if (kind == 0) k_elem_lanes<0><<<g, kLaneBlock, 0, s>>>(a);
-    else if (kind == 1) k_elem_lanes<1><<<g, kLaneBlock, 0, s>>>(a);
-    else k_elem_lanes<2><<<g, kLaneBlock, 0, s>>>(a);
+    if (kind == 0) launch(k_elem_lanes<0>, g, kLaneBlock, s, a);
+    else if (kind == 1) launch(k_elem_lanes<1>, g, kLaneBlock, s, a);
+    else launch(k_elem_lanes<2>, g, kLaneBlock, s, a);
     return;
   }
   if (a.inst) launch_elem_t<true, false>(a, kind, s);
@@ -852,12 +860,12 @@ static void launch_elem(const ElemArgs& a, int kind, cudaStream_t s) {
 }
 static_assert(kLaneTile == kGroups, "one CFL partial per warp of the lane passes");
 static void launch_dt(const DtArgs& a, cudaStream_t s) {
-  if (a.part_start) k_dt_batch<<<a.ninst, 256, 0, s>>>(a);
-  else k_dt<<<1, 1024, 0, s>>>(a);
+  if (a.part_start) launch(k_dt_batch, a.ninst, 256, s, a);
+  else launch(k_dt, 1, 1024, s, a);
 }
-static void launch_end(Ctrl* c, const LoopParams& lp, cudaStream_t s) { k_end<<<1, 1, 0, s>>>(c, lp); }
+static void launch_end(Ctrl* c, const LoopParams& lp, cudaStream_t s) { launch(k_end, 1, 1, s, c, lp); }
 static void launch_end_batch(Ctrl* c, const LoopParams* lps, int ninst, cudaStream_t s) {
-  k_end_batch<<<blocks_for(ninst, 128), 128, 0, s>>>(c, lps, ninst);
+  launch(k_end_batch, blocks_for(ninst, 128), 128, s, c, lps, ninst);
 }
 static int batch_max_blocks(int kernel, int block) {
   int n = 0;

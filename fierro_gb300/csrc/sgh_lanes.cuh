@@ -115,15 +115,16 @@ constexpr int kGroups = 4;                   // elements per warp
 __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   // per element: the corners' velocities and impedance terms, rows u, v, w, mu
   __shared__ double s_v[kLaneWarps][kGroups][4][9];
-  if (!a.ctrl->active) return;
   const int t = blockIdx.x * kLaneBlock + threadIdx.x;
   const int lane = threadIdx.x & 31, l = lane & 7, ne = a.ne;
-  if ((t & ~31) >= 8 * ne) return;  // whole warps past the end
   const bool live = (t >> 3) < ne;
   const int e = live ? t >> 3 : ne - 1;
   double(*sv)[9] = s_v[threadIdx.x >> 5][lane >> 3];
-  const int n = __ldg(a.nie + 8 * (size_t)e + l);
-  const double vu = __ldg(a.u + n), vv = __ldg(a.v + n), vw = __ldg(a.w + n);
+  const int n = __ldg(a.nie + 8 * (size_t)e + l);  // the mesh does not change: before the wait
+  const int k0 = __ldg(a.eie_start + e), k1 = __ldg(a.eie_start + e + 1);
+  previous_launch_done();
+  if (!a.ctrl->active || (t & ~31) >= 8 * ne) return;  // whole warps past the end
+  const double vu = a.u[n], vv = a.v[n], vw = a.w[n];
   const double b0 = a.bmat[(size_t)(l * 3 + 0) * ne + e];
   const double b1 = a.bmat[(size_t)(l * 3 + 1) * ne + e];
   const double b2 = a.bmat[(size_t)(l * 3 + 2) * ne + e];
@@ -132,10 +133,9 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   const bool compress = is_negative(div);
   const double qa = compress ? q[0] : q[1], qb = compress ? q[2] : q[3];
   // the limiter's neighbours, eight at a time
-  const int k0 = a.eie_start[e], k1 = a.eie_start[e + 1];
   long long kmin = 0x7FFFFFFFFFFFFFFFLL, kmax = (long long)0x8000000000000000ULL;
   for (int k = k0 + l; k < k1; k += 8) {
-    const long long key = okey(__ldg(a.div + __ldg(a.eie + k)));
+    const long long key = okey(a.div[__ldg(a.eie + k)]);
     kmin = key < kmin ? key : kmin;
     kmax = key > kmax ? key : kmax;
   }
@@ -194,18 +194,19 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
 // ---------------------------------------------------------------------------
 // One component of one node per thread (blockIdx.y the component).
 __global__ void __launch_bounds__(kNodeBlock) k_node_lanes(const NodeArgs a) {
-  if (!a.ctrl->active) return;
   const int n = blockIdx.x * blockDim.x + threadIdx.x, d = blockIdx.y;
-  if (n >= a.nn) return;
+  const bool in = n < a.nn;
+  const int c0 = in ? __ldg(a.cin_start + n) : 0, c1 = in ? __ldg(a.cin_start + n + 1) : 0;
+  previous_launch_done();
+  if (!in || !a.ctrl->active) return;
   const size_t ne = (size_t)a.ne;
-  const int c0 = a.cin_start[n], c1 = a.cin_start[n + 1];
   double f = 0.0;
   for (int base = c0; base < c1; base += 8) {
     double g[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int cid = base + k < c1 ? __ldg(a.cin + base + k) : 0;
-      g[k] = base + k < c1 ? __ldg(a.force + (size_t)((cid & 7) * 3 + d) * ne + (cid >> 3)) : 0.0;
+      g[k] = base + k < c1 ? a.force[(size_t)((cid & 7) * 3 + d) * ne + (cid >> 3)] : 0.0;
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k)
@@ -247,23 +248,23 @@ struct LaneElem {
 template <int KIND>
 __global__ void __launch_bounds__(kLaneBlock) k_elem_lanes(const ElemArgs a) {
   __shared__ LaneElem s_e[kLaneWarps][kGroups];
-  if (KIND != 2 && !a.ctrl->active) return;
   const int t = blockIdx.x * kLaneBlock + threadIdx.x;
   const int lane = threadIdx.x & 31, l = lane & 7, ne = a.ne;
-  if ((t & ~31) >= 8 * ne) return;
   const bool live = (t >> 3) < ne;
   const int e = live ? t >> 3 : ne - 1;
   LaneElem& s = s_e[threadIdx.x >> 5][lane >> 3];
   const int n = __ldg(a.nie + 8 * (size_t)e + l);
-  const double x[3] = {__ldg(a.x + n), __ldg(a.y + n), __ldg(a.z + n)};
-  const double v[3] = {__ldg(a.u + n), __ldg(a.v + n), __ldg(a.w + n)};
+  previous_launch_done();
+  if ((KIND != 2 && !a.ctrl->active) || (t & ~31) >= 8 * ne) return;
+  const double x[3] = {a.x[n], a.y[n], a.z[n]};
+  const double v[3] = {a.u[n], a.v[n], a.w[n]};
   double fc[3] = {0.0, 0.0, 0.0}, h[3] = {0.0, 0.0, 0.0};
   if (KIND != 2) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) fc[d] = a.force[(size_t)(l * 3 + d) * ne + e];
-    h[0] = __ldg(a.hx + n);
-    h[1] = __ldg(a.hy + n);
-    h[2] = __ldg(a.hz + n);
+    h[0] = a.hx[n];
+    h[1] = a.hy[n];
+    h[2] = a.hz[n];
   }
   const double mass = KIND != 2 ? a.mass[e] : 0.0, sie0 = KIND != 2 ? a.sie0[e] : 0.0;
   const double gamma = KIND != 2 ? a.gamma[e] : 0.0, csmin = KIND != 2 ? a.csmin[e] : 0.0;
