@@ -403,8 +403,8 @@ static int create_impl(fierro_sgh* h, const fierro_mesh* mesh, const fierro_mate
   h->lanes_force = (long long)ne <= kLanesForce && !h->strength;
   h->lanes_node = (long long)nn <= kLanesNode;
   h->lanes_elem = (long long)ne <= kLanesElem && !h->has_hyper;
-  const size_t tile = h->lanes_elem ? kLaneTile : h->blk_elem;
-  h->ncfl = (int)((ne + tile - 1) / tile);
+  h->cfl_tile = h->lanes_elem ? kLaneTile : h->blk_elem;
+  h->ncfl = (int)((ne + h->cfl_tile - 1) / h->cfl_tile);
   TRY(dalloc(h, &h->d_cfl, (size_t)h->ncfl));
   TRY(dalloc(h, &h->d_ctrl, 1));
   TRY(dalloc(h, &h->d_node_ext2int, nn));
@@ -990,8 +990,8 @@ struct Block {
 };
 
 // The CFL partials a file holds, and how many of a handle's fall on each.
-int64_t ckpt_ncfl(const fierro_sgh* h) { return h->lanes_elem ? (h->ne + h->blk_elem - 1) / h->blk_elem : h->ncfl; }
-int64_t ckpt_cfl_group(const fierro_sgh* h) { return h->lanes_elem ? h->blk_elem / kLaneTile : 1; }
+int64_t ckpt_ncfl(const fierro_sgh* h) { return (h->ne + h->blk_elem - 1) / h->blk_elem; }
+int64_t ckpt_cfl_group(const fierro_sgh* h) { return h->blk_elem / h->cfl_tile; }
 
 uint64_t fnv1a(uint64_t h, const void* p, size_t n) {
   const unsigned char* c = static_cast<const unsigned char*>(p);

@@ -64,7 +64,8 @@ struct fierro_sgh {
   double* d_sie[2] = {};
   double *d_bmat = nullptr, *d_force = nullptr;
   long long* d_cfl = nullptr;
-  int ncfl = 0;  // CFL partials: one per element block
+  int ncfl = 0;  // CFL partials, one per cfl_tile elements (an element block, or a lane pass's warp)
+  int cfl_tile = fierro::kElemBlock;
   // threads per block of the element, force and node kernels (small_mesh_block)
   int blk_elem = fierro::kElemBlock, blk_force = fierro::kForceBlock, blk_node = fierro::kNodeBlock;
   bool lanes_force = false, lanes_node = false, lanes_elem = false;  // small meshes: sgh_lanes.cuh

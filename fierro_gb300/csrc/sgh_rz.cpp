@@ -351,7 +351,10 @@ int create(fierro_sgh* h, const fierro_mesh* mesh, const fierro_material* materi
   TRY(dalloc(h, &h->d_axis, t.axis_nodes.size()));
   TRY(dalloc(h, &h->d_axis_nin_start, t.axis_nin_start.size()));
   TRY(dalloc(h, &h->d_axis_nin, t.axis_nin.size()));
-  h->ncfl = (int)((ne + kElemBlock - 1) / kElemBlock);
+  h->lanes_force = (long long)ne <= kRzLanesForce && !h->strength;
+  h->lanes_elem = (long long)ne <= kRzLanesElem;
+  h->cfl_tile = h->lanes_elem ? kRzLaneTile : kElemBlock;
+  h->ncfl = (int)((ne + h->cfl_tile - 1) / h->cfl_tile);
   TRY(dalloc(h, &h->d_cfl, (size_t)h->ncfl));
   TRY(dalloc(h, &h->d_ctrl, 1));
   TRY(dalloc(h, &h->d_energy_part, 2 * 512));
@@ -468,6 +471,7 @@ static RzElemArgs elem_args_rz(fierro_sgh* h, int cur, int c, double alpha, int 
   a.rk_alpha = alpha;
   a.dt_cfl = h->lp.dt_cfl;
   a.fuzz = h->lp.fuzz;
+  a.lanes = h->lanes_elem;
   return a;
 }
 
@@ -553,6 +557,7 @@ int enqueue_stage(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k) {
     f.rk_alpha = alpha;
     f.copy_stress = s == 0;
   }
+  f.lanes = h->lanes_force;
   RzNodeArgs n{};
   n.nn = (int)h->nn;
   n.ne = (int)h->ne;

@@ -43,6 +43,7 @@ struct RzForceArgs {
   const double* sie0;
   double rk_alpha;
   int copy_stress;
+  int lanes;  // four lanes per element (small gas-only meshes, sgh_rz_lanes.cuh)
 };
 
 struct RzNodeArgs {
@@ -89,6 +90,7 @@ struct RzElemArgs {
   long long* cfl_part;
   Ctrl* ctrl;
   double rk_alpha, dt_cfl, fuzz;
+  int lanes;  // four lanes per element, one CFL partial per kRzLaneTile elements
 };
 
 struct RzEnergyArgs {
@@ -98,6 +100,16 @@ struct RzEnergyArgs {
   double* part;  // [2][nblocks]
   double* out;   // [2]
 };
+
+// Quad meshes of at most this many elements run the lane passes of
+// sgh_rz_lanes.cuh.  Per launch (events, us), one thread per element against four
+// lanes:           16^2         64^2         96^2         128^2        160^2
+//   force exact   16.3 / 10.5  16.4 / 12.3  16.4 / 14.5  16.6 / 20.5  18.8 / 28.8
+//   force FMA     14.5 / 10.3  14.2 / 10.3  14.4 / 12.9  14.5 / 16.5  16.6 / 24.4
+//   elem exact    11.6 /  8.8  12.0 / 10.2  11.9 / 12.3  12.1 / 16.5  15.9 / 22.6
+//   elem FMA      10.2 /  8.3  10.4 /  8.2  10.3 / 10.0  10.2 / 13.8  12.5 / 18.4
+constexpr long long kRzLanesForce = 11500, kRzLanesElem = 9000;
+constexpr int kRzLaneTile = 8;  // elements per warp of a lane pass
 
 struct RzKernelSet {
   void (*force)(const RzForceArgs&, cudaStream_t);

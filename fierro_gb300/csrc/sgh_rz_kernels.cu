@@ -40,7 +40,9 @@
 namespace fierro {
 namespace FIERRO_RZ_IMPL {
 
+#include "sgh_launch.cuh"
 #include "sgh_common.cuh"
+#include "sgh_hex_geometry.cuh"  // mul_add, mul_mul
 #include "sgh_user_mat.cuh"
 
 constexpr int kRzBlock = 128;
@@ -84,7 +86,9 @@ __device__ __forceinline__ void rz_bmatrix(const RzDiffs& d, double (&B)[4][2]) 
 }
 
 // get_area_quad (geometry.cpp:438-466)
-__device__ __forceinline__ double rz_area(const RzDiffs& d) { return 0.5 * (d.x02 * d.y13 + (-d.x13) * d.y02); }
+__device__ __forceinline__ double rz_area(const RzDiffs& d) {
+  return 0.5 * mul_mul(d.x02, d.y13, -d.x13, d.y02);
+}
 
 // v / 6, correctly rounded (the IEEE quotient in both modes): a quotient one
 // ulp off at most and one remainder step through the rounded reciprocal
@@ -97,8 +101,8 @@ __device__ __forceinline__ double sixth(double v) {
 
 // get_vol_quad (geometry.cpp:369-434): volume per radian of the revolved quad.
 __device__ __forceinline__ double rz_vol(const double (&y)[4], const RzDiffs& d) {
-  return sixth((y[2] + y[3] + y[0]) * (d.y23 * d.x03 - d.y03 * d.x23) +
-               (y[0] + y[1] + y[2]) * (d.y01 * d.x21 - d.y21 * d.x01));
+  return sixth(mul_mul(y[2] + y[3] + y[0], mul_mul(d.y23, d.x03, -d.y03, d.x23),  //
+                       y[0] + y[1] + y[2], mul_mul(d.y01, d.x21, -d.y21, d.x01)));
 }
 
 // heron (geometry.cpp:470-500)
@@ -155,10 +159,11 @@ __device__ __forceinline__ float f32_signed(double d) {
   const unsigned m = (unsigned)((b >> 29) & 0x7FFFFF), s = (unsigned)(b >> 32) & 0x80000000u;
   return __uint_as_float(s | (e <= 0 ? 0u : e >= 255 ? 0x7F800000u : ((unsigned)e << 23) | m));
 }
-__device__ __forceinline__ bool rz_corner_areas_finite(const RzDiffs& d) {
-  const float ax = 0.5f * f32_signed(-d.x02), bx = 0.5f * f32_signed(-d.x13);
-  const float ay = 0.5f * f32_signed(-d.y02), by = 0.5f * f32_signed(-d.y13);
-  const float mx = 0.25f * f32_signed(-d.x01 - d.x23), my = 0.25f * f32_signed(-d.y01 - d.y23);
+__device__ __forceinline__ bool rz_corner_areas_finite(double x02, double x13, double y02, double y13, double m_x,
+                                                       double m_y) {
+  const float ax = 0.5f * f32_signed(-x02), bx = 0.5f * f32_signed(-x13);
+  const float ay = 0.5f * f32_signed(-y02), by = 0.5f * f32_signed(-y13);
+  const float mx = 0.25f * f32_signed(m_x), my = 0.25f * f32_signed(m_y);
   const float px[4] = {-ax - mx, -bx + mx, ax - mx, bx + mx};
   const float py[4] = {-ay - my, -by + my, ay - my, by + my};
   bool ok = true;
@@ -182,6 +187,42 @@ __device__ __forceinline__ void gather4(const int* nie, int e, int (&nid)[4]) {
   nid[3] = q.w;
 }
 
+// The scalar steps the one-thread-per-element passes and the lane passes
+// (sgh_rz_lanes.cuh) share.  den (q1 c + q2 |v - v_avg|), force_sgh.cpp:520-636:
+__device__ __forceinline__ double rz_impedance(double den, double q1c, double qb, double d0, double d1) {
+  return den * mul_add(q1c, qb, mode_sqrt(mul_mul(d0, d0, d1, d1)));
+}
+// shock detector (:653-690): the minimum over neighbours of the monotone
+// r_face(div_nb) sits at the smallest (div + small > 0) or largest neighbour
+// divergence, as in the 3D kernel
+__device__ __forceinline__ double rz_limiter_min(const RzForceArgs& a, double div, int k0, int k1, long long kmin,
+                                                 long long kmax) {
+  const double D = div + a.small;
+  double r_min = 1.0;
+  if (k1 > k0) {
+    const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
+    if (is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel)) {
+      const double r_face = newton_div(0.9 * (dsel + a.small), D);
+      r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
+    } else {
+      for (int k = k0; k < k1; ++k) {
+        const double r_face = newton_div(0.9 * (a.div[__ldg(a.eie + k)] + a.small), D);
+        r_min = fmin(r_face, r_min);
+      }
+    }
+  }
+  return r_min;
+}
+// Mach-number detector with the characteristic length sqrt(area) (:692-700)
+__device__ __forceinline__ double rz_mach_switch(double area, double div, double sspd, double fuzz) {
+  return at_most_1(newton_div(20.0 * (mode_sqrt(area) * fabs(div)), sspd + fuzz));
+}
+// Order key of the element CFL step (time_integration.cpp:189-228); a NaN bounds nothing.
+__device__ __forceinline__ long long rz_cfl_key(double d2, double sspd, double dt_cfl, double fuzz) {
+  const double dt_l = newton_div(dt_cfl * mode_sqrt(d2), sspd + fuzz);
+  return (__double_as_longlong(dt_l) & kAbsMask) > 0x7FF0000000000000LL ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);
+}
+
 // ---------------------------------------------------------------------------
 // Corner forces of the quad (force_sgh.cpp:407-808).  The shock-direction and
 // curl terms feed only unused values (use_shock_dir = 0, phi_curl unused) and
@@ -189,6 +230,7 @@ __device__ __forceinline__ void gather4(const int* nie, int e, int (&nid)[4]) {
 // RZ velocity gradient (momentum.cpp:151-217); otherwise stress is zero.
 template <bool STRENGTH>
 __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
+  previous_launch_done();
   if (!a.ctrl->active) return;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.ne) return;
@@ -198,17 +240,18 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
   double x[4], y[4], u[4], v[4];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    x[l] = __ldg(a.x + nid[l]);
-    y[l] = __ldg(a.y + nid[l]);
-    u[l] = __ldg(a.u + nid[l]);
-    v[l] = __ldg(a.v + nid[l]);
+    x[l] = a.x[nid[l]];
+    y[l] = a.y[nid[l]];
+    u[l] = a.u[nid[l]];
+    v[l] = a.v[nid[l]];
   }
   const RzDiffs df = rz_diffs(x, y);
   double B[4][2], ca[4] = {0.0, 0.0, 0.0, 0.0};
   rz_bmatrix(df, B);
   const double area = rz_area(df);
   const double den = a.den[e], pres = a.pres[e], sspd = a.sspd[e], vol = a.vol[e], div = a.div[e];
-  const bool hoop_zero = !STRENGTH && is_finite(pres) && rz_corner_areas_finite(df);
+  const bool hoop_zero = !STRENGTH && is_finite(pres) && 
+      rz_corner_areas_finite(df.x02, df.x13, df.y02, df.y13, -df.x01 - df.x23, -df.y01 - df.y23);
   if (!hoop_zero) rz_corner_areas(x, y, ca);
   const int mat = a.mat[e];
   const double* q = a.qtab + 4 * mat;
@@ -233,19 +276,16 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     vs1 = fma(0.25, v[l], vs1);
   }
   // MARS impedances (:520-636); |inward normal| = |B|, the same at opposite corners
-  const double bn[2] = {mode_sqrt(B[0][0] * B[0][0] + B[0][1] * B[0][1]),
-                        mode_sqrt(B[1][0] * B[1][0] + B[1][1] * B[1][1])};
+  const double bn[2] = {mode_sqrt(mul_mul(B[0][0], B[0][0], B[0][1], B[0][1])),
+                        mode_sqrt(mul_mul(B[1][0], B[1][0], B[1][1], B[1][1]))};
   double mu[4];
   double s0 = 0.0, s1 = 0.0, s3 = 0.0;
   const double q1c = qa * sspd;
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    const double d0 = u[l] - vs0, d1 = v[l] - vs1;
-    const double mag_vel = mode_sqrt(d0 * d0 + d1 * d1);
-    const double muc = den * (q1c + qb * mag_vel);
-    const double mu_term = muc * bn[l & 1];
-    s0 = s0 + mu_term * u[l];
-    s1 = s1 + mu_term * v[l];
+    const double mu_term = rz_impedance(den, q1c, qb, u[l] - vs0, v[l] - vs1) * bn[l & 1];
+    s0 = mul_add(s0, mu_term, u[l]);
+    s1 = mul_add(s1, mu_term, v[l]);
     s3 = s3 + mu_term;
     mu[l] = mu_term;
   }
@@ -261,36 +301,15 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     vstar1 = quot(s1, ds3);
 #endif
   }
-  // shock detector (:653-690): the minimum over neighbours of the monotone
-  // r_face(div_nb) sits at the smallest (div + small > 0) or largest neighbour
-  // divergence, as in the 3D kernel
-  const double small = a.small;
-  const double D = div + small;
   const int k0 = a.eie_start[e], k1 = a.eie_start[e + 1];
   long long kmin = 0x7FFFFFFFFFFFFFFFLL, kmax = (long long)0x8000000000000000ULL;
   for (int k = k0; k < k1; ++k) {
-    const long long key = okey(__ldg(a.div + __ldg(a.eie + k)));
+    const long long key = okey(a.div[__ldg(a.eie + k)]);
     kmin = key < kmin ? key : kmin;
     kmax = key > kmax ? key : kmax;
   }
-  double r_min = 1.0;
-  if (k1 > k0) {
-    const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
-    if (is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel)) {
-      const double r_face = newton_div(0.9 * (dsel + small), D);
-      r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
-    } else {
-      for (int k = k0; k < k1; ++k) {
-        const double r_face = newton_div(0.9 * (__ldg(a.div + __ldg(a.eie + k)) + small), D);
-        r_min = fmin(r_face, r_min);
-      }
-    }
-  }
-  double phi = 1.0 - at_least_0(r_min);
-  // Mach-number detector with the characteristic length sqrt(area) (:692-700)
-  const double c_length = mode_sqrt(area);
-  const double alpha = at_most_1(newton_div(20.0 * (c_length * fabs(div)), sspd + a.fuzz));
-  phi = alpha * phi;
+  const double phi = rz_mach_switch(area, div, sspd, a.fuzz) *
+                     (1.0 - at_least_0(rz_limiter_min(a, div, k0, k1, kmin, kmax)));
   // corner forces with the inward normals -B, then the hoop-stress terms (:718-755)
   const double vs[2] = {vstar0, vstar1};
 #pragma unroll
@@ -303,14 +322,14 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
       // finite normals and no shear: the products with tau's zeros are zeros, and so
       // are the hoop terms; adding those would only turn a -0.0 force into +0.0,
       // which is done on the bits
-      f[0] = a0 * t[0] + pm * (vs[0] - vl[0]);
-      f[1] = a1 * t[4] + pm * (vs[1] - vl[1]);
+      f[0] = mul_mul(a0, t[0], pm, vs[0] - vl[0]);
+      f[1] = mul_mul(a1, t[4], pm, vs[1] - vl[1]);
 #pragma unroll
       for (int d = 0; d < 2; ++d)
         if ((__double_as_longlong(f[d]) & kAbsMask) == 0) f[d] = 0.0;
     } else {
 #pragma unroll
-      for (int d = 0; d < 2; ++d) f[d] = a0 * t[d] + a1 * t[3 + d] + pm * (vs[d] - vl[d]);
+      for (int d = 0; d < 2; ++d) f[d] = mul_add(mul_mul(a0, t[d], a1, t[3 + d]), pm, vs[d] - vl[d]);
       const double r = y[l];
       if (r > 1e-14) {
         f[0] = f[0] + t[3] * ca[l] / r;
@@ -352,25 +371,39 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
 // mass of the new position replaces it at the end (the reference recomputes it
 // after update_state2D, and nothing in between reads it).
 __global__ void __launch_bounds__(kRzNodeBlock) k_node_rz(const RzNodeArgs a) {
+  previous_launch_done();
   if (!a.ctrl->active) return;
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.nn) return;
   const size_t ne = (size_t)a.ne;
   double f0 = 0.0, f1 = 0.0;
   const int c0 = a.cin_start[n], c1 = a.cin_start[n + 1];
-  for (int c = c0; c < c1; ++c) {
-    const int cid = __ldg(a.cin + c);
-    const int e = cid >> 2, l = cid & 3;
-    f0 = f0 + __ldg(a.force + (size_t)(l * 2 + 0) * ne + e);
-    f1 = f1 + __ldg(a.force + (size_t)(l * 2 + 1) * ne + e);
+  // four corners' ids, then their force loads, are issued together; the sums keep
+  // the corner order
+  for (int base = c0; base < c1; base += 4) {
+    double g[4][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool in = base + k < c1;
+      const int cid = in ? __ldg(a.cin + base + k) : 0;
+      const size_t at = (size_t)((cid & 3) * 2) * ne + (cid >> 2);
+      g[k][0] = in ? a.force[at] : 0.0;
+      g[k][1] = in ? a.force[at + ne] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (base + k < c1) {
+        f0 = f0 + g[k][0];
+        f1 = f1 + g[k][1];
+      }
   }
   const double adt = a.rk_alpha * a.ctrl->dt;
   const double m = a.node_mass[n];
   const double u0 = a.u0[n], v0 = a.v0[n];
 #if FIERRO_FMA
   const double rm = mode_rcp(m);
-  double u1 = u0 + adt * f0 * rm;
-  double v1 = v0 + adt * f1 * rm;
+  double u1 = mul_add(u0, adt * f0, rm);
+  double v1 = mul_add(v0, adt * f1, rm);
 #else
   const Divisor dm = divisor(m);  // correctly rounded quotients, one reciprocal seed
   double u1 = u0 + quot(adt * f0, dm);
@@ -386,8 +419,8 @@ __global__ void __launch_bounds__(kRzNodeBlock) k_node_rz(const RzNodeArgs a) {
   a.hx[n] = hu;
   a.hy[n] = hv;
   a.rad[n] = r_in;
-  const double x1 = a.x0[n] + adt * hu;
-  const double y1 = a.y0[n] + adt * hv;
+  const double x1 = mul_add(a.x0[n], adt, hu);
+  const double y1 = mul_add(a.y0[n], adt, hv);
   a.x1[n] = x1;
   a.y1[n] = y1;
   double mn = 0.0;
@@ -398,6 +431,7 @@ __global__ void __launch_bounds__(kRzNodeBlock) k_node_rz(const RzNodeArgs a) {
 // Nodes on the axis (y < tiny) among the boundary nodes: the largest half-mass
 // of their off-axis edge neighbours.  Off-axis masses are not written here.
 __global__ void __launch_bounds__(kRzNodeBlock) k_axis_rz(const RzAxisArgs a) {
+  previous_launch_done();
   if (!a.ctrl->active) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.naxis) return;
@@ -414,6 +448,7 @@ __global__ void __launch_bounds__(kRzNodeBlock) k_axis_rz(const RzAxisArgs a) {
 // ---------------------------------------------------------------------------
 template <int KIND>
 __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
+  previous_launch_done();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   Ctrl* ctrl = a.ctrl;
   if (KIND != 2 && !ctrl->active) return;
@@ -425,10 +460,10 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     double x[4], y[4], u[4], v[4];
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-      x[l] = __ldg(a.x + nid[l]);
-      y[l] = __ldg(a.y + nid[l]);
-      u[l] = __ldg(a.u + nid[l]);
-      v[l] = __ldg(a.v + nid[l]);
+      x[l] = a.x[nid[l]];
+      y[l] = a.y[nid[l]];
+      u[l] = a.u[nid[l]];
+      v[l] = a.v[nid[l]];
     }
     double sie1 = 0.0;
     if (KIND != 2) {
@@ -437,12 +472,12 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
       double power = 0.0;
 #pragma unroll
       for (int l = 0; l < 4; ++l) {
-        const double r = __ldg(a.rad + nid[l]);
-        power = power + a.force[(size_t)(l * 2 + 0) * ne + e] * r * __ldg(a.hx + nid[l]);
-        power = power + a.force[(size_t)(l * 2 + 1) * ne + e] * r * __ldg(a.hy + nid[l]);
+        const double r = a.rad[nid[l]];
+        power = mul_add(power, a.force[(size_t)(l * 2 + 0) * ne + e] * r, a.hx[nid[l]]);
+        power = mul_add(power, a.force[(size_t)(l * 2 + 1) * ne + e] * r, a.hy[nid[l]]);
       }
       const double adt = a.rk_alpha * ctrl->dt;
-      sie1 = a.sie0[e] - newton_div(adt, a.mass[e]) * power;
+      sie1 = mul_add(a.sie0[e], -newton_div(adt, a.mass[e]), power);
       a.sie1[e] = sie1;
     }
     const RzDiffs df = rz_diffs(x, y);
@@ -455,10 +490,10 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     const double inverse_area = quot(1.0, da);
     const double mean_radius = quot(vol, da);
     const double elem_vel_r = 0.25 * (v[0] + v[1] + v[2] + v[3]);
-    double div = 0.0;
-    div = div + (u[0] * B[0][0] + u[1] * B[1][0] + u[2] * B[2][0] + u[3] * B[3][0]) * inverse_area;
-    div = div + ((v[0] * B[0][1] + v[1] * B[1][1] + v[2] * B[2][1] + v[3] * B[3][1]) * inverse_area +
-                 newton_div(elem_vel_r, mean_radius));
+    const double su = mul_add(mul_add(mul_mul(u[0], B[0][0], u[1], B[1][0]), u[2], B[2][0]), u[3], B[3][0]);
+    const double sv = mul_add(mul_add(mul_mul(v[0], B[0][1], v[1], B[1][1]), v[2], B[2][1]), v[3], B[3][1]);
+    double div = mul_add(0.0, su, inverse_area);
+    div = div + mul_add(newton_div(elem_vel_r, mean_radius), sv, inverse_area);
     a.div[e] = div;
     double sspd;
     if (KIND != 2) {
@@ -485,14 +520,10 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
       long long kd = 0x7FFFFFFFFFFFFFFFLL;  // squares are >= 0: their bits order as they do
 #pragma unroll
       for (int i = 0; i < 6; ++i) {
-        const long long k = __double_as_longlong(dx[i] * dx[i] + dy[i] * dy[i]) & kAbsMask;
+        const long long k = __double_as_longlong(mul_mul(dx[i], dx[i], dy[i], dy[i])) & kAbsMask;
         kd = k < kd ? k : kd;
       }
-      const double d2 = __longlong_as_double(kd);
-      const double dist_min = mode_sqrt(d2);
-      const double dt_l = newton_div(a.dt_cfl * dist_min, sspd + a.fuzz);
-      const long long db = __double_as_longlong(dt_l);
-      dkey = (db & kAbsMask) > 0x7FF0000000000000LL ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);  // NaN: no bound
+      dkey = rz_cfl_key(__longlong_as_double(kd), sspd, a.dt_cfl, a.fuzz);
     }
   }
   if (KIND != 0) {
@@ -500,6 +531,8 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     if (threadIdx.x == 0) a.cfl_part[blockIdx.x] = k;
   }
 }
+
+#include "sgh_rz_lanes.cuh"
 
 __global__ void __launch_bounds__(kRzNodeBlock) k_ext_rz(int nn, const double* node_mass, const double* y,
                                                         double* ext) {
@@ -551,20 +584,31 @@ __global__ void k_energy_rz_final(const RzEnergyArgs a, int nblocks) {
 static unsigned blocks_for(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 static void launch_force(const RzForceArgs& a, cudaStream_t s) {
-  if (a.stress_out) k_force_rz<true><<<blocks_for(a.ne, kRzBlock), kRzBlock, 0, s>>>(a);
-  else k_force_rz<false><<<blocks_for(a.ne, kRzBlock), kRzBlock, 0, s>>>(a);
+  const int bs = small_mesh_block(a.ne, kRzBlock);
+  if (a.stress_out) launch(k_force_rz<true>, blocks_for(a.ne, bs), bs, s, a);
+  else if (a.lanes) launch(k_force_rz_lanes, blocks_for(4LL * a.ne, kRzLaneBlock), kRzLaneBlock, s, a);
+  else launch(k_force_rz<false>, blocks_for(a.ne, bs), bs, s, a);
 }
 static void launch_node(const RzNodeArgs& a, cudaStream_t s) {
-  k_node_rz<<<blocks_for(a.nn, kRzNodeBlock), kRzNodeBlock, 0, s>>>(a);
+  const int bs = small_mesh_block(a.nn, kRzNodeBlock);
+  launch(k_node_rz, blocks_for(a.nn, bs), bs, s, a);
 }
 static void launch_axis(const RzAxisArgs& a, cudaStream_t s) {
-  k_axis_rz<<<blocks_for(a.naxis > 0 ? a.naxis : 1, kRzNodeBlock), kRzNodeBlock, 0, s>>>(a);
+  const int bs = small_mesh_block(a.naxis, kRzNodeBlock);
+  launch(k_axis_rz, blocks_for(a.naxis > 0 ? a.naxis : 1, bs), bs, s, a);
 }
 static void launch_elem(const RzElemArgs& a, int kind, cudaStream_t s) {
+  if (a.lanes) {
+    const unsigned g = blocks_for(4LL * a.ne, kRzLaneBlock);
+    if (kind == 0) launch(k_elem_rz_lanes<0>, g, kRzLaneBlock, s, a);
+    else if (kind == 1) launch(k_elem_rz_lanes<1>, g, kRzLaneBlock, s, a);
+    else launch(k_elem_rz_lanes<2>, g, kRzLaneBlock, s, a);
+    return;
+  }
   const unsigned g = blocks_for(a.ne, kRzBlock);
-  if (kind == 0) k_elem_rz<0><<<g, kRzBlock, 0, s>>>(a);
-  else if (kind == 1) k_elem_rz<1><<<g, kRzBlock, 0, s>>>(a);
-  else k_elem_rz<2><<<g, kRzBlock, 0, s>>>(a);
+  if (kind == 0) launch(k_elem_rz<0>, g, kRzBlock, s, a);
+  else if (kind == 1) launch(k_elem_rz<1>, g, kRzBlock, s, a);
+  else launch(k_elem_rz<2>, g, kRzBlock, s, a);
 }
 static void launch_ext(int nn, const double* node_mass, const double* y, double* ext, cudaStream_t s) {
   k_ext_rz<<<blocks_for(nn, kRzNodeBlock), kRzNodeBlock, 0, s>>>(nn, node_mass, y, ext);

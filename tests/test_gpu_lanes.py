@@ -69,3 +69,45 @@ def test_checkpoint_of_a_lane_handle(lib_built, tmp_path, shape):
     assert gt == wt
     for k in want:
         assert np.array_equal(got[k], want[k]), k
+
+
+# 1 and 3 elements, a warp's eight and one more, 9000 | 9020 (element pass), 11500 | 11504 (force pass)
+RZ_SHAPES = [(1, 1), (3, 1), (4, 2), (3, 3), (90, 100), (82, 110), (115, 100), (16, 719)]
+
+
+def _rz_deck(shape, cycles):
+    from fierro_gb300 import mesh, problems
+    m = mesh.quad_mesh(*shape, length=(1.0, 1.2), jitter=0.1, seed=sum(shape), permute=True)
+    p = problems.noh_rz(max(shape), mesh=m, cycles=cycles)
+    p.materials[0].q2ex = 0.4
+    p.fills[0].sie = 0.02
+    return p
+
+
+@pytest.mark.parametrize("shape", RZ_SHAPES)
+def test_quad_lanes_equal_the_restatement(oracle_built, lib_built, shape):
+    """Exact mode, bit for bit against the C restatement; the FMA mode within the
+    one-cycle gate of the exact one."""
+    from conftest import assert_fields
+    from fierro_gb300 import sgh
+    from oracle import orc
+    p = _rz_deck(shape, 8)
+    st = sgh.setup(p)
+    o = orc.Oracle(p, variant="crpow")
+    o.run_cycles(8)
+    ref = o.state()
+    with sgh.SGHSolver(p) as s:
+        s.set_state(st)
+        s.run(1)
+        one = sgh.compared_fields(s.get_state())
+        s.run(7)
+        got = s.get_state()
+    flat = sgh.compared_fields(got)
+    flat.update(corner_force=got["corner_force"], node_mass=got["node_mass"])
+    for k in ("coords", "vel", "den", "pres", "sie", "sspd", "vol", "corner_force", "node_mass"):
+        assert np.array_equal(np.asarray(flat[k]).ravel(), np.asarray(ref[k]).ravel()), k
+    with sgh.SGHSolver(p, fp_mode=sgh.FP_FMA) as s:
+        s.set_state(st)
+        s.run(1)
+        fma = sgh.compared_fields(s.get_state())
+    assert_fields(fma, one, 1e-12, keys=("coords", "vel", "den", "pres", "sie"), label="fma %s" % (shape,))
