@@ -521,9 +521,15 @@ __global__ void __launch_bounds__(kAdjForceBlock, 3) k_adj_force(const AdjMesh m
     const double g = fma(F0, vstar0 - vu[l], fma(F1, vstar1 - vv[l], F2 * (vstar2 - vw[l])));
     phib = fma(mu[l], g, phib);
     mub[l] = phi * g;
-    vsb0 = fma(pm, F0, vsb0);
-    vsb1 = fma(pm, F1, vsb1);
-    vsb2 = fma(pm, F2, vsb2);
+    // phi mu_l Fbar_l: v*'s adjoint, and with a minus sign this corner's velocity's,
+    // kept in the output rows for pass 2
+    const double pf0 = pm * F0, pf1 = pm * F1, pf2 = pm * F2;
+    vsb0 += pf0;
+    vsb1 += pf1;
+    vsb2 += pf2;
+    b.cv[i0] = -pf0;
+    b.cv[i1] = -pf1;
+    b.cv[i2] = -pf2;
   }
   const double alphab = phib * phi0, phi0b = phib * alpha;
   double divb = 0.0, sspdb = 0.0, volb = 0.0, denb = 0.0;
@@ -554,18 +560,14 @@ __global__ void __launch_bounds__(kAdjForceBlock, 3) k_adj_force(const AdjMesh m
   // Pass 2: per corner, the velocity adjoint (viscous term, v*, |v_l - v_avg|)
   // and the |B_l| term of mu_l.
   double vss0 = 0.0, vss1 = 0.0, vss2 = 0.0, q1cb = 0.0;
+  const double den_qb = den * qb;
 #pragma unroll
   for (int l = 0; l < 8; ++l) {
-    const int n = nid[l];
-    const double F0 = fma(we, s1.hx[n], b.fbar[0][n]);
-    const double F1 = fma(we, s1.hy[n], b.fbar[1][n]);
-    const double F2 = fma(we, s1.hz[n], b.fbar[2][n]);
-    const double pm = phi * mu[l];
-    double vb0 = fma(mu[l], sb0, -pm * F0);
-    double vb1 = fma(mu[l], sb1, -pm * F1);
-    double vb2 = fma(mu[l], sb2, -pm * F2);
-    const double mubl = fma(sb0, vu[l], fma(sb1, vv[l], fma(sb2, vw[l], mub[l] + s3b)));
     const size_t i0 = (size_t)(l * 3) * ne + e, i1 = i0 + ne, i2 = i1 + ne;
+    double vb0 = fma(mu[l], sb0, b.cv[i0]);
+    double vb1 = fma(mu[l], sb1, b.cv[i1]);
+    double vb2 = fma(mu[l], sb2, b.cv[i2]);
+    const double mubl = fma(sb0, vu[l], fma(sb1, vv[l], fma(sb2, vw[l], mub[l] + s3b)));
     const double b0 = s0.bmat[i0], b1 = s0.bmat[i1], b2 = s0.bmat[i2];
     const double qB = fma(b0, b0, fma(b1, b1, b2 * b2));
     const double rB = fast_rsqrt(qB);
@@ -580,7 +582,7 @@ __global__ void __launch_bounds__(kAdjForceBlock, 3) k_adj_force(const AdjMesh m
     q1cb = fma(mucb, den, q1cb);
     if (mv[l] > 0.0) {
       const double d0 = vu[l] - vs0, d1 = vv[l] - vs1, d2 = vw[l] - vs2;
-      const double sm = mucb * den * qb * fast_rsqrt(fma(d0, d0, fma(d1, d1, d2 * d2)));
+      const double sm = mucb * den_qb * fast_rcp(mv[l]);  // mv = |v_l - v_avg|
       vb0 = fma(sm, d0, vb0);
       vb1 = fma(sm, d1, vb1);
       vb2 = fma(sm, d2, vb2);
