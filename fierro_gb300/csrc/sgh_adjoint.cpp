@@ -193,8 +193,9 @@ int ensure(fierro_sgh* h, int k, int nseg) {
     for (int d = 0; d < 6; ++d)
       if ((rc = aalloc(a, &a->an[i][d], nn))) return fail(rc);
   }
-  b.nbe = (int)((ne + 127) / 128);
-  b.nbn = (int)((nn + 255) / 256);
+  const int be = small_mesh_block(ne, kAdjElemBlock), bn = small_mesh_block(nn, kAdjNodeBlock);
+  b.nbe = (int)((ne + be - 1) / be);
+  b.nbn = (int)((nn + bn - 1) / bn);
   if ((rc = aalloc(a, &b.part_e, (size_t)S * b.nbe))) return fail(rc);
   if ((rc = aalloc(a, &b.part_n, (size_t)S * b.nbn))) return fail(rc);
   if ((rc = aalloc(a, &b.sc, 1))) return fail(rc);

@@ -40,9 +40,7 @@ namespace adj_impl {
 #include "sgh_hex_geometry.cuh"
 #include "sgh_cfl.cuh"
 
-constexpr int kAdjElemBlock = 128;
 constexpr int kAdjForceBlock = 128;
-constexpr int kAdjNodeBlock = 256;
 constexpr long long kMaxKey = 0x7FFFFFFFFFFFFFFFLL;
 
 enum { BR_GROW = 0, BR_CFL = 1, BR_DTMAX = 2, BR_DTMIN = 3, BR_GRAPH = 4, BR_FINAL = 5 };
@@ -365,24 +363,41 @@ __global__ void __launch_bounds__(kAdjNodeBlock) k_adj_node(const AdjMesh m, con
     double gx = 0.0, gy = 0.0, gz = 0.0, gu = 0.0, gv = 0.0, gw = 0.0;
     double f0 = 0.0, f1 = 0.0, f2 = 0.0, hb0 = 0.0, hb1 = 0.0, hb2 = 0.0;
     const int c0 = m.cin_start[n], c1 = m.cin_start[n + 1];
-    for (int c = c0; c < c1; ++c) {
-      const int cid = __ldg(m.cin + c);
-      const int e = cid >> 3, l = cid & 7;
-      const size_t i0 = (size_t)(l * 3) * ne + e, i1 = i0 + ne, i2 = i1 + ne;
-      gx += b.cx[i0];
-      gy += b.cx[i1];
-      gz += b.cx[i2];
-      gu += b.cv[i0];
-      gv += b.cv[i1];
-      gw += b.cv[i2];
-      const double we = b.w[e];
-      const double F0 = force[i0], F1 = force[i1], F2 = force[i2];
-      f0 += F0;
-      f1 += F1;
-      f2 += F2;
-      hb0 += we * F0;
-      hb1 += we * F1;
-      hb2 += we * F2;
+    // four corners' ids, then their ten loads each, are issued together; the sums
+    // keep the corner order
+    for (int base = c0; base < c1; base += 4) {
+      double g[4][10];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool in = base + k < c1;
+        const int cid = in ? __ldg(m.cin + base + k) : 0;
+        const int e = cid >> 3, l = cid & 7;
+        const size_t i0 = (size_t)(l * 3) * ne + e;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const size_t i = i0 + d * ne;
+          g[k][d] = in ? b.cx[i] : 0.0;
+          g[k][3 + d] = in ? b.cv[i] : 0.0;
+          g[k][6 + d] = in ? force[i] : 0.0;
+        }
+        g[k][9] = in ? b.w[e] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (base + k >= c1) break;
+        gx += g[k][0];
+        gy += g[k][1];
+        gz += g[k][2];
+        gu += g[k][3];
+        gv += g[k][4];
+        gw += g[k][5];
+        f0 += g[k][6];
+        f1 += g[k][7];
+        f2 += g[k][8];
+        hb0 = fma(g[k][9], g[k][6], hb0);
+        hb1 = fma(g[k][9], g[k][7], hb1);
+        hb2 = fma(g[k][9], g[k][8], hb2);
+      }
     }
     if (an_in.p[0]) {
       gx += an_in.p[0][n];
@@ -799,7 +814,8 @@ static void launch_pre(AdjRecord* r, const long long* cfl_part, int nparts, cons
 }
 static void launch_argmin(AdjRecord* r, const Ctrl* ctrl, const LoopParams& lp, const AdjMesh& m, const Slot& s,
                           cudaStream_t st) {
-  k_adj_argmin<<<blocks_for(m.ne, kAdjElemBlock), kAdjElemBlock, 0, st>>>(r, ctrl, lp, m, s);
+  const int bs = small_mesh_block(m.ne, kAdjElemBlock);
+  k_adj_argmin<<<blocks_for(m.ne, bs), bs, 0, st>>>(r, ctrl, lp, m, s);
 }
 static void launch_seed(const AdjMesh& m, const AdjBufs& b, const Slot& fin, const double* eseed,
                         const double* nseed, unsigned mask, double* sb_next, const Node6& an, cudaStream_t st) {
@@ -809,21 +825,23 @@ static void launch_seed(const AdjMesh& m, const AdjBufs& b, const Slot& fin, con
 static void launch_elem(const AdjMesh& m, const AdjBufs& b, const Slot& s1, const double* force,
                         const AdjRecord* r, double alpha, const double* sie_in, double* sie_c, int assign,
                         double* part, int kind, cudaStream_t st) {
-  const unsigned g = blocks_for(m.ne, kAdjElemBlock);
-  if (kind == 2) k_adj_elem<2><<<g, kAdjElemBlock, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
-  else k_adj_elem<0><<<g, kAdjElemBlock, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
+  const int bs = small_mesh_block(m.ne, kAdjElemBlock);
+  const unsigned g = blocks_for(m.ne, bs);
+  if (kind == 2) k_adj_elem<2><<<g, bs, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
+  else k_adj_elem<0><<<g, bs, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
 }
 static void launch_node(const AdjMesh& m, const AdjBufs& b, const Slot& s1, const double* force,
                         const AdjRecord* r, double alpha, const Node6& an_in, const Node6& an_c, int assign,
                         double* part, cudaStream_t st) {
-  k_adj_node<<<blocks_for(m.nn, kAdjNodeBlock), kAdjNodeBlock, 0, st>>>(m, b, s1, force, r, alpha, an_in, an_c,
-                                                                         assign, part);
+  const int bs = small_mesh_block(m.nn, kAdjNodeBlock);
+  k_adj_node<<<blocks_for(m.nn, bs), bs, 0, st>>>(m, b, s1, force, r, alpha, an_in, an_c, assign, part);
 }
 static void launch_force(const AdjMesh& m, const AdjBufs& b, const Slot& s0, const Slot& s1,
                          const double* force_tape, const double* ft, const int* fsel, double fuzz, double small,
                          double* sie_out, int accumulate, cudaStream_t st) {
-  k_adj_force<<<blocks_for(m.ne, kAdjForceBlock), kAdjForceBlock, 0, st>>>(m, b, s0, s1, force_tape, ft, fsel, fuzz,
-                                                                            small, sie_out, accumulate);
+  const int bs = small_mesh_block(m.ne, kAdjForceBlock);
+  k_adj_force<<<blocks_for(m.ne, bs), bs, 0, st>>>(m, b, s0, s1, force_tape, ft, fsel, fuzz, small, sie_out,
+                                                   accumulate);
 }
 static void launch_dt(const AdjMesh& m, const AdjBufs& b, const AdjRecord* r, const LoopParams& lp,
                       const Slot& s0, int stages, const AdjAlphas& al, const Node6& an_c, double* sie_c,

@@ -32,6 +32,11 @@
 
 namespace fierro {
 
+// Default threads per block of the reverse element and node passes, whose blocks
+// leave one partial sum each (smaller on small meshes: small_mesh_block).
+constexpr int kAdjElemBlock = 128;
+constexpr int kAdjNodeBlock = 256;
+
 struct Slot {
   double *x, *y, *z, *u, *v, *w;
   double *hx, *hy, *hz;

@@ -404,6 +404,7 @@ static int create_impl(fierro_sgh* h, const fierro_mesh* mesh, const fierro_mate
   h->lanes_node = (long long)nn <= kLanesNode;
   h->lanes_elem = (long long)ne <= kLanesElem && !h->has_hyper;
   h->cfl_tile = h->lanes_elem ? kLaneTile : h->blk_elem;
+  h->ckpt_tile = checkpoint_tile((long long)ne);
   h->ncfl = (int)((ne + h->cfl_tile - 1) / h->cfl_tile);
   TRY(dalloc(h, &h->d_cfl, (size_t)h->ncfl));
   TRY(dalloc(h, &h->d_ctrl, 1));
@@ -986,12 +987,12 @@ struct CkptHeader {
 struct Block {
   void* ptr;
   size_t bytes;
-  bool cfl = false;  // the CFL partials: in the file one per element block, also of a lane handle
+  bool cfl = false;  // the CFL partials: in the file one per ckpt_tile elements
 };
 
 // The CFL partials a file holds, and how many of a handle's fall on each.
-int64_t ckpt_ncfl(const fierro_sgh* h) { return (h->ne + h->blk_elem - 1) / h->blk_elem; }
-int64_t ckpt_cfl_group(const fierro_sgh* h) { return h->blk_elem / h->cfl_tile; }
+int64_t ckpt_ncfl(const fierro_sgh* h) { return (h->ne + h->ckpt_tile - 1) / h->ckpt_tile; }
+int64_t ckpt_cfl_group(const fierro_sgh* h) { return h->ckpt_tile / h->cfl_tile; }
 
 uint64_t fnv1a(uint64_t h, const void* p, size_t n) {
   const unsigned char* c = static_cast<const unsigned char*>(p);

@@ -224,14 +224,20 @@ constexpr int kEnergyBlock = 256;
 
 // Launch block for `n` threads of a kernel whose default block is `bs`: halved
 // (down to one warp) while the grid would have fewer than kMinBlocks blocks, so a
-// small mesh spreads over more SMs (each SM's FP64 rate, not the chip's, bounds
-// a kernel that occupies few of them).  It depends on n alone, so the number of
-// CFL partials (one per element block) is a property of the mesh.
-constexpr long long kMinBlocks = 304;  // two per SM of a 152-SM GB300
-inline int small_mesh_block(long long n, int bs) {
-  while (bs > 32 && (n + bs - 1) / bs < kMinBlocks) bs >>= 1;
+// small mesh spreads evenly over the SMs (each SM's FP64 rate, not the chip's,
+// bounds a kernel: with blocks of 64 threads the 1024 warps of a 32^3 mesh fall
+// as 6 or 8 to an SM, with one-warp blocks as 6 or 7: cycle 141 -> 130 us FMA,
+// 192 -> 175 exact; 40^3 252 -> 242; from 48^3 on, blocks of 128 do as well, with
+// fewer CFL partials).  It depends on n alone, so the number of CFL partials (one
+// per element block) is a property of the mesh.
+constexpr long long kMinBlocks = 800;
+inline int small_mesh_block(long long n, int bs, long long min_blocks = kMinBlocks) {
+  while (bs > 32 && (n + bs - 1) / bs < min_blocks) bs >>= 1;
   return bs;
 }
+// Elements per CFL partial of a hex checkpoint file (its format: the element
+// block such a handle had when at least 304 blocks were asked for).
+inline int checkpoint_tile(long long ne) { return small_mesh_block(ne, kElemBlock, 304); }
 
 // Meshes of at most this many elements (nodes) run the lane passes of
 // sgh_lanes.cuh.  A lane pass does about twice the work in an eighth-long chain:

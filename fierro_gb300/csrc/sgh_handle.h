@@ -66,6 +66,7 @@ struct fierro_sgh {
   long long* d_cfl = nullptr;
   int ncfl = 0;  // CFL partials, one per cfl_tile elements (an element block, or a lane pass's warp)
   int cfl_tile = fierro::kElemBlock;
+  int ckpt_tile = fierro::kElemBlock;  // elements per partial in a checkpoint file, a multiple of cfl_tile
   // threads per block of the element, force and node kernels (small_mesh_block)
   int blk_elem = fierro::kElemBlock, blk_force = fierro::kForceBlock, blk_node = fierro::kNodeBlock;
   bool lanes_force = false, lanes_node = false, lanes_elem = false;  // small meshes: sgh_lanes.cuh
