@@ -12,6 +12,8 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <exception>
+#include <string>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -105,10 +107,14 @@ int put(fierro_batch* b, T* dst, const std::vector<T>& src) {
   return FIERRO_OK;
 }
 
+// Values a host loop over one instance's array shares among the threads from.
+constexpr int64_t kHostParallel = 4096;
+
 // dst[off + k] = src[map[k] * stride + sub] through the pinned staging buffer.
 int gather_up(fierro_batch* b, double* dst, int64_t off, const double* src, const std::vector<int64_t>& map,
               size_t stride, size_t sub) {
   const int64_t n = (int64_t)map.size();
+#pragma omp parallel for schedule(static) if (n >= kHostParallel)
   for (int64_t k = 0; k < n; ++k) b->h_stage[k] = src[(size_t)map[k] * stride + sub];
   CUDA_TRY(cudaMemcpyAsync(dst + off, b->h_stage, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, b->stream));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
@@ -120,6 +126,7 @@ int scatter_down(fierro_batch* b, double* out, const double* src, int64_t off, c
   const int64_t n = (int64_t)map.size();
   CUDA_TRY(cudaMemcpyAsync(b->h_stage, src + off, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, b->stream));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
+#pragma omp parallel for schedule(static) if (n >= kHostParallel)
   for (int64_t k = 0; k < n; ++k) out[(size_t)map[k] * stride + sub] = b->h_stage[k];
   return FIERRO_OK;
 }
@@ -329,6 +336,50 @@ int apply_shape(fierro_batch* b, const fierro_batch_shape& sh) {
   return FIERRO_OK;
 }
 
+int check_instance(const fierro_batch_instance& I, const fierro_sgh_params& p0, int64_t i) {
+  const fierro_sgh_params& p = I.params;
+  if (p.rk_num_stages != p0.rk_num_stages || p.fuzz != p0.fuzz || p.small != p0.small || p.tiny != p0.tiny)
+    return set_error(FIERRO_EINVAL, "batch: instance %lld: rk_num_stages, fuzz, tiny and small must match", (long long)i);
+  if (p.graphics_cyc_ival < 1 || !(p.dt_cfl > 0) || !(p.dt_max > 0) || !(p.dt_min > 0) || !(p.dt_start > 0))
+    return set_error(FIERRO_EINVAL, "batch: instance %lld: bad time-step controls", (long long)i);
+  if (I.num_materials < 1 || !I.materials) return set_error(FIERRO_EINVAL, "batch: instance %lld: no material", (long long)i);
+  for (int64_t m = 0; m < I.num_materials; ++m)
+    if (I.materials[m].eos_model != 0 || I.materials[m].strength_type != 0)
+      return set_error(FIERRO_ENOTSUP, "batch: instance %lld: only ideal gas without strength", (long long)i);
+  if (mesh_dims(&I.mesh) == 2)
+    return set_error(FIERRO_ENOTSUP, "batch: instance %lld is a 2D-RZ mesh (hex meshes only)", (long long)i);
+  return FIERRO_OK;
+}
+
+// The instances' topologies, inst[0..count): several at a time, one host thread
+// each (build_topology's own loops are too short to fill the threads on an
+// ensemble's meshes: twelve decks of 148,000 elements 56 ms one after the other);
+// instances above an eighth of the ensemble run by themselves over all threads.
+// Reports the error of the lowest-numbered instance, as one after the other did.
+int build_topologies(fierro_batch* b, const fierro_batch_instance* inst, int64_t count) {
+  std::vector<int> rc((size_t)count, FIERRO_OK);
+  std::vector<std::string> msg((size_t)count);
+  int64_t total = 0;
+  for (int64_t i = 0; i < count; ++i) total += std::max<int64_t>(inst[i].mesh.num_elems, 0);
+  auto one = [&](int64_t i) {
+    try {
+      rc[i] = build_topology(&inst[i].mesh, inst[i].boundaries, inst[i].num_bcs, true, &b->topo[i]);
+      if (rc[i]) msg[i] = fierro_last_error();
+    } catch (const std::exception&) {
+      rc[i] = FIERRO_ENOMEM;
+    }
+  };
+  auto alone = [&](int64_t i) { return inst[i].mesh.num_elems > total / 8; };
+  for (int64_t i = 0; i < count; ++i)
+    if (alone(i)) one(i);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int64_t i = 0; i < count; ++i)
+    if (!alone(i)) one(i);
+  for (int64_t i = 0; i < count; ++i)
+    if (rc[i]) return set_error(rc[i], "batch: instance %lld: %s", (long long)i, msg[i].empty() ? "host allocation failed" : msg[i].c_str());
+  return FIERRO_OK;
+}
+
 int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, int fp_mode, void* stream) {
   if (!inst || n < 1) return set_error(FIERRO_EINVAL, "batch: need at least one instance");
   if (n > (1 << 24)) return set_error(FIERRO_EINVAL, "batch: too many instances");
@@ -348,24 +399,19 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   b->lps.resize((size_t)n);
   b->dt_start.resize((size_t)n);
   b->has_state.assign((size_t)n, 0);
+  // the instances' controls in order, up to the first that is refused
+  int64_t checked = 0;
+  int bad_rc = FIERRO_OK;
+  for (; checked < n; ++checked) {
+    bad_rc = check_instance(inst[checked], p0, checked);
+    if (bad_rc) break;
+  }
+  std::string bad_msg = bad_rc ? fierro_last_error() : "";
+  TRY(build_topologies(b, inst, checked));
+  if (bad_rc) return set_error(bad_rc, "%s", bad_msg.c_str());
   for (int64_t i = 0; i < n; ++i) {
     const fierro_batch_instance& I = inst[i];
     const fierro_sgh_params& p = I.params;
-    if (p.rk_num_stages != p0.rk_num_stages || p.fuzz != p0.fuzz || p.small != p0.small || p.tiny != p0.tiny)
-      return set_error(FIERRO_EINVAL, "batch: instance %lld: rk_num_stages, fuzz, tiny and small must match", (long long)i);
-    if (p.graphics_cyc_ival < 1 || !(p.dt_cfl > 0) || !(p.dt_max > 0) || !(p.dt_min > 0) || !(p.dt_start > 0))
-      return set_error(FIERRO_EINVAL, "batch: instance %lld: bad time-step controls", (long long)i);
-    if (I.num_materials < 1 || !I.materials) return set_error(FIERRO_EINVAL, "batch: instance %lld: no material", (long long)i);
-    for (int64_t m = 0; m < I.num_materials; ++m)
-      if (I.materials[m].eos_model != 0 || I.materials[m].strength_type != 0)
-        return set_error(FIERRO_ENOTSUP, "batch: instance %lld: only ideal gas without strength", (long long)i);
-    if (mesh_dims(&I.mesh) == 2)
-      return set_error(FIERRO_ENOTSUP, "batch: instance %lld is a 2D-RZ mesh (hex meshes only)", (long long)i);
-    int rc = build_topology(&I.mesh, I.boundaries, I.num_bcs, true, &b->topo[i]);
-    if (rc) {
-      std::string msg = fierro_last_error();
-      return set_error(rc, "batch: instance %lld: %s", (long long)i, msg.c_str());
-    }
     const int64_t ne_pad = (I.mesh.num_elems + kElemBlock - 1) / kElemBlock * kElemBlock;
     b->node_off[i + 1] = b->node_off[i] + I.mesh.num_nodes;
     b->elem_off[i + 1] = b->elem_off[i] + ne_pad;
@@ -382,24 +428,31 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
     return set_error(FIERRO_EINVAL, "batch too large for 32-bit device indices");
   // concatenated mesh arrays (global ids)
   const int64_t NN = b->NN, NE = b->NE;
-  std::vector<int32_t> nie((size_t)NE * 8, 0), cin_start((size_t)NN + 1, 0), cin, eie_start((size_t)NE + 1, 0), eie;
+  std::vector<int64_t> cin_off((size_t)n + 1, 0), eie_off((size_t)n + 1, 0);
+  for (int64_t i = 0; i < n; ++i) {
+    cin_off[i + 1] = cin_off[i] + (int64_t)b->topo[i].cin.size();
+    eie_off[i + 1] = eie_off[i] + (int64_t)b->topo[i].eie.size();
+  }
+  std::vector<int32_t> nie((size_t)NE * 8, 0), cin_start((size_t)NN + 1, 0), cin((size_t)cin_off[n]);
+  std::vector<int32_t> eie_start((size_t)NE + 1, 0), eie((size_t)eie_off[n]);
   std::vector<int32_t> mat((size_t)NE, 0), inst_e((size_t)NE, 0), inst_n((size_t)NN, 0);
   std::vector<uint8_t> bc((size_t)NN, 0);
   std::vector<double> qtab((size_t)b->mat_off[n] * 4), dtc((size_t)n);
-  cin.reserve((size_t)NE * 8);
+#pragma omp parallel for schedule(dynamic, 1) if (NE >= kHostParallel)
   for (int64_t i = 0; i < n; ++i) {
     const HostTopo& t = b->topo[i];
     const int64_t no = b->node_off[i], eo = b->elem_off[i];
     for (int64_t e = 0; e < t.ne * 8; ++e) nie[(size_t)eo * 8 + e] = (int32_t)(t.nie[e] + no);
     for (int64_t e = eo; e < b->elem_off[i + 1]; ++e) inst_e[e] = (e - eo < t.ne) ? (int32_t)i : (int32_t)(-i - 1);
     for (int64_t k = 0; k < t.nn; ++k) {
-      cin_start[no + k + 1] = (int32_t)(t.cin_start[k + 1] - t.cin_start[k]);
+      cin_start[no + k + 1] = (int32_t)(cin_off[i] + t.cin_start[k + 1]);
       inst_n[no + k] = (int32_t)i;
       bc[no + k] = t.bc_mask[k];
     }
-    for (int32_t c : t.cin) cin.push_back((int32_t)(c + eo * 8));
-    for (int64_t e = 0; e < t.ne; ++e) eie_start[eo + e + 1] = t.eie_start[e + 1] - t.eie_start[e];
-    for (int32_t o : t.eie) eie.push_back((int32_t)(o + eo));
+    for (size_t k = 0; k < t.cin.size(); ++k) cin[(size_t)cin_off[i] + k] = (int32_t)(t.cin[k] + eo * 8);
+    for (int64_t e = eo; e < b->elem_off[i + 1]; ++e)
+      eie_start[e + 1] = (int32_t)(eie_off[i] + t.eie_start[std::min(e - eo + 1, t.ne)]);
+    for (size_t k = 0; k < t.eie.size(); ++k) eie[(size_t)eie_off[i] + k] = (int32_t)(t.eie[k] + eo);
     const fierro_batch_instance& I = inst[i];
     for (int64_t m = 0; m < I.num_materials; ++m) {
       double* q = &qtab[(size_t)(b->mat_off[i] + m) * 4];
@@ -410,8 +463,6 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
     }
     dtc[i] = I.params.dt_cfl;
   }
-  for (int64_t k = 0; k < NN; ++k) cin_start[k + 1] += cin_start[k];
-  for (int64_t e = 0; e < NE; ++e) eie_start[e + 1] += eie_start[e];
 
   if (stream) {
     b->stream = static_cast<cudaStream_t>(stream);

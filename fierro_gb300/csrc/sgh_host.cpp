@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <numeric>
 #include <vector>
 
@@ -84,22 +85,51 @@ uint64_t spread21(uint64_t v) {
   return v;
 }
 
-// Stable LSD radix sort of indices by 63-bit keys (16-bit digits).
+// Stable LSD radix sort of indices by 63-bit keys: 16-bit digits, 11-bit ones
+// where clearing and summing 65536 counters would outweigh the items.
 std::vector<int64_t> radix_order(const std::vector<uint64_t>& key) {
   const size_t n = key.size();
+  const int bits = n < (1u << 20) ? 11 : 16;
+  const uint64_t mask = (1u << bits) - 1;
   std::vector<int64_t> idx(n), tmp(n);
   std::iota(idx.begin(), idx.end(), 0);
-  std::vector<size_t> cnt(65537);
-  for (int pass = 0; pass < 4; ++pass) {
-    const int sh = pass * 16;
+  std::vector<size_t> cnt((size_t)mask + 2);
+  for (int sh = 0; sh < 63; sh += bits) {
     std::fill(cnt.begin(), cnt.end(), 0);
-    for (size_t i = 0; i < n; ++i) cnt[((key[idx[i]] >> sh) & 0xFFFF) + 1]++;
-    for (size_t d = 0; d < 65536; ++d) cnt[d + 1] += cnt[d];
-    for (size_t i = 0; i < n; ++i) tmp[cnt[(key[idx[i]] >> sh) & 0xFFFF]++] = idx[i];
+    for (size_t i = 0; i < n; ++i) cnt[((key[idx[i]] >> sh) & mask) + 1]++;
+    for (size_t d = 0; d <= mask; ++d) cnt[d + 1] += cnt[d];
+    for (size_t i = 0; i < n; ++i) tmp[cnt[(key[idx[i]] >> sh) & mask]++] = idx[i];
     idx.swap(tmp);
   }
   return idx;
 }
+
+// The elements met so far around one element and which of its nodes each holds
+// (bit l), in a hash table of 256 entries that keeps one free; full() once it
+// cannot take another.
+struct MetElems {
+  int32_t key[256];
+  uint8_t nodes[256];
+  int used[256], count = 0;
+  MetElems() { std::memset(key, 0xFF, sizeof(key)); }
+  bool full() const { return count >= 255; }
+  // The entry of element o; *fresh when this is its first meeting (call only while !full()).
+  int at(int32_t o, bool* fresh) {
+    uint32_t h = (uint32_t)o * 2654435761u >> 24;
+    while (key[h] != o && key[h] >= 0) h = (h + 1) & 255;
+    *fresh = key[h] < 0;
+    if (*fresh) {
+      key[h] = o;
+      nodes[h] = 0;
+      used[count++] = (int)h;
+    }
+    return (int)h;
+  }
+  void clear() {
+    for (int i = 0; i < count; ++i) key[used[i]] = -1;
+    count = 0;
+  }
+};
 
 // Morton keys of points, quantised on the bounding box to 21 bits per axis.
 std::vector<uint64_t> morton_keys(const double* pts, int64_t n) {
@@ -294,38 +324,86 @@ int build_topology(const fierro_mesh* mesh, const fierro_boundary* bcs, int64_t 
     }
   }
   // ---- neighbours: every other element sharing a node (mesh.h:274-322)
-  std::vector<int32_t> cnt((size_t)ne);
-  auto neighbours = [&](int64_t e, int32_t* out) -> int {
-    int k = 0;
-    for (int l = 0; l < 8; ++l) {
-      int32_t n = t->nie[e * 8 + l];
-      for (int32_t c = t->cin_start[n]; c < t->cin_start[n + 1]; ++c) {
-        int32_t o = t->cin[c] >> 3;
-        if (o == e) continue;
-        bool seen = false;
-        for (int i = 0; i < k; ++i)
-          if (out[i] == o) { seen = true; break; }
-        if (!seen && k < 256) out[k++] = o;
+  // Each thread lists a contiguous range's neighbours once, in the order it meets
+  // them (at most 256), and copies its lists into place.  The same meetings tell
+  // the boundary patches: faces whose four nodes no other element holds.
+  t->eie_start.assign((size_t)ne + 1, 0);
+  std::vector<std::vector<int64_t>> patches((size_t)omp_get_max_threads());
+  bool out_of_memory = false;
+#pragma omp parallel
+  {
+    const int64_t nth = omp_get_num_threads(), me = omp_get_thread_num();
+    const int64_t lo = ne * me / nth, hi = ne * (me + 1) / nth;
+    std::vector<int32_t> mine;
+    try {
+      mine.reserve((size_t)(hi - lo) * 27);
+      MetElems met;
+      for (int64_t e = lo; e < hi; ++e) {
+        met.clear();
+        const size_t first = mine.size();
+        for (int l = 0; l < 8; ++l) {
+          const int32_t n = t->nie[e * 8 + l];
+          for (int32_t c = t->cin_start[n]; c < t->cin_start[n + 1]; ++c) {
+            const int32_t o = t->cin[c] >> 3;
+            if (o == e) continue;
+            bool fresh = false;
+            if (!met.full()) met.nodes[met.at(o, &fresh)] |= (uint8_t)(1u << l);
+            else if (mine.size() - first < 256) fresh = std::find(mine.begin() + first, mine.end(), o) == mine.end();
+            if (fresh) mine.push_back(o);
+          }
+        }
+        t->eie_start[e + 1] = (int32_t)(mine.size() - first);
+        for (int f = 0; f < 6; ++f) {
+          bool shared = false;
+          if (!met.full()) {
+            uint8_t face = 0;
+            for (int k = 0; k < 4; ++k) face |= (uint8_t)(1u << hex::PATCH[f][k]);
+            for (int i = 0; i < met.count && !shared; ++i) shared = (met.nodes[met.used[i]] & face) == face;
+          } else {
+            const int32_t a = t->nie[e * 8 + hex::PATCH[f][0]];
+            for (int32_t c = t->cin_start[a]; c < t->cin_start[a + 1] && !shared; ++c) {
+              const int32_t o = t->cin[c] >> 3;
+              int held = 0;
+              for (int k = 1; k < 4; ++k)
+                for (int m = 0; m < 8; ++m) held += t->nie[(int64_t)o * 8 + m] == t->nie[e * 8 + hex::PATCH[f][k]];
+              shared = o != e && held == 3;
+            }
+          }
+          if (!shared) patches[(size_t)me].push_back(e * 6 + f);
+        }
+      }
+    } catch (const std::bad_alloc&) {
+#pragma omp critical
+      out_of_memory = true;
+    }
+#pragma omp barrier
+#pragma omp single
+    if (!out_of_memory) {
+      for (int64_t e = 0; e < ne; ++e) t->eie_start[e + 1] += t->eie_start[e];
+      try {
+        t->eie.resize((size_t)t->eie_start[ne]);
+      } catch (const std::bad_alloc&) {
+        out_of_memory = true;
       }
     }
-    return k;
-  };
-#pragma omp parallel for schedule(static)
-  for (int64_t e = 0; e < ne; ++e) {
-    int32_t buf[256];
-    cnt[e] = neighbours(e, buf);
+    if (!out_of_memory) std::copy(mine.begin(), mine.end(), t->eie.begin() + t->eie_start[lo]);
   }
-  t->eie_start.assign((size_t)ne + 1, 0);
-  for (int64_t e = 0; e < ne; ++e) t->eie_start[e + 1] = t->eie_start[e] + cnt[e];
-  t->eie.resize((size_t)t->eie_start[ne]);
-#pragma omp parallel for schedule(static)
-  for (int64_t e = 0; e < ne; ++e) neighbours(e, t->eie.data() + t->eie_start[e]);
-  // ---- boundary masks
-  std::vector<uint8_t> mask_ext;
-  rc = boundary_masks(mesh, bcs, num_bcs, mesh->coords, &mask_ext, nullptr);
-  if (rc) return rc;
-  t->bc_mask.resize((size_t)nn);
-  for (int64_t n = 0; n < nn; ++n) t->bc_mask[n] = mask_ext[t->node_int2ext[n]];
+  if (out_of_memory) return set_error(FIERRO_ENOMEM, "host allocation failed");
+  // ---- boundary masks: the nodes of every patch that lies on a condition's surface
+  t->bc_mask.assign((size_t)nn, 0);
+  for (int64_t s = 0; s < num_bcs; ++s) {
+    const uint8_t bits = bc_mask_bits(bcs[s].hydro_bc, bcs[s].surface, 3);
+    for (const auto& v : patches)
+      for (int64_t pf : v) {
+        const int32_t* n = &t->nie[(size_t)(pf / 6) * 8];
+        const int* lid = hex::PATCH[pf % 6];
+        bool all = true;
+        for (int k = 0; k < 4 && all; ++k)
+          all = node_on_surface(mesh->coords + t->node_int2ext[n[lid[k]]] * 3, bcs[s].surface, bcs[s].value);
+        if (all)
+          for (int k = 0; k < 4; ++k) t->bc_mask[n[lid[k]]] |= bits;
+      }
+  }
   return FIERRO_OK;
 }
 
