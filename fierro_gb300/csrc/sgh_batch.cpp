@@ -79,7 +79,8 @@ struct fierro_batch {
   size_t stage_elems = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   // launch shape of the cycle kernels (fierro_batch_set_shape / fierro_batch_autotune)
-  fierro_batch_shape shape{kForceBlock, kNodeBlock, kElemBlock, 0, 0};
+  // and the one launched: `shape` once it was set, before that smaller blocks for a small batch
+  fierro_batch_shape shape{kForceBlock, kNodeBlock, kElemBlock, 0, 0}, launch = shape;
   int sm_count = 0;
   std::vector<fierro_batch_shape> tune_shapes;
   std::vector<double> tune_ms;
@@ -106,6 +107,13 @@ int put(fierro_batch* b, T* dst, const std::vector<T>& src) {
   CUDA_TRY(cudaStreamSynchronize(b->stream));
   return FIERRO_OK;
 }
+
+// Until a shape is set, a batch of fewer elements launches one-warp element blocks
+// and small node blocks, which fall more evenly on the SMs.  us a cycle, {128, 256, 128} against
+// {32, 64, 32}: 22,700 elements 142.6 / 112.4 FMA, 194 / 148 exact; 148,000 543.8 /
+// 533.4, 762 / 754; 305,000 1011 / 1004, 1447 / 1418; in larger ones the shapes
+// differ by the last wave alone and blocks of 128 leave fewer CFL partials.
+constexpr int64_t kSmallBatch = 1 << 19;
 
 // Values a host loop over one instance's array shares among the threads from.
 constexpr int64_t kHostParallel = 4096;
@@ -134,15 +142,15 @@ int scatter_down(fierro_batch* b, double* out, const double* src, int64_t off, c
 // A persistent grid fills every SM `shape.persistent` times over with the
 // kernel's resident blocks at this block size; 0 = one block per tile.
 int persistent_grid(const fierro_batch* b, int kernel, int block) {
-  if (!b->shape.persistent) return 0;
-  return b->sm_count * b->ks->batch_max_blocks(kernel, block) * b->shape.persistent;
+  if (!b->launch.persistent) return 0;
+  return b->sm_count * b->ks->batch_max_blocks(kernel, block) * b->launch.persistent;
 }
 
 // A fused stage whose grid barrier gave up waiting (never expected: the launch
 // is cooperative) leaves results that cannot be trusted: report it, and reset
 // the barrier for the next launch.  Call with the stream idle.
 int check_sync(fierro_batch* b) {
-  if (!b->shape.fused_stage) return FIERRO_OK;
+  if (!b->launch.fused_stage) return FIERRO_OK;
   unsigned int st = 0;
   CUDA_TRY(cudaMemcpy(&st, b->d_sync + 2, sizeof(st), cudaMemcpyDeviceToHost));
   if (st == 0) return FIERRO_OK;
@@ -161,8 +169,8 @@ int fused_oversubscribe() {
   return k > 1 && k <= 16 ? k : 0;
 }
 int fused_grid(const fierro_batch* b) {
-  const long long tiles = b->NE / b->shape.elem_block;
-  const long long resident = (long long)b->sm_count * b->ks->fused_max_blocks(b->shape.elem_block);
+  const long long tiles = b->NE / b->launch.elem_block;
+  const long long resident = (long long)b->sm_count * b->ks->fused_max_blocks(b->launch.elem_block);
   if (const int k = fused_oversubscribe()) return (int)std::max<long long>(1, resident * k);
   return (int)std::max<long long>(1, std::min(tiles, resident));
 }
@@ -189,8 +197,8 @@ ForceArgs b_force(fierro_batch* b, int rb, int q) {
   a.inst = b->d_inst_e;
   a.fuzz = b->fuzz;
   a.small = b->small;
-  a.block = b->shape.force_block;
-  a.grid = persistent_grid(b, 0, b->shape.force_block);
+  a.block = b->launch.force_block;
+  a.grid = persistent_grid(b, 0, b->launch.force_block);
   return a;
 }
 
@@ -222,8 +230,8 @@ NodeArgs b_node(fierro_batch* b, int c, double alpha) {
   a.ctrl = b->d_ctrl;
   a.inst = b->d_inst_n;
   a.rk_alpha = alpha;
-  a.block = b->shape.node_block;
-  a.grid = persistent_grid(b, 1, b->shape.node_block);
+  a.block = b->launch.node_block;
+  a.grid = persistent_grid(b, 1, b->launch.node_block);
   return a;
 }
 
@@ -258,8 +266,8 @@ ElemArgs b_elem(fierro_batch* b, int cur_bin, int c, double alpha, int div_out) 
   a.dt_cfl_tab = b->d_dt_cfl;
   a.rk_alpha = alpha;
   a.fuzz = b->fuzz;
-  a.block = b->shape.elem_block;
-  a.grid = persistent_grid(b, 2, b->shape.elem_block);
+  a.block = b->launch.elem_block;
+  a.grid = persistent_grid(b, 2, b->launch.elem_block);
   return a;
 }
 
@@ -277,7 +285,7 @@ void b_cycle(fierro_batch* b, int c) {
     const double alpha = 1.0 / ((double)S - (double)s);  // sgh_solve.cpp:353
     const int rb = (s == 0) ? c : (c ^ 1);
     const int q = (c * S + s) & 1;
-    if (b->shape.fused_stage) {
+    if (b->launch.fused_stage) {
       // one cooperative launch for the stage, its barrier's arrival count reset first
       ForceArgs fa = b_force(b, rb, q);
       NodeArgs na = b_node(b, c, alpha);
@@ -306,14 +314,14 @@ bool shape_valid(const fierro_batch_shape& sh) {
          sh.persistent >= 0 && sh.persistent <= 8 && (sh.fused_stage == 0 || sh.fused_stage == 1);
 }
 
-// Makes `sh` the batch's launch shape: the per-instance CFL partial ranges in
+// Makes `sh` what the batch launches: the per-instance CFL partial ranges in
 // tiles of sh.elem_block elements, and the two per-parity cycle graphs.
-int apply_shape(fierro_batch* b, const fierro_batch_shape& sh) {
+int apply_launch(fierro_batch* b, const fierro_batch_shape& sh) {
   if (!shape_valid(sh))
     return set_error(FIERRO_EINVAL, "batch shape: blocks must be powers of two, force 32..%d, node 32..1024, "
                      "element 32..%d, persistent 0..8 fills of the SMs, fused_stage 0 or 1", kForceBlock, kElemBlock);
   CUDA_TRY(cudaStreamSynchronize(b->stream));
-  b->shape = sh;
+  b->launch = sh;
   for (size_t i = 0; i < b->part_start.size(); ++i)
     b->part_start[i] = (int)(b->elem_off[i] / sh.elem_block);
   b->nparts = b->part_start.back();
@@ -333,6 +341,13 @@ int apply_shape(fierro_batch* b, const fierro_batch_shape& sh) {
     if (g) cudaGraphDestroy(g);
     if (err != cudaSuccess) return set_error(FIERRO_ECUDA, "batch cycle graph: %s", cudaGetErrorString(err));
   }
+  return FIERRO_OK;
+}
+
+// Makes `sh` the batch's shape, launched as it is.
+int apply_shape(fierro_batch* b, const fierro_batch_shape& sh) {
+  TRY(apply_launch(b, sh));
+  b->shape = sh;
   return FIERRO_OK;
 }
 
@@ -536,7 +551,7 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   CUDA_TRY(cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, dev));
-  TRY(apply_shape(b, b->shape));
+  TRY(apply_launch(b, NE < kSmallBatch ? fierro_batch_shape{32, 64, 32, 0, 0} : b->shape));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
   return FIERRO_OK;
 }
@@ -792,7 +807,7 @@ extern "C" int fierro_batch_autotune(fierro_batch* b, int64_t cycles, fierro_bat
   b->tune_shapes.clear();
   b->tune_ms.clear();
   int rc = copy_arrays(b, save, arrs, true);
-  const fierro_batch_shape start = b->shape;
+  const fierro_batch_shape start = b->shape, start_launch = b->launch;
   fierro_batch_shape best = b->shape;
   double best_ms = 0.0;
   bool have = false;
@@ -857,7 +872,8 @@ extern "C" int fierro_batch_autotune(fierro_batch* b, int64_t cycles, fierro_bat
   cudaStreamSynchronize(b->stream);
   cudaFree(save);
   if (rc) {
-    apply_shape(b, start);
+    apply_launch(b, start_launch);
+    b->shape = start;
     return rc;
   }
   if (rc_restore) return rc_restore;

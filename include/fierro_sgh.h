@@ -278,7 +278,8 @@ int64_t fierro_batch_device_bytes(const fierro_batch* b);
  * grid barrier, element pass; the other blocks and `persistent` are then
  * unused).  Results do not depend on the shape (every element and node runs the
  * same arithmetic; the CFL minimum is order-independent).
- * Default {128, 256, 128, 0, 0}. */
+ * Default {128, 256, 128, 0, 0}; until a shape is set or tuned, a batch of fewer
+ * than 2^19 (padded) elements launches smaller blocks than it says. */
 typedef struct {
   int force_block;
   int node_block;
