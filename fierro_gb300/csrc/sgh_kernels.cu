@@ -789,15 +789,17 @@ __global__ void __launch_bounds__(kEnergyBlock) k_energy_part(const EnergyArgs a
   }
 }
 
-__global__ void k_energy_final(const EnergyArgs a, int nblocks) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double ie = 0.0, ke = 0.0;
-  for (int b = 0; b < nblocks; ++b) {
-    ie += a.part[b];
-    ke += a.part[nblocks + b];
-  }
-  a.out[0] = ie;
-  a.out[1] = 0.5 * ke;
+// One warp's two lanes add the blocks' partials in order, energies and kinetic
+// energies in the same instructions.
+__global__ void __launch_bounds__(2 * kEnergyMaxBlocks) k_energy_final(const EnergyArgs a, int nblocks) {
+  __shared__ double sh[2 * kEnergyMaxBlocks];
+  if (threadIdx.x < 2 * nblocks) sh[threadIdx.x] = a.part[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x >= 2) return;
+  const double* p = sh + threadIdx.x * nblocks;
+  double t = 0.0;
+  for (int b = 0; b < nblocks; ++b) t += p[b];
+  a.out[threadIdx.x] = threadIdx.x ? 0.5 * t : t;
 }
 
 // ---------------------------------------------------------------------------
@@ -995,9 +997,9 @@ static int fused_max_blocks(int block) {
   return n0 < n1 ? n0 : n1;
 }
 static void launch_energy(const EnergyArgs& a, cudaStream_t s) {
-  const int nb = 512;
+  const int nb = energy_blocks(a.ne, a.nn);
   k_energy_part<<<nb, kEnergyBlock, 0, s>>>(a);
-  k_energy_final<<<1, 32, 0, s>>>(a, nb);
+  k_energy_final<<<1, 2 * kEnergyMaxBlocks, 0, s>>>(a, nb);
 }
 
 }  // namespace FIERRO_IMPL

@@ -569,15 +569,17 @@ __global__ void __launch_bounds__(kRzEnergyBlock) k_energy_rz_part(const RzEnerg
   }
 }
 
-__global__ void k_energy_rz_final(const RzEnergyArgs a, int nblocks) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double ie = 0.0, ke = 0.0;
-  for (int b = 0; b < nblocks; ++b) {
-    ie += a.part[b];
-    ke += a.part[nblocks + b];
-  }
-  a.out[0] = ie;
-  a.out[1] = 0.5 * ke;
+// One warp's two lanes add the blocks' partials in order, energies and kinetic
+// energies in the same instructions.
+__global__ void __launch_bounds__(2 * kEnergyMaxBlocks) k_energy_rz_final(const RzEnergyArgs a, int nblocks) {
+  __shared__ double sh[2 * kEnergyMaxBlocks];
+  if (threadIdx.x < 2 * nblocks) sh[threadIdx.x] = a.part[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x >= 2) return;
+  const double* p = sh + threadIdx.x * nblocks;
+  double t = 0.0;
+  for (int b = 0; b < nblocks; ++b) t += p[b];
+  a.out[threadIdx.x] = threadIdx.x ? 0.5 * t : t;
 }
 
 // ---------------------------------------------------------------------------
@@ -614,9 +616,9 @@ static void launch_ext(int nn, const double* node_mass, const double* y, double*
   k_ext_rz<<<blocks_for(nn, kRzNodeBlock), kRzNodeBlock, 0, s>>>(nn, node_mass, y, ext);
 }
 static void launch_energy(const RzEnergyArgs& a, cudaStream_t s) {
-  const int nb = 512;
+  const int nb = energy_blocks(a.ne, a.nn);
   k_energy_rz_part<<<nb, kRzEnergyBlock, 0, s>>>(a);
-  k_energy_rz_final<<<1, 32, 0, s>>>(a, nb);
+  k_energy_rz_final<<<1, 2 * kEnergyMaxBlocks, 0, s>>>(a, nb);
 }
 
 }  // namespace FIERRO_RZ_IMPL
