@@ -156,17 +156,14 @@ __device__ __forceinline__ double corner_impedance(const Impedance& z, double d0
 // Shock detector (force_sgh.cpp:287-315): r_face = 0.9 (div_nb + small) / (div + small)
 // is monotone in div_nb (non-decreasing for div + small > 0, non-increasing for < 0),
 // so the minimum over neighbours is attained at the smallest (resp. largest)
-// neighbour divergence (keys kmin, kmax) and needs one division instead of one
-// per neighbour.
-__device__ __forceinline__ double limiter_min(const ForceArgs& a, double div, int k0, int k1, long long kmin,
-                                              long long kmax) {
-  const double D = div + a.small;
+// neighbour divergence dsel and needs one division (r_face) instead of one per
+// neighbour; D = div + small.
+__device__ __forceinline__ double limiter_min(const ForceArgs& a, double D, double dsel, double r_face, int k0,
+                                              int k1) {
   double r_min = 1.0;
   if (k1 > k0) {
-    const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
     const bool regular = is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel);
     if (regular) {
-      const double r_face = newton_div(0.9 * (dsel + a.small), D);
       r_min = okey(r_face) < okey(1.0) ? r_face : 1.0;
     } else {
       for (int k = k0; k < k1; ++k) {
@@ -177,13 +174,8 @@ __device__ __forceinline__ double limiter_min(const ForceArgs& a, double div, in
   }
   return r_min;
 }
-// Mach-number detector (force_sgh.cpp:318-328)
-__device__ __forceinline__ double mach_switch(double vol, double div, double sspd, double fuzz) {
-  return at_most_1(newton_div(20.0 * (pow_third(vol) * fabs(div)), sspd + fuzz));
-}
 // Divergence from the velocity sums (momentum.cpp:265-286)
-__device__ __forceinline__ double divergence(double Sx, double Sy, double Sz, double vol) {
-  const double inverse_vol = mode_rcp(vol);
+__device__ __forceinline__ double divergence(double Sx, double Sy, double Sz, double inverse_vol) {
   double div = 0.0;
   div = mul_add(div, Sx, inverse_vol);
   div = mul_add(div, Sy, inverse_vol);
@@ -193,7 +185,7 @@ __device__ __forceinline__ double divergence(double Sx, double Sy, double Sz, do
 // Order key of the element CFL step dt_cfl * min distance / (c + fuzz)
 // (time_integration.cpp:124-131); a NaN bounds nothing.
 __device__ __forceinline__ long long cfl_key(double d2min, double sspd, double dt_cfl, double fuzz) {
-  const double dt_l = mode_div(dt_cfl * mode_sqrt(d2min), sspd + fuzz);
+  const double dt_l = newton_div(dt_cfl * mode_sqrt(d2min), sspd + fuzz);
   return (__double_as_longlong(dt_l) & kAbsMask) > 0x7FF0000000000000LL ? 0x7FFFFFFFFFFFFFFFLL : okey(dt_l);
 }
 
@@ -282,7 +274,8 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     kmin = key < kmin ? key : kmin;
     kmax = key > kmax ? key : kmax;
   }
-  const double r_min = limiter_min(a, div, k0, k1, kmin, kmax);
+  const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
+  const double r_min = limiter_min(a, D, dsel, newton_div(0.9 * (dsel + small), D), k0, k1);
   double phi = 1.0 - at_least_0(r_min);  // pow(phi, 1.0) == phi
   // Mach-number detector (:318-328)
   const double c_length = pow_third(vol);
@@ -556,7 +549,7 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
     // the priming pass keeps the uploaded volume, as get_divergence reads elem_vol
     const double vol = (KIND == 2) ? a.vol[e] : vol_geo;
     // divergence for the next stage (momentum.cpp:265-286), with this geometry
-    const double div = divergence(Sx, Sy, Sz, vol);
+    const double div = divergence(Sx, Sy, Sz, mode_rcp(vol));
     a.div[e] = div;
     double sspd;
     if (KIND != 2) {

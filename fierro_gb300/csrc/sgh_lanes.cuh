@@ -172,18 +172,23 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   for (int k = 0; k < 8; ++k) s = s + sv[r][k];
 #endif
   const double s3 = from_lane(s, 3);
-  double vstar = 0.0;
-  if (s3 > a.fuzz) {
-#if FIERRO_FMA
-    vstar = s * mode_rcp(s3);
-#else
-    vstar = quot(s, divisor(s3));
-#endif
-  }
+  // the element's quotients in different lanes of the same instructions: the
+  // Riemann velocity's (0-2), the limiter's (3), the Mach switch's (4 and on)
+  const double D = div + a.small;
+  const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
+  const double mach = 20.0 * (pow_third(vol) * fabs(div));
   __syncwarp();
+#if FIERRO_FMA
+  const double num = l < 3 ? 1.0 : l == 3 ? 0.9 * (dsel + a.small) : mach;
+#else
+  const double num = l < 3 ? s : l == 3 ? 0.9 * (dsel + a.small) : mach;
+#endif
+  const double qt = newton_div(num, l < 3 ? s3 : l == 3 ? D : sspd + a.fuzz);
+  __syncwarp();
+  const double vstar = !(s3 > a.fuzz) ? 0.0 : FIERRO_FMA ? s * qt : qt;
   const double vstar0 = from_lane(vstar, 0), vstar1 = from_lane(vstar, 1), vstar2 = from_lane(vstar, 2);
-  const double r_min = limiter_min(a, div, k0, k1, kmin, kmax);
-  const double phi = mach_switch(vol, div, sspd, a.fuzz) * (1.0 - at_least_0(r_min));
+  const double r_min = limiter_min(a, D, dsel, from_lane(qt, 3), k0, k1);
+  const double phi = at_most_1(from_lane(qt, 4)) * (1.0 - at_least_0(r_min));
   const double pm = phi * mu;
   if (!live) return;
   a.force[(size_t)(l * 3 + 0) * ne + e] = mul_mul(b0, pres, pm, vstar0 - vu);
@@ -266,7 +271,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_elem_lanes(const ElemArgs a) {
     h[1] = a.hy[n];
     h[2] = a.hz[n];
   }
-  const double mass = KIND != 2 ? a.mass[e] : 0.0, sie0 = KIND != 2 ? a.sie0[e] : 0.0;
+  const double mass = KIND != 2 ? a.mass[e] : 1.0, sie0 = KIND != 2 ? a.sie0[e] : 0.0;
   const double gamma = KIND != 2 ? a.gamma[e] : 0.0, csmin = KIND != 2 ? a.csmin[e] : 0.0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) s.x[d][l] = x[d];
@@ -375,13 +380,16 @@ __global__ void __launch_bounds__(kLaneBlock) k_elem_lanes(const ElemArgs a) {
   const double vol_geo = FX_MUL(from_lane(acc, 3), twelth);
   const double power = from_lane(acc, 4);
   const double vol = (KIND == 2) ? a.vol[e] : vol_geo;
-  const double div = divergence(Sx, Sy, Sz, vol);
+  // three quotients at once: 1 / vol, dt / mass, mass / vol
+  const double adt = KIND != 2 ? a.rk_alpha * a.ctrl->dt : 0.0;
+  const double qt = newton_div(l == 0 ? 1.0 : l == 1 ? adt : mass, l == 1 ? mass : vol);
+  __syncwarp();
+  const double div = divergence(Sx, Sy, Sz, from_lane(qt, 0));
   double sspd;
   const bool writer = live && l == 0;
   if (KIND != 2) {
-    const double adt = a.rk_alpha * a.ctrl->dt;
-    const double sie1 = sie0 - FX_MUL(mode_div(adt, mass), power);
-    const double den = mode_div(mass, vol);
+    const double sie1 = sie0 - FX_MUL(from_lane(qt, 1), power);
+    const double den = from_lane(qt, 2);
     const double pres = (gamma - 1.0) * sie1 * den;
     sspd = mode_sqrt(gamma * (gamma - 1.0) * sie1);
     if (sspd < csmin) sspd = csmin;
