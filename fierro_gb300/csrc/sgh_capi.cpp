@@ -400,7 +400,7 @@ static int create_impl(fierro_sgh* h, const fierro_mesh* mesh, const fierro_mate
   h->blk_elem = small_mesh_block(ne, kElemBlock);
   h->blk_force = small_mesh_block(ne, kForceBlock);
   h->blk_node = small_mesh_block(nn, kNodeBlock);
-  h->lanes_force = (long long)ne <= kLanesForce && !h->strength;
+  h->lanes_force = (long long)ne <= kLanesForce;
   h->lanes_node = (long long)nn <= kLanesNode;
   h->lanes_elem = (long long)ne <= kLanesElem && !h->has_hyper;
   h->cfl_tile = h->lanes_elem ? kLaneTile : h->blk_elem;

@@ -81,7 +81,7 @@ struct ForceArgs {
   const double* sie0;  // cycle-start energy (the reference passes elem_sie bin 0)
   double rk_alpha;
   int copy_stress;     // stage 0: elements without a hypo model carry stress_cur over
-  int lanes;           // eight lanes per element (small gas-only meshes, sgh_lanes.cuh)
+  int lanes;           // eight lanes per element (small meshes, sgh_lanes.cuh)
   int block;           // threads per block (0: kForceBlock)
   int grid;            // batch only: blocks of a persistent grid (0: one block per tile)
 };

@@ -108,18 +108,18 @@ __device__ __forceinline__ void velocity_gradient(const double (&u)[8], const do
   const double inverse_vol = mode_rcp(vol);
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    double b = bmat[(size_t)j * ne + e];
-    double su = u[0] * b, sv = v[0] * b, sw = w[0] * b;
+    const double b0 = bmat[(size_t)j * ne + e], b1 = bmat[(size_t)(3 + j) * ne + e];
+    double su = mul_mul(u[0], b0, u[1], b1), sv = mul_mul(v[0], b0, v[1], b1), sw = mul_mul(w[0], b0, w[1], b1);
 #pragma unroll
-    for (int l = 1; l < 8; ++l) {
-      b = bmat[(size_t)(l * 3 + j) * ne + e];
-      su = su + u[l] * b;
-      sv = sv + v[l] * b;
-      sw = sw + w[l] * b;
+    for (int l = 2; l < 8; ++l) {
+      const double b = bmat[(size_t)(l * 3 + j) * ne + e];
+      su = mul_add(su, u[l], b);
+      sv = mul_add(sv, v[l], b);
+      sw = mul_add(sw, w[l], b);
     }
-    L[j] = su * inverse_vol;
-    L[3 + j] = sv * inverse_vol;
-    L[6 + j] = sw * inverse_vol;
+    L[j] = FX_MUL(su, inverse_vol);  // rounded before the model's sums, as the lane pass has them
+    L[3 + j] = FX_MUL(sv, inverse_vol);
+    L[6 + j] = FX_MUL(sw, inverse_vol);
   }
 }
 
@@ -383,7 +383,7 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
 #pragma unroll
       for (int d = 0; d < 3; ++d)
         a.force[(size_t)(l * 3 + d) * ne + e] =
-            a0 * tau[d] + a1 * tau[3 + d] + a2 * tau[6 + d] + pm * (vs[d] - vl[d]);
+            mul_add(mul_add(mul_mul(a0, tau[d], a1, tau[3 + d]), a2, tau[6 + d]), pm, vs[d] - vl[d]);
     }
     // stress update of hypo materials (:362-391); the others carry stress(1) over
     // from the cycle-start bin on the first stage (rk_init's copy)
@@ -811,7 +811,8 @@ static unsigned grid_or(int grid, unsigned blocks) {
 static void launch_force(const ForceArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);
   const unsigned g = blocks_for(a.ne, bs);
-  if (a.lanes) launch(k_force_lanes, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
+  if (a.lanes && a.stress_out) launch(k_force_lanes<true>, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
+  else if (a.lanes) launch(k_force_lanes<false>, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
   else if (a.inst) launch(k_force<true, false, false>, grid_or(a.grid, g), bs, s, a);
   else if (a.stress_out) launch(k_force<false, false, true>, g, bs, s, a);
   else launch(k_force<false, false, false>, g, bs, s, a);

@@ -112,6 +112,10 @@ constexpr int kLaneWarps = kLaneBlock / 32;
 constexpr int kGroups = 4;                   // elements per warp
 
 // ---------------------------------------------------------------------------
+// STRENGTH as in force_elem: each lane reads one stress component (lane 0 the
+// ninth too), the velocity gradient's nine sums run in the eight lanes (one twice),
+// and lane 0 runs the model.
+template <bool STRENGTH>
 __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   // per element: the corners' velocities and impedance terms, rows u, v, w, mu
   __shared__ double s_v[kLaneWarps][kGroups][4][9];
@@ -190,10 +194,61 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   const double r_min = limiter_min(a, D, dsel, from_lane(qt, 3), k0, k1);
   const double phi = at_most_1(from_lane(qt, 4)) * (1.0 - at_least_0(r_min));
   const double pm = phi * mu;
-  if (!live) return;
-  a.force[(size_t)(l * 3 + 0) * ne + e] = mul_mul(b0, pres, pm, vstar0 - vu);
-  a.force[(size_t)(l * 3 + 1) * ne + e] = mul_mul(b1, pres, pm, vstar1 - vv);
-  a.force[(size_t)(l * 3 + 2) * ne + e] = mul_mul(b2, pres, pm, vstar2 - vw);
+  if constexpr (!STRENGTH) {
+    if (!live) return;
+    a.force[(size_t)(l * 3 + 0) * ne + e] = mul_mul(b0, pres, pm, vstar0 - vu);
+    a.force[(size_t)(l * 3 + 1) * ne + e] = mul_mul(b1, pres, pm, vstar1 - vv);
+    a.force[(size_t)(l * 3 + 2) * ne + e] = mul_mul(b2, pres, pm, vstar2 - vw);
+  } else {
+    // per element: stress(1), then the corners' velocities and normals and L
+    __shared__ double s_t[kLaneWarps][kGroups][3 * 9 + 2 * 27 + 1];
+    double* st = s_t[threadIdx.x >> 5][lane >> 3];
+    double *tau = st, *L = st + 9, *sb = st + 27, *sw = st + 54;
+    const double mine = a.stress_cur[(size_t)l * ne + e];
+    const double ninth = l == 0 ? a.stress_cur[(size_t)8 * ne + e] : 0.0;
+    tau[l] = (l & 3) == 0 ? mine - pres : mine;
+    if (l == 0) tau[8] = ninth - pres;
+    sb[l] = b0, sb[9 + l] = b1, sb[18 + l] = b2;
+    sw[l] = vu, sw[9 + l] = vv, sw[18 + l] = vw;
+    __syncwarp();
+    const double vs[3] = {vstar0, vstar1, vstar2}, vl[3] = {vu, vv, vw};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double f = mul_add(mul_add(mul_mul(-b0, tau[d], -b1, tau[3 + d]), -b2, tau[6 + d]), pm, vs[d] - vl[d]);
+      if (live) a.force[(size_t)(l * 3 + d) * ne + e] = f;
+    }
+    const int mat = a.mat[e];
+    const bool hypo = a.stype[mat] == 1;  // the same in an element's eight lanes
+    const double inverse_vol = mode_rcp(vol);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int k = i == 0 ? l : 8;
+      const double *x = sw + 9 * (k / 3), *y = sb + 9 * (k % 3);
+      double t = mul_mul(x[0], y[0], x[1], y[1]);
+#pragma unroll
+      for (int m = 2; m < 8; ++m) t = mul_add(t, x[m], y[m]);
+      L[k] = FX_MUL(t, inverse_vol);
+    }
+    __syncwarp();
+    if (!live) return;
+    if (hypo) {
+      if (l != 0) return;
+      double sc[9], s0[9], G[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        sc[k] = a.stress_cur[(size_t)k * ne + e];
+        s0[k] = a.stress0[(size_t)k * ne + e];
+        G[k] = L[k];
+      }
+      user_strength_model(sc, s0, G, a.statev + e, ne, mat, den, a.sie0[e], vol, a.ctrl->dt, a.rk_alpha);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) a.stress_out[(size_t)k * ne + e] = sc[k];
+    } else if (a.copy_stress) {
+      a.stress_out[(size_t)l * ne + e] = mine;
+      if (l == 0) a.stress_out[(size_t)8 * ne + e] = ninth;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
