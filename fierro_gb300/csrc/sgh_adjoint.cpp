@@ -193,7 +193,7 @@ int ensure(fierro_sgh* h, int k, int nseg) {
     for (int d = 0; d < 6; ++d)
       if ((rc = aalloc(a, &a->an[i][d], nn))) return fail(rc);
   }
-  const int be = small_mesh_block(ne, kAdjElemBlock), bn = small_mesh_block(nn, kAdjNodeBlock);
+  const int be = (long long)ne <= kLanesAdjoint ? kAdjLaneTile : small_mesh_block(ne, kAdjElemBlock), bn = small_mesh_block(nn, kAdjNodeBlock);
   b.nbe = (int)((ne + be - 1) / be);
   b.nbn = (int)((nn + bn - 1) / bn);
   if ((rc = aalloc(a, &b.part_e, (size_t)S * b.nbe))) return fail(rc);
@@ -217,6 +217,7 @@ int ensure(fierro_sgh* h, int k, int nseg) {
   m.node_mass = h->d_node_mass;
   m.gamma = h->d_gamma;
   m.csmin = h->d_csmin;
+  m.lanes = (long long)ne <= kLanesAdjoint;
   return FIERRO_OK;
 }
 
@@ -290,6 +291,7 @@ int replay_segment(fierro_sgh* h, AdjState* a, int g, int n) {
       fa.small = h->lp.small;
       fa.tape = a->ftape + (size_t)j * kForceTapeRows * ne;
       fa.tape_sel = a->fsel + (size_t)j * ne;
+      fa.lanes = h->lanes_force;
       fa.block = h->blk_force;
       h->ks->force_tape(fa, st);
       NodeArgs na{};

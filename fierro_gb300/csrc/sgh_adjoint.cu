@@ -30,6 +30,7 @@
 #include <cstdint>
 
 #include "sgh_adjoint.h"
+#include "sgh_hex.h"
 
 #define FIERRO_FMA 0
 
@@ -39,6 +40,7 @@ namespace adj_impl {
 #include "sgh_common.cuh"
 #include "sgh_hex_geometry.cuh"
 #include "sgh_cfl.cuh"
+#include "sgh_lane_tables.cuh"
 
 constexpr int kAdjForceBlock = 128;
 constexpr long long kMaxKey = 0x7FFFFFFFFFFFFFFFLL;
@@ -630,6 +632,8 @@ __global__ void __launch_bounds__(kAdjForceBlock, 3) k_adj_force(const AdjMesh m
   b.gbar[e] += gb;
 }
 
+#include "sgh_adjoint_lanes.cuh"
+
 // ---------------------------------------------------------------------------
 // dt and time bookkeeping of one cycle in reverse (time_integration.cpp:54-154,
 // sgh_solve.cpp:590-632).  dt = rk_alpha-weighted sum of the stages' partial
@@ -825,11 +829,19 @@ static void launch_seed(const AdjMesh& m, const AdjBufs& b, const Slot& fin, con
 static void launch_elem(const AdjMesh& m, const AdjBufs& b, const Slot& s1, const double* force,
                         const AdjRecord* r, double alpha, const double* sie_in, double* sie_c, int assign,
                         double* part, int kind, cudaStream_t st) {
+  if (m.lanes) {
+    const unsigned gl = blocks_for(8LL * m.ne, kLaneBlock);
+    if (kind == 2)
+      k_adj_elem_lanes<2><<<gl, kLaneBlock, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
+    else k_adj_elem_lanes<0><<<gl, kLaneBlock, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
+    return;
+  }
   const int bs = small_mesh_block(m.ne, kAdjElemBlock);
   const unsigned g = blocks_for(m.ne, bs);
   if (kind == 2) k_adj_elem<2><<<g, bs, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
   else k_adj_elem<0><<<g, bs, 0, st>>>(m, b, s1, force, r, alpha, sie_in, sie_c, assign, part);
 }
+static_assert(kAdjLaneTile * 8 == kLaneBlock, "one partial per block of the lane pass");
 static void launch_node(const AdjMesh& m, const AdjBufs& b, const Slot& s1, const double* force,
                         const AdjRecord* r, double alpha, const Node6& an_in, const Node6& an_c, int assign,
                         double* part, cudaStream_t st) {
@@ -839,6 +851,11 @@ static void launch_node(const AdjMesh& m, const AdjBufs& b, const Slot& s1, cons
 static void launch_force(const AdjMesh& m, const AdjBufs& b, const Slot& s0, const Slot& s1,
                          const double* force_tape, const double* ft, const int* fsel, double fuzz, double small,
                          double* sie_out, int accumulate, cudaStream_t st) {
+  if (m.lanes) {
+    k_adj_force_lanes<<<blocks_for(8LL * m.ne, kLaneBlock), kLaneBlock, 0, st>>>(m, b, s0, s1, force_tape, ft, fsel, fuzz,
+                                                                                small, sie_out, accumulate);
+    return;
+  }
   const int bs = small_mesh_block(m.ne, kAdjForceBlock);
   k_adj_force<<<blocks_for(m.ne, bs), bs, 0, st>>>(m, b, s0, s1, force_tape, ft, fsel, fuzz, small, sie_out,
                                                    accumulate);

@@ -36,6 +36,11 @@ namespace fierro {
 // leave one partial sum each (smaller on small meshes: small_mesh_block).
 constexpr int kAdjElemBlock = 128;
 constexpr int kAdjNodeBlock = 256;
+// Meshes of at most kLanesAdjoint elements run the reverse element and force
+// passes with eight lanes per element (sgh_adjoint_lanes.cuh), kAdjLaneTile elements
+// a block.  us a backward cycle, one thread per element against eight lanes: 9^3
+// 225 / 136, 16^3 239 / 167, 20^3 269 / 233, 22^3 307 / 300, 24^3 311 / 329, 32^3 450 / 583.
+constexpr int kLanesAdjoint = 10500, kAdjLaneTile = 8;
 
 struct Slot {
   double *x, *y, *z, *u, *v, *w;
@@ -72,6 +77,7 @@ struct AdjMesh {
   const double* qtab;
   const unsigned char* bc;
   const double *elem_mass, *node_mass, *gamma, *csmin;
+  int lanes;
 };
 
 struct AdjBufs {

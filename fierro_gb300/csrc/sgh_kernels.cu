@@ -144,8 +144,9 @@ __device__ __forceinline__ Impedance impedance(double den, double sspd, double q
 #endif
 }
 __device__ __forceinline__ double corner_impedance(const Impedance& z, double d0, double d1, double d2, double b0,
-                                                   double b1, double b2) {
+                                                   double b1, double b2, double* mag = nullptr) {
   const double mag_vel = mode_sqrt(sum_sq(d0, d1, d2));
+  if (mag) *mag = mag_vel;
 #if FIERRO_FMA
   const double muc = fma(z.quad, mag_vel, z.lin);
 #else
@@ -811,15 +812,16 @@ static unsigned grid_or(int grid, unsigned blocks) {
 static void launch_force(const ForceArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);
   const unsigned g = blocks_for(a.ne, bs);
-  if (a.lanes && a.stress_out) launch(k_force_lanes<true>, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
-  else if (a.lanes) launch(k_force_lanes<false>, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
+  if (a.lanes && a.stress_out) launch(k_force_lanes<true, false>, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
+  else if (a.lanes) launch(k_force_lanes<false, false>, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
   else if (a.inst) launch(k_force<true, false, false>, grid_or(a.grid, g), bs, s, a);
   else if (a.stress_out) launch(k_force<false, false, true>, g, bs, s, a);
   else launch(k_force<false, false, false>, g, bs, s, a);
 }
 static void launch_force_tape(const ForceArgs& a, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);
-  launch(k_force<false, true, false>, blocks_for(a.ne, bs), bs, s, a);
+  if (a.lanes) launch(k_force_lanes<false, true>, blocks_for(8LL * a.ne, kLaneBlock), kLaneBlock, s, a);
+  else launch(k_force<false, true, false>, blocks_for(a.ne, bs), bs, s, a);
 }
 static void launch_force_branch(const ForceArgs& a, int mode, cudaStream_t s) {
   const int bs = block_or(a.block, kForceBlock);

@@ -15,107 +15,13 @@
 // different quantities in the same instructions); everything else is per corner.
 #pragma once
 
-// ---------------------------------------------------------------------------
-// The hex cofactor tables (sgh_hex.h), rearranged per lane.  two[m] = (i, j): the
-// combo I[i] - I[j]; four[m]: signed 1-based terms summed left to right; a lane's
-// row: for each of its six products the O node (3 bits), the combo (5 bits: 0-11
-// two-term, 12-17 four-term) and its sign (1 bit); vol: the volume's order of the
-// six products (3 bits each) and the node's place in the volume's sum (3 bits).
-struct LaneTables {
-  unsigned long long two[2], four[2], row[8];
-  unsigned vol[8];
-};
-constexpr LaneTables make_lane_tables() {
-  LaneTables r{};
-  signed char uniq[18][4] = {};
-  int n2 = 0, n4 = 0;
-  for (int pass = 0; pass < 2; ++pass)
-    for (int p = 0; p < 8; ++p)
-      for (int t = 0; t < 6; ++t) {
-        const signed char* T = hex::TERMS[p][t];
-        const bool is4 = T[2] != 0;
-        if (is4 != (pass == 1) || hex::J[p][t] < p) continue;
-        bool known = false;
-        const int lo = is4 ? 12 : 0, hi = is4 ? 12 + n4 : n2;
-        for (int k = lo; k < hi; ++k) {
-          bool same = true, neg = true;
-          for (int q = 0; q < 4; ++q) {
-            if (uniq[k][q] != T[q]) same = false;
-            if (uniq[k][q] != -T[q]) neg = false;
-          }
-          if (same || neg) known = true;
-        }
-        if (known) continue;
-        const int at = is4 ? 12 + n4++ : n2++;
-        for (int q = 0; q < 4; ++q) uniq[at][q] = T[q];
-      }
-  for (int k = 0; k < 12; ++k) {
-    const int i = (uniq[k][0] > 0 ? uniq[k][0] : uniq[k][1]) - 1, j = -(uniq[k][0] > 0 ? uniq[k][1] : uniq[k][0]) - 1;
-    r.two[k / 10] |= (unsigned long long)(i | (j << 3)) << (6 * (k % 10));
-  }
-  for (int k = 0; k < 6; ++k) {
-    unsigned long long w = 0;
-    for (int q = 0; q < 4; ++q) {
-      const int v = uniq[12 + k][q];
-      w |= (unsigned long long)(((v > 0 ? v : -v) - 1) | (v < 0 ? 8 : 0)) << (4 * q);
-    }
-    r.four[k / 4] |= w << (16 * (k % 4));
-  }
-  for (int p = 0; p < 8; ++p) {
-    for (int t = 0; t < 6; ++t) {
-      const signed char* T = hex::TERMS[p][t];
-      const int lo = T[2] != 0 ? 12 : 0, hi = T[2] != 0 ? 18 : 12;
-      for (int k = lo; k < hi; ++k) {
-        bool same = true, neg = true;
-        for (int q = 0; q < 4; ++q) {
-          if (uniq[k][q] != T[q]) same = false;
-          if (uniq[k][q] != -T[q]) neg = false;
-        }
-        // a two-term combo is kept as (positive) - (negative): -a + b is b - a
-        if (same || neg) r.row[p] |= (unsigned long long)(hex::J[p][t] | (k << 3) | (neg ? 256 : 0)) << (9 * t);
-      }
-    }
-    for (int a = 0; a < 8; ++a)
-      if (hex::VI[a] == p) {
-        for (int b = 0; b < 6; ++b) r.vol[p] |= (unsigned)hex::slot(p, hex::VJ[a][b]) << (3 * b);
-        r.vol[p] |= (unsigned)a << 18;
-      }
-  }
-  return r;
-}
-constexpr LaneTables kLane = make_lane_tables();
-
-// One of eight constants by lane, by selects (no memory access).
-__device__ __forceinline__ unsigned long long by_lane(int l, unsigned long long a, unsigned long long b,
-                                                      unsigned long long c, unsigned long long d, unsigned long long e,
-                                                      unsigned long long f, unsigned long long g,
-                                                      unsigned long long h) {
-  const unsigned long long ab = l & 1 ? b : a, cd = l & 1 ? d : c, ef = l & 1 ? f : e, gh = l & 1 ? h : g;
-  const unsigned long long lo = l & 2 ? cd : ab, hi = l & 2 ? gh : ef;
-  return l & 4 ? hi : lo;
-}
-__device__ __forceinline__ double flip(double v, unsigned neg) {
-  return __hiloint2double(__double2hiint(v) ^ (int)(neg << 31), __double2loint(v));
-}
-// Value of the first lane of each group of eight, or of its lane `src`.
-__device__ __forceinline__ double from_lane(double v, int src) { return __shfl_sync(0xFFFFFFFFu, v, src, 8); }
-__device__ __forceinline__ long long group_min(long long k) {
-  for (int o = 4; o > 0; o >>= 1) {
-    const long long t = __shfl_xor_sync(0xFFFFFFFFu, k, o);
-    k = t < k ? t : k;
-  }
-  return k;
-}
-
-constexpr int kLaneBlock = 64;               // threads: two warps, eight elements
-constexpr int kLaneWarps = kLaneBlock / 32;
-constexpr int kGroups = 4;                   // elements per warp
+#include "sgh_lane_tables.cuh"
 
 // ---------------------------------------------------------------------------
 // STRENGTH as in force_elem: each lane reads one stress component (lane 0 the
 // ninth too), the velocity gradient's nine sums run in the eight lanes (one twice),
-// and lane 0 runs the model.
-template <bool STRENGTH>
+// and lane 0 runs the model.  TAPE as there: the viscosity intermediates, stored.
+template <bool STRENGTH, bool TAPE>
 __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   // per element: the corners' velocities and impedance terms, rows u, v, w, mu
   __shared__ double s_v[kLaneWarps][kGroups][4][9];
@@ -157,7 +63,8 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   for (int k = 0; k < 8; ++k) vs = fma(0.125, sv[c][k], vs);
   const double vs0 = from_lane(vs, 0), vs1 = from_lane(vs, 1), vs2 = from_lane(vs, 2);
   const Impedance z = impedance(den, sspd, qa, qb);
-  const double mu = corner_impedance(z, vu - vs0, vv - vs1, vw - vs2, b0, b1, b2);
+  double mag_vel;
+  const double mu = corner_impedance(z, vu - vs0, vv - vs1, vw - vs2, b0, b1, b2, &mag_vel);
   __syncwarp();
 #if FIERRO_FMA
   sv[3][l] = mu;
@@ -180,7 +87,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   // Riemann velocity's (0-2), the limiter's (3), the Mach switch's (4 and on)
   const double D = div + a.small;
   const double dsel = okey_decode(__double_as_longlong(D) > 0 ? kmin : kmax);
-  const double mach = 20.0 * (pow_third(vol) * fabs(div));
+  const double c_length = pow_third(vol), mach = 20.0 * (c_length * fabs(div));
   __syncwarp();
 #if FIERRO_FMA
   const double num = l < 3 ? 1.0 : l == 3 ? 0.9 * (dsel + a.small) : mach;
@@ -192,7 +99,30 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   const double vstar = !(s3 > a.fuzz) ? 0.0 : FIERRO_FMA ? s * qt : qt;
   const double vstar0 = from_lane(vstar, 0), vstar1 = from_lane(vstar, 1), vstar2 = from_lane(vstar, 2);
   const double r_min = limiter_min(a, D, dsel, from_lane(qt, 3), k0, k1);
-  const double phi = at_most_1(from_lane(qt, 4)) * (1.0 - at_least_0(r_min));
+  const double phi0 = 1.0 - at_least_0(r_min);
+  const double phi = at_most_1(from_lane(qt, 4)) * phi0;
+  if (TAPE) {
+    const double araw = from_lane(qt, 4);
+    // the neighbour whose divergence set phi0 when the limiter is active: the first
+    // that attains it
+    int at = 0x7FFFFFFF;
+    const long long ksel = __double_as_longlong(D) > 0 ? kmin : kmax;
+    if (k1 > k0 && is_finite(D) && (__double_as_longlong(D) & kAbsMask) != 0 && is_finite(dsel) && r_min < 1.0 &&
+        r_min > 0.0)
+      for (int k = k0 + l; k < k1; k += 8)
+        if (at == 0x7FFFFFFF && okey(a.div[__ldg(a.eie + k)]) == ksel) at = k;
+    __syncwarp();
+    for (int o = 4; o > 0; o >>= 1) at = min(at, __shfl_xor_sync(0xFFFFFFFFu, at, o));
+    if (live) {
+      double* t = a.tape + e;
+      t[(size_t)l * ne] = mu;
+      t[(size_t)(8 + l) * ne] = mag_vel;
+      const double all = l == 0 ? vstar0 : l == 1 ? vstar1 : l == 2 ? vstar2 : l == 3 ? s3 : l == 4 ? phi0 : l == 5 ? araw
+                         : l == 6 ? c_length : r_min;
+      t[(size_t)(16 + l) * ne] = all;
+      if (l == 0) a.tape_sel[e] = at == 0x7FFFFFFF ? -1 : __ldg(a.eie + at);
+    }
+  }
   const double pm = phi * mu;
   if constexpr (!STRENGTH) {
     if (!live) return;
