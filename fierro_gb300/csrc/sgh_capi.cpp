@@ -233,7 +233,50 @@ void enqueue_cycle(fierro_sgh* h, int c) {
   if (h->out) xfer::launch_snapshot(output_snap_args(h, c ^ 1, 0), h->stream);
 }
 
+void release_run_graphs(fierro_sgh* h) {
+  for (int c = 0; c < 2; ++c)
+    if (h->run_graph[c]) {
+      cudaGraphExecDestroy(h->run_graph[c]);
+      h->run_graph[c] = nullptr;
+    }
+  h->graph_cycles = 0;
+}
+
+// Launching a graph leaves the device idle for ~3 us after the one before it: a
+// run on a small mesh launches four cycles at a time (8^3 41.5 -> 38.3 us a cycle,
+// 16^3 45.5 -> 43.0, 32^3 127.9 -> 124.6; eight at a time 38.1, 42.7, 124.2).  The larger
+// graphs take ~0.2 ms to make, so they are made when a handle has run kRunAfter
+// cycles; meshes above kRunElems gain under 1 %.
+constexpr int kRunCycles = 4;
+constexpr long long kRunAfter = 24, kRunElems = 150000;
+
+// True when cycles may be launched kRunCycles at a time.  A handle whose graphs
+// cannot be made keeps launching single cycles.
+bool run_graphs_ready(fierro_sgh* h) {
+  if (h->out || h->ne > kRunElems) return false;
+  if (h->run_graph[0]) return true;
+  if (h->graph_cycles < kRunAfter) return false;
+  for (int c = 0; c < 2; ++c) {
+    cudaGraph_t g = nullptr;
+    cudaError_t err = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
+    if (err == cudaSuccess) {
+      for (int k = 0; k < kRunCycles; ++k) enqueue_cycle(h, (c + k) & 1);
+      err = cudaStreamEndCapture(h->stream, &g);
+    }
+    if (err == cudaSuccess) err = cudaGraphInstantiate(&h->run_graph[c], g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (err != cudaSuccess) {
+      cudaGetLastError();
+      h->run_graph[c] = nullptr;
+      release_run_graphs(h);  // tries again after kRunAfter more cycles
+      return false;
+    }
+  }
+  return true;
+}
+
 int build_graphs(fierro_sgh* h) {
+  release_run_graphs(h);
   for (int c = 0; c < 2; ++c) {
     if (h->graph[c]) {
       cudaGraphExecDestroy(h->graph[c]);
@@ -279,6 +322,7 @@ extern "C" int fierro_sgh_destroy(fierro_sgh* h) {
   adj_branches_release(h);
   for (int c = 0; c < 2; ++c)
     if (h->graph[c]) cudaGraphExecDestroy(h->graph[c]);
+  release_run_graphs(h);
   for (void* p : h->allocations) cudaFree(p);
   if (h->d_statev) cudaFree(h->d_statev);
   for (int i = 0; i < 2; ++i) {
@@ -751,12 +795,15 @@ extern "C" int fierro_sgh_enqueue_cycles(fierro_sgh* h, int64_t cycles) {
   NvtxRange nvtx_("fierro_sgh_enqueue_cycles");
   if (!h || !h->has_state) return set_error(FIERRO_EINVAL, "enqueue before set_state");
   if (h->stage != 0) return set_error(FIERRO_EINVAL, "a cycle is partly run; finish it with run_stages");
-  for (int64_t i = 0; i < cycles; ++i) {
+  for (int64_t i = 0; i < cycles;) {
     const int c = (int)((h->base + h->enq_cycles) & 1);
+    const int step = cycles - i >= kRunCycles && run_graphs_ready(h) ? kRunCycles : 1;
     if (h->out) TRY(output_before_cycle(h, h->enq_cycles));
-    CUDA_TRY(cudaGraphLaunch(h->graph[c], h->stream));
+    CUDA_TRY(cudaGraphLaunch(step > 1 ? h->run_graph[c] : h->graph[c], h->stream));
     if (h->out) TRY(output_after_cycle(h));
-    h->enq_cycles++;
+    h->enq_cycles += step;
+    h->graph_cycles += step;
+    i += step;
   }
   return FIERRO_OK;
 }

@@ -82,6 +82,10 @@ struct fierro_sgh {
   int stage = 0;         // next RK stage of the current cycle (stage stepping)
   bool has_state = false;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  // small meshes: kRunCycles cycles in one graph, made once graph_cycles cycles of
+  // the current graphs have been enqueued (sgh_capi.cpp)
+  cudaGraphExec_t run_graph[2] = {nullptr, nullptr};
+  long long graph_cycles = 0;
   fierro::AdjState* adj = nullptr;  // discrete-adjoint tape and checkpoints (sgh_adjoint.cpp)
   fierro::AdjBranches* adj_br = nullptr;  // branch record of the frozen-branch forward (sgh_adjoint.cpp)
   // direct transfers (sgh_xfer.cu): caller -> internal maps and the validation word

@@ -163,3 +163,37 @@ def test_adjoint_on_both_sides_of_the_lane_passes(lib_built, n):
         w = want[k].cpu().numpy()
         assert np.linalg.norm(got[k] - w) <= 1e-10 * np.linalg.norm(w), k
     state["solver"].close()
+
+
+@pytest.mark.parametrize("pieces", [(108,), (23, 41, 5, 7, 2, 30), (24, 1, 3, 4, 76)])
+def test_runs_in_graphs_of_several_cycles(lib_built, tmp_path, pieces):
+    """A handle that has run for a while launches four cycles at a time: any split of a run
+    gives what stepping stage by stage gives, across a restart and a stop at the
+    final time too."""
+    from fierro_gb300 import sgh
+    p = _deck((7, 5, 6), 200)
+    st = sgh.setup(p)
+    with sgh.SGHSolver(p) as a, sgh.SGHSolver(p) as b:
+        a.set_state(st)
+        b.set_state(st)
+        for n in pieces:
+            assert a.run(n) == n
+        b.run_stages(2 * sum(pieces))
+        want, got = b.get_state(), a.get_state()
+        assert a.time() == b.time()
+        for k in want:
+            assert np.array_equal(got[k], want[k]), k
+        a.checkpoint(str(tmp_path / "a"))
+        ran = a.run(21)  # up to the deck's final time
+        want = a.get_state()
+        b.run(70)
+        b.restart(str(tmp_path / "a"))
+        assert b.run(21) == ran
+        got = b.get_state()
+        for k in want:
+            assert np.array_equal(got[k], want[k]), k
+    p.params.time_final = 0.12
+    with sgh.SGHSolver(p) as a:
+        a.set_state(st)
+        ran = a.run(66) + a.run(301)
+        assert a.time()[0] >= 0.12 and ran == a.time()[3] < 367 and a.run(9) == 0
