@@ -355,7 +355,7 @@ int replay_segment(fierro_sgh* h, AdjState* a, int g, int n) {
       ea.block = h->blk_elem;
       h->ks->elem(ea, s == S - 1 ? 1 : 0, st);
     }
-    h->ks->end(a->ctrl, h->lp, st);
+    h->ks->end(a->ctrl, h->lp, 0, st);
   }
   CUDA_TRY(cudaGetLastError());
   return FIERRO_OK;
@@ -463,7 +463,7 @@ void branch_cycle(fierro_sgh* h, AdjBranches* br, long long i, int mode) {
     h->ks->node(node_args(h, c, stage_alpha(h, s)), h->stream);
     h->ks->elem(stage_elem_args(h, c, s), s == S - 1 ? 1 : 0, h->stream);
   }
-  h->ks->end(h->d_ctrl, h->lp, h->stream);
+  h->ks->end(h->d_ctrl, h->lp, 0, h->stream);
 }
 
 int upload_seed(fierro_sgh* h, double* dst, const double* src, const std::vector<int64_t>& map, size_t stride,

@@ -53,6 +53,17 @@ int download_scatter(fierro_sgh* h, double* out, const double* src, const std::v
   return FIERRO_OK;
 }
 
+int fork_side(fierro_sgh* h) {
+  CUDA_TRY(cudaEventRecord(h->side_ev[0], h->stream));
+  CUDA_TRY(cudaStreamWaitEvent(h->side, h->side_ev[0], 0));
+  return FIERRO_OK;
+}
+int join_side(fierro_sgh* h) {
+  CUDA_TRY(cudaEventRecord(h->side_ev[1], h->side));
+  CUDA_TRY(cudaStreamWaitEvent(h->stream, h->side_ev[1], 0));
+  return FIERRO_OK;
+}
+
 int check_status(fierro_sgh* h) {
   Ctrl c;
   CUDA_TRY(cudaMemcpyAsync(&c, h->d_ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
@@ -202,35 +213,50 @@ using namespace fierro::hd;
 namespace {
 
 // Stage s of a cycle whose start state is in bin c; with `ev`, an event is
-// recorded after each launch.
-int enqueue_stage_ev(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k) {
-  if (h->dims == 2) return rz::enqueue_stage(h, c, s, ev, k);
-  h->ks->force(stage_force_args(h, c, s), h->stream);
+// recorded after each launch; with `fork` (a cycle graph's capture), the first
+// stage's force launch runs beside k_dt on the side stream (it does not read the
+// time step; with a strength model it does, and follows k_dt), and k_end beside
+// the last stage's element launch.
+int enqueue_stage_ev(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k, bool fork = false) {
+  if (h->dims == 2) return rz::enqueue_stage(h, c, s, ev, k, fork);
+  ForceArgs f = stage_force_args(h, c, s);
+  f.beside_dt = fork && s == 0 && !h->strength;
+  h->ks->force(f, h->stream);
+  if (fork && s == 0) TRY(join_side(h));
   if (ev) CUDA_TRY(cudaEventRecord(ev[(*k)++], h->stream));
   h->ks->node(node_args(h, c, stage_alpha(h, s)), h->stream);
   if (ev) CUDA_TRY(cudaEventRecord(ev[(*k)++], h->stream));
-  h->ks->elem(stage_elem_args(h, c, s), (s == h->rk_num_stages - 1) ? 1 : 0, h->stream);
+  const bool last = s == h->rk_num_stages - 1;
+  if (fork && last) {
+    TRY(fork_side(h));
+    h->ks->end(h->d_ctrl, h->lp, 1, h->side);
+  }
+  h->ks->elem(stage_elem_args(h, c, s), last ? 1 : 0, h->stream);
+  if (fork && last) TRY(join_side(h));
   if (ev) CUDA_TRY(cudaEventRecord(ev[(*k)++], h->stream));
   return FIERRO_OK;
 }
 
 void enqueue_stage(fierro_sgh* h, int c, int s) { enqueue_stage_ev(h, c, s, nullptr, nullptr); }
 
-void enqueue_dt(fierro_sgh* h) {
+void enqueue_dt(fierro_sgh* h, cudaStream_t stream) {
   DtArgs d{};
   d.cfl_part = h->d_cfl;
   d.nparts = h->ncfl;
   d.ctrl = h->d_ctrl;
   d.lp = h->lp;
-  h->ks->dt(d, h->stream);
+  h->ks->dt(d, stream);
 }
+void enqueue_dt(fierro_sgh* h) { enqueue_dt(h, h->stream); }
 
-void enqueue_cycle(fierro_sgh* h, int c) {
-  enqueue_dt(h);
-  for (int s = 0; s < h->rk_num_stages; ++s) enqueue_stage(h, c, s);
-  h->ks->end(h->d_ctrl, h->lp, h->stream);
+// One cycle into a graph's capture.
+int enqueue_cycle(fierro_sgh* h, int c) {
+  TRY(fork_side(h));
+  enqueue_dt(h, h->strength ? h->stream : h->side);
+  for (int s = 0; s < h->rk_num_stages; ++s) TRY(enqueue_stage_ev(h, c, s, nullptr, nullptr, true));
   // a write event of this cycle: snapshot of the state it left in bin c ^ 1
   if (h->out) xfer::launch_snapshot(output_snap_args(h, c ^ 1, 0), h->stream);
+  return FIERRO_OK;
 }
 
 void release_run_graphs(fierro_sgh* h) {
@@ -260,8 +286,10 @@ bool run_graphs_ready(fierro_sgh* h) {
     cudaGraph_t g = nullptr;
     cudaError_t err = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
     if (err == cudaSuccess) {
-      for (int k = 0; k < kRunCycles; ++k) enqueue_cycle(h, (c + k) & 1);
+      bool ok = true;
+      for (int k = 0; k < kRunCycles && ok; ++k) ok = enqueue_cycle(h, (c + k) & 1) == FIERRO_OK;
       err = cudaStreamEndCapture(h->stream, &g);
+      if (err == cudaSuccess && !ok) err = cudaErrorUnknown;
     }
     if (err == cudaSuccess) err = cudaGraphInstantiate(&h->run_graph[c], g, 0);
     if (g) cudaGraphDestroy(g);
@@ -277,6 +305,9 @@ bool run_graphs_ready(fierro_sgh* h) {
 
 int build_graphs(fierro_sgh* h) {
   release_run_graphs(h);
+  if (!h->side) CUDA_TRY(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+  for (cudaEvent_t& e : h->side_ev)
+    if (!e) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (int c = 0; c < 2; ++c) {
     if (h->graph[c]) {
       cudaGraphExecDestroy(h->graph[c]);
@@ -284,8 +315,12 @@ int build_graphs(fierro_sgh* h) {
     }
     cudaGraph_t g = nullptr;
     CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    enqueue_cycle(h, c);
+    const int rc = enqueue_cycle(h, c);
     CUDA_TRY(cudaStreamEndCapture(h->stream, &g));
+    if (rc) {
+      cudaGraphDestroy(g);
+      return rc;
+    }
     cudaError_t err = cudaGraphInstantiate(&h->graph[c], g, 0);
     cudaGraphDestroy(g);
     if (err != cudaSuccess) return set_error(FIERRO_ECUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(err));
@@ -323,6 +358,9 @@ extern "C" int fierro_sgh_destroy(fierro_sgh* h) {
   for (int c = 0; c < 2; ++c)
     if (h->graph[c]) cudaGraphExecDestroy(h->graph[c]);
   release_run_graphs(h);
+  if (h->side) cudaStreamDestroy(h->side);
+  for (cudaEvent_t e : h->side_ev)
+    if (e) cudaEventDestroy(e);
   for (void* p : h->allocations) cudaFree(p);
   if (h->d_statev) cudaFree(h->d_statev);
   for (int i = 0; i < 2; ++i) {
@@ -849,7 +887,7 @@ extern "C" int fierro_sgh_run_stages(fierro_sgh* h, int64_t stages) {
     enqueue_stage(h, c, h->stage);
     h->stage++;
     if (h->stage == h->rk_num_stages) {
-      h->ks->end(h->d_ctrl, h->lp, h->stream);
+      h->ks->end(h->d_ctrl, h->lp, 0, h->stream);
       h->stage = 0;
       h->enq_cycles++;
     }
@@ -879,7 +917,7 @@ extern "C" int fierro_sgh_run_timed(fierro_sgh* h, int64_t cycles, float* kernel
     enqueue_dt(h);
     CUDA_TRY(cudaEventRecord(ev[k++], h->stream));
     for (int s = 0; s < h->rk_num_stages; ++s) TRY(enqueue_stage_ev(h, c, s, ev.data(), &k));
-    h->ks->end(h->d_ctrl, h->lp, h->stream);
+    h->ks->end(h->d_ctrl, h->lp, 0, h->stream);
     CUDA_TRY(cudaEventRecord(ev[k++], h->stream));
     h->enq_cycles++;
   }
@@ -1147,6 +1185,7 @@ extern "C" int fierro_sgh_checkpoint(fierro_sgh* h, const char* path) {
       std::fclose(f);
       return set_error(FIERRO_ECUDA, "checkpoint: %s", cudaGetErrorString(err));
     }
+    if (b.ptr == h->d_ctrl && err == cudaSuccess) reinterpret_cast<Ctrl*>(buf.data())->active = 0;
     if (b.cfl && err == cudaSuccess) {
       long long* k = reinterpret_cast<long long*>(buf.data());
       const int64_t g = ckpt_cfl_group(h), n = ckpt_ncfl(h);

@@ -82,6 +82,7 @@ struct ForceArgs {
   double rk_alpha;
   int copy_stress;     // stage 0: elements without a hypo model carry stress_cur over
   int lanes;           // eight lanes per element (small meshes, sgh_lanes.cuh)
+  int beside_dt;       // this launch runs beside the cycle's k_dt: it takes the cycle as active unless stopped
   int block;           // threads per block (0: kForceBlock)
   int grid;            // batch only: blocks of a persistent grid (0: one block per tile)
 };
@@ -194,7 +195,9 @@ struct KernelSet {
   void (*node)(const NodeArgs&, cudaStream_t);
   void (*elem)(const ElemArgs&, int kind, cudaStream_t);
   void (*dt)(const DtArgs&, cudaStream_t);
-  void (*end)(Ctrl*, const LoopParams&, cudaStream_t);
+  // beside: runs beside the cycle's last element launch, which still reads
+  // `active`: leaves it for the next k_dt to set
+  void (*end)(Ctrl*, const LoopParams&, int beside, cudaStream_t);
   void (*energy)(const EnergyArgs&, cudaStream_t);
   void (*end_batch)(Ctrl*, const LoopParams*, int, cudaStream_t);
   const char* name;

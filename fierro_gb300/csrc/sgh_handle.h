@@ -46,6 +46,10 @@ struct fierro_sgh {
   double dt_start = 1e-5;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  // a cycle graph's side branch: k_dt beside the first force launch, k_axis_rz
+  // beside the element launch
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_ev[2] = {};
   std::vector<void*> allocations;
   size_t dev_bytes = 0;
   // mesh
@@ -150,6 +154,10 @@ int upload_gather(fierro_sgh* h, double* dst, const double* src, const std::vect
 // Permuted download: out[map[i]*stride + off] = src[i].
 int download_scatter(fierro_sgh* h, double* out, const double* src, const std::vector<int64_t>& map,
                      size_t stride, size_t off);
+// In a capture: what is enqueued on h->side from here on follows h->stream's work
+// so far; h->stream's work from here on follows h->side's.
+int fork_side(fierro_sgh* h);
+int join_side(fierro_sgh* h);
 int check_status(fierro_sgh* h);
 int cycles_done(fierro_sgh* h, long long* cyc);
 ForceArgs force_args(fierro_sgh* h, int rb, int q);

@@ -123,6 +123,12 @@ __device__ __forceinline__ void velocity_gradient(const double (&u)[8], const do
   }
 }
 
+// Whether the cycle runs.  Beside its k_dt (which sets `active` to that) the
+// force pass asks what k_dt asks.
+__device__ __forceinline__ bool force_active(const ForceArgs& a) {
+  return a.beside_dt ? !a.ctrl->stopped : a.ctrl->active != 0;
+}
+
 // ---------------------------------------------------------------------------
 // The scalar steps the one-thread-per-element passes and the lane passes
 // (sgh_lanes.cuh) share; what the FMA mode fuses is written out, as the two must
@@ -412,7 +418,7 @@ __global__ void FIERRO_FORCE_BOUNDS k_force(const ForceArgs a) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.ne; e += gridDim.x * blockDim.x)
       force_elem<true, TAPE, STRENGTH, BR>(a, e);
   } else {
-    if (!a.ctrl->active) return;
+    if (!force_active(a)) return;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= a.ne) return;
     force_elem<false, TAPE, STRENGTH, BR>(a, e);
@@ -727,7 +733,7 @@ __global__ void __launch_bounds__(256) k_dt_batch(const DtArgs a) {
 }
 
 // End of a cycle (sgh_solve.cpp:590-632).
-__device__ __forceinline__ void end_update(Ctrl* c, const LoopParams& lp) {
+__device__ __forceinline__ void end_update(Ctrl* c, const LoopParams& lp, bool beside = false) {
   c->wrote = 0;
   if (!c->active) return;
   c->time_value += c->dt;
@@ -740,12 +746,12 @@ __device__ __forceinline__ void end_update(Ctrl* c, const LoopParams& lp) {
   c->wrote = write ? 1 : 0;
   if (c->time_value >= lp.time_final) c->stopped = 1;
   c->cycle = cycle + 1;
-  c->active = 0;
+  if (!beside) c->active = 0;
 }
 
-__global__ void k_end(Ctrl* c, const LoopParams lp) {
+__global__ void k_end(Ctrl* c, const LoopParams lp, int beside) {
   previous_launch_done();
-  end_update(c, lp);
+  end_update(c, lp, beside != 0);
 }
 
 __global__ void k_end_batch(Ctrl* c, const LoopParams* lps, int ninst) {
@@ -861,7 +867,9 @@ static void launch_dt(const DtArgs& a, cudaStream_t s) {
   if (a.part_start) launch(k_dt_batch, a.ninst, 256, s, a);
   else launch(k_dt, 1, 1024, s, a);
 }
-static void launch_end(Ctrl* c, const LoopParams& lp, cudaStream_t s) { launch(k_end, 1, 1, s, c, lp); }
+static void launch_end(Ctrl* c, const LoopParams& lp, int beside, cudaStream_t s) {
+  launch(k_end, 1, 1, s, c, lp, beside);
+}
 static void launch_end_batch(Ctrl* c, const LoopParams* lps, int ninst, cudaStream_t s) {
   launch(k_end_batch, blocks_for(ninst, 128), 128, s, c, lps, ninst);
 }

@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
   const int n = __ldg(a.nie + 8 * (size_t)e + l);  // the mesh does not change: before the wait
   const int k0 = __ldg(a.eie_start + e), k1 = __ldg(a.eie_start + e + 1);
   previous_launch_done();
-  if (!a.ctrl->active || (t & ~31) >= 8 * ne) return;  // whole warps past the end
+  if (!force_active(a) || (t & ~31) >= 8 * ne) return;  // whole warps past the end
   const double vu = a.u[n], vv = a.v[n], vw = a.w[n];
   const double b0 = a.bmat[(size_t)(l * 3 + 0) * ne + e];
   const double b1 = a.bmat[(size_t)(l * 3 + 1) * ne + e];

@@ -523,7 +523,7 @@ int get_state(fierro_sgh* h, fierro_sgh_state* s, const int bins[2], int qb) {
   return FIERRO_OK;
 }
 
-int enqueue_stage(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k) {
+int enqueue_stage(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k, bool fork) {
   const double alpha = stage_alpha(h, s);
   const int rb = (s == 0) ? c : (c ^ 1);
   const int q = div_parity(h, c, s);
@@ -558,6 +558,7 @@ int enqueue_stage(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k) {
     f.copy_stress = s == 0;
   }
   f.lanes = h->lanes_force;
+  f.beside_dt = fork && s == 0 && !h->strength;
   RzNodeArgs n{};
   n.nn = (int)h->nn;
   n.ne = (int)h->ne;
@@ -598,11 +599,16 @@ int enqueue_stage(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k) {
   };
   h->rks->force(f, h->stream);
   TRY(mark());
+  if (fork) TRY(join_side(h));  // the time step, or the last stage's axis masses
   h->rks->node(n, h->stream);
   TRY(mark());
-  h->rks->axis(x, h->stream);
+  if (fork) TRY(fork_side(h));
+  h->rks->axis(x, fork ? h->side : h->stream);
   TRY(mark());
-  h->rks->elem(e, (s == h->rk_num_stages - 1) ? 1 : 0, h->stream);
+  const bool last = s == h->rk_num_stages - 1;
+  if (fork && last) h->ks->end(h->d_ctrl, h->lp, 1, h->side);
+  h->rks->elem(e, last ? 1 : 0, h->stream);
+  if (fork && last) TRY(join_side(h));
   TRY(mark());
   return FIERRO_OK;
 }

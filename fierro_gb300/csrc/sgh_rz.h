@@ -44,6 +44,7 @@ struct RzForceArgs {
   double rk_alpha;
   int copy_stress;
   int lanes;  // four lanes per element (small gas-only meshes, sgh_rz_lanes.cuh)
+  int beside_dt;  // as in ForceArgs
 };
 
 struct RzNodeArgs {
@@ -133,7 +134,9 @@ int prime(fierro_sgh* h);
 int get_state(fierro_sgh* h, fierro_sgh_state* s, const int bins[2], int div_buffer);
 // Enqueues RK stage s of a cycle whose start state is in bin c; with `ev`, an
 // event is recorded after each launch.
-int enqueue_stage(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k);
+// `fork` (in a capture): the axis launch on the handle's side stream, beside the
+// element launch and what follows up to the next join.
+int enqueue_stage(fierro_sgh* h, int c, int s, cudaEvent_t* ev, size_t* k, bool fork);
 int energy(fierro_sgh* h, int bin, double* ie, double* ke);
 // setup (setup.cpp:10-424) with num_dims == 2, in the caller's numbering.
 int setup(const fierro_mesh* mesh, const fierro_material* materials, int64_t num_materials,

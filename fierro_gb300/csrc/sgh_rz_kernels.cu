@@ -187,6 +187,11 @@ __device__ __forceinline__ void gather4(const int* nie, int e, int (&nid)[4]) {
   nid[3] = q.w;
 }
 
+// Whether the cycle runs; beside its k_dt, asked as k_dt asks it.
+__device__ __forceinline__ bool force_active(const RzForceArgs& a) {
+  return a.beside_dt ? !a.ctrl->stopped : a.ctrl->active != 0;
+}
+
 // The scalar steps the one-thread-per-element passes and the lane passes
 // (sgh_rz_lanes.cuh) share.  den (q1 c + q2 |v - v_avg|), force_sgh.cpp:520-636:
 __device__ __forceinline__ double rz_impedance(double den, double q1c, double qb, double d0, double d1) {
@@ -231,7 +236,7 @@ __device__ __forceinline__ long long rz_cfl_key(double d2, double sspd, double d
 template <bool STRENGTH>
 __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
   previous_launch_done();
-  if (!a.ctrl->active) return;
+  if (!force_active(a)) return;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.ne) return;
   const int ne = a.ne;

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kRzLaneBlock) k_force_rz_lanes(const RzForceAr
   const int n = __ldg(a.nie + 4 * (size_t)e + l);
   const int k0 = __ldg(a.eie_start + e), k1 = __ldg(a.eie_start + e + 1);
   previous_launch_done();
-  if (!a.ctrl->active || (t & ~31) >= 4 * ne) return;  // whole warps past the end
+  if (!force_active(a) || (t & ~31) >= 4 * ne) return;  // whole warps past the end
   const double xl = a.x[n], yl = a.y[n], ul = a.u[n], vl = a.v[n];
   const double den = a.den[e], pres = a.pres[e], sspd = a.sspd[e], div = a.div[e];
   const double* q = a.qtab + 4 * a.mat[e];
