@@ -353,7 +353,8 @@ int create(fierro_sgh* h, const fierro_mesh* mesh, const fierro_material* materi
   TRY(dalloc(h, &h->d_axis_nin, t.axis_nin.size()));
   h->lanes_force = (long long)ne <= kRzLanesForce && !h->strength;
   h->lanes_elem = (long long)ne <= kRzLanesElem;
-  h->cfl_tile = h->lanes_elem ? kRzLaneTile : kElemBlock;
+  h->blk_elem = small_mesh_block((long long)ne, kElemBlock);
+  h->cfl_tile = h->lanes_elem ? kRzLaneTile : h->blk_elem;
   h->ncfl = (int)((ne + h->cfl_tile - 1) / h->cfl_tile);
   TRY(dalloc(h, &h->d_cfl, (size_t)h->ncfl));
   TRY(dalloc(h, &h->d_ctrl, 1));
@@ -472,6 +473,7 @@ static RzElemArgs elem_args_rz(fierro_sgh* h, int cur, int c, double alpha, int 
   a.dt_cfl = h->lp.dt_cfl;
   a.fuzz = h->lp.fuzz;
   a.lanes = h->lanes_elem;
+  a.block = h->blk_elem;
   return a;
 }
 

@@ -92,6 +92,7 @@ struct RzElemArgs {
   Ctrl* ctrl;
   double rk_alpha, dt_cfl, fuzz;
   int lanes;  // four lanes per element, one CFL partial per kRzLaneTile elements
+  int block;  // threads per block, one CFL partial each (0: kElemBlock)
 };
 
 struct RzEnergyArgs {

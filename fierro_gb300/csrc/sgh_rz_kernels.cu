@@ -612,10 +612,11 @@ static void launch_elem(const RzElemArgs& a, int kind, cudaStream_t s) {
     else launch(k_elem_rz_lanes<2>, g, kRzLaneBlock, s, a);
     return;
   }
-  const unsigned g = blocks_for(a.ne, kRzBlock);
-  if (kind == 0) launch(k_elem_rz<0>, g, kRzBlock, s, a);
-  else if (kind == 1) launch(k_elem_rz<1>, g, kRzBlock, s, a);
-  else launch(k_elem_rz<2>, g, kRzBlock, s, a);
+  const int bs = a.block ? a.block : kRzBlock;
+  const unsigned g = blocks_for(a.ne, bs);
+  if (kind == 0) launch(k_elem_rz<0>, g, bs, s, a);
+  else if (kind == 1) launch(k_elem_rz<1>, g, bs, s, a);
+  else launch(k_elem_rz<2>, g, bs, s, a);
 }
 static void launch_ext(int nn, const double* node_mass, const double* y, double* ext, cudaStream_t s) {
   k_ext_rz<<<blocks_for(nn, kRzNodeBlock), kRzNodeBlock, 0, s>>>(nn, node_mass, y, ext);
