@@ -254,13 +254,14 @@ inline int checkpoint_tile(long long ne) { return small_mesh_block(ne, kElemBloc
 // sgh_lanes.cuh.  A lane pass does about twice the work in an eighth-long chain:
 // it wins until the chip's sub-partitions hold several of its warps each.  Per
 // launch (events, us), one thread per element against eight lanes:
-//                 12^3         20^3         22^3         24^3         32^3
-//   force exact   26.6 / 12.4  26.7 / 22.6  26.7 / 26.9  26.8 / 34.8  42.5 / 68.6
-//   force FMA     20.6 / 10.3  21.4 / 16.6  22.1 / 18.8  22.3 / 24.5  30.6 / 45.0
-//   elem exact    24.5 / 12.2  24.7 / 22.7  24.6 / 28.5  24.8 / 35.0  49.2 / 71.8
-//   elem FMA      20.4 / 10.4  20.5 / 18.7  20.5 / 22.4  20.6 / 27.0  37.0 / 53.9
-//   node exact    10.3 /  8.3  10.4 /  8.4  10.3 /  8.4  10.4 /  9.0  12.3 / 12.3
-constexpr long long kLanesForce = 10500, kLanesElem = 9000, kLanesNode = 30000;
+//                        12^3         18^3         20^3         22^3         23^3
+//   force exact          26.6 / 12.3  26.8 / 16.5  26.7 / 20.4  26.7 / 24.5  26.7 / 28.4
+//   force FMA            20.6 / 10.3               20.7 / 16.3  21.2 / 18.4  20.6 / 20.4
+//   elem exact, CFL step 28.8 / 13.0  28.9 / 20.4  29.9 / 24.7  28.9 / 30.7  29.1 / 36.8
+//   elem FMA, CFL step   23.7 / 12.5               24.6 / 20.5  24.6 / 24.6  24.5 / 28.7
+// and for the nodes, one thread per node against three: 12^3 10.3 / 8.3, 24^3 10.4 /
+// 9.0, 32^3 12.3 / 12.3 (exact).
+constexpr long long kLanesForce = 11500, kLanesElem = 10000, kLanesNode = 30000;
 constexpr int kLaneTile = 4;  // elements per warp of a lane pass
 
 const KernelSet& kernels_exact();

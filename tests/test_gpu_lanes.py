@@ -7,10 +7,10 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# 1, 3, 4, 5, 27, 315 elements; 9000 | 9009 (element pass), 10500 | 10520 (force
+# 1, 3, 4, 5, 27, 315 elements; 10000 | 10010 (element pass), 11500 | 11550 (force
 # pass), 27 x 30 x 33 elements on 29,512 nodes and 29 x 31 x 31 on 30,720 (node pass)
-SHAPES = [(1, 1, 1), (3, 1, 1), (2, 2, 1), (5, 1, 1), (3, 3, 3), (7, 9, 5), (20, 18, 25), (21, 13, 33), (20, 21, 25),
-          (20, 2, 263), (27, 30, 33), (29, 31, 31)]
+SHAPES = [(1, 1, 1), (3, 1, 1), (2, 2, 1), (5, 1, 1), (3, 3, 3), (7, 9, 5), (20, 20, 25), (11, 10, 91), (20, 23, 25),
+          (21, 22, 25), (27, 30, 33), (29, 31, 31)]
 
 
 def _deck(shape, cycles=12):
@@ -42,7 +42,7 @@ def test_lanes_equal_the_batch(lib_built, shape, mode):
         assert np.array_equal(got[k], want[k]), k
 
 
-@pytest.mark.parametrize("shape", [(5, 1, 1), (7, 9, 5), (21, 13, 33)])
+@pytest.mark.parametrize("shape", [(5, 1, 1), (7, 9, 5), (21, 13, 33), (20, 20, 25)])
 def test_checkpoint_of_a_lane_handle(lib_built, tmp_path, shape):
     """The file holds one CFL partial per element block, as it always has, and a
     restart from it takes the same time steps."""
@@ -113,11 +113,11 @@ def test_quad_lanes_equal_the_restatement(oracle_built, lib_built, shape):
     assert_fields(fma, one, 1e-12, keys=("coords", "vel", "den", "pres", "sie"), label="fma %s" % (shape,))
 
 
-@pytest.mark.parametrize("shape", [(2, 2, 1), (7, 9, 5), (20, 21, 25), (21, 21, 24)])
+@pytest.mark.parametrize("shape", [(2, 2, 1), (7, 9, 5), (20, 23, 25), (21, 22, 25)])
 @pytest.mark.parametrize("kind", ["hypo", "mixed"])
 def test_strength_force_equals_the_restatement(oracle_built, lib_built, shape, kind):
     """Exact mode with a strength model, on both sides of the force pass's
-    change-over (10500 | 10584 elements), bit for bit against the C restatement."""
+    change-over (11500 | 11550 elements), bit for bit against the C restatement."""
     import copy
 
     from fierro_gb300 import problems, sgh
