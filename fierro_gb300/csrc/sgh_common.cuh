@@ -109,6 +109,15 @@ __device__ __forceinline__ double f64_of_signed(float f) {
   return __longlong_as_double(e == 0 ? 0LL : bits);
 }
 
+// Single-precision image of a double of either sign (truncated): zero below
+// float's normal range, infinity above it.
+__device__ __forceinline__ float f32_of(double d) {
+  const long long b = __double_as_longlong(d);
+  const int e = (int)((b >> 52) & 0x7FF) - 1023 + 127;
+  const unsigned m = (unsigned)((b >> 29) & 0x7FFFFF), s = (unsigned)(b >> 32) & 0x80000000u;
+  return __uint_as_float(s | (e <= 0 ? 0u : e >= 255 ? 0x7F800000u : ((unsigned)e << 23) | m));
+}
+
 // sqrt(x) to ~2^-64 before the final rounding; b = x's bits, x positive and
 // normal, ex its biased exponent.
 __device__ __forceinline__ double sqrt_newton(double x, long long b, int ex) {
@@ -328,15 +337,20 @@ __device__ __forceinline__ double pow_third(double v) {
   const double q = p * c0;
   const double qe = fma(p, c0, -q) + pe * c0;
   const double r = (v - q) - qe;  // v - q is exact (Sterbenz), qe carries the rest
-  const float rf = (float)r;
-  const float inv3p = __frcp_rn(3.0f * (float)p);
-  const float step = rf * inv3p;  // (v - c0^3) / (3 c0^2)
-  // ln v from the exponent and a single-precision log of the significand
+  // (v - c0^3) / (3 c0^2) in single precision, with v scaled by 2^-3k (on the bits)
+  // to lie in [1, 8); conversions of doubles take FP64 issue slots, the images do not
   const int ex = (int)((bits >> 52) & 0x7FF) - 1023;
+  const int k = ex >= 0 ? ex / 3 : -((2 - ex) / 3);  // floor(ex / 3)
+  const long long rb = __double_as_longlong(r);
+  const float rf = (rb & kAbsMask) == 0 ? 0.0f : f32_of(__longlong_as_double(rb - ((long long)(3 * k) << 52)));
+  const float p1 = f32_image(__longlong_as_double(__double_as_longlong(p) - ((long long)(2 * k) << 52)));
+  const long long sb = __double_as_longlong(f64_of_signed(rf * __frcp_rn(3.0f * p1)));
+  const double step = __longlong_as_double(sb == 0 ? 0LL : sb + ((long long)k << 52));
+  // ln v from the exponent and a single-precision log of the significand
   const double m = __longlong_as_double((bits & 0x000FFFFFFFFFFFFFLL) | 0x3FF0000000000000LL);
-  const float lnv = (float)ex * 0.69314718f + __logf((float)m);
+  const float lnv = (float)ex * 0.69314718f + __logf(f32_image(m));
   const float dlog = lnv * 1.8503717077085943e-17f;  // d = 2^-54 / 3
-  const double lo = (double)step - c0 * (double)dlog;
+  const double lo = step - c0 * f64_of_signed(dlog);
   return c0 + lo;
 #endif
 }

@@ -183,8 +183,7 @@ __device__ __forceinline__ double limiter_min(const ForceArgs& a, double D, doub
 }
 // Divergence from the velocity sums (momentum.cpp:265-286)
 __device__ __forceinline__ double divergence(double Sx, double Sy, double Sz, double inverse_vol) {
-  double div = 0.0;
-  div = mul_add(div, Sx, inverse_vol);
+  double div = Sx * inverse_vol;
   div = mul_add(div, Sy, inverse_vol);
   div = mul_add(div, Sz, inverse_vol);
   return div;
@@ -251,10 +250,11 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     const double b1 = a.bmat[(size_t)(l * 3 + 1) * ne + e];
     const double b2 = a.bmat[(size_t)(l * 3 + 2) * ne + e];
     const double mu_term = corner_impedance(z, vu[l] - vs0, vv[l] - vs1, vw[l] - vs2, b0, b1, b2);
-    s0 = mul_add(s0, mu_term, vu[l]);
-    s1 = mul_add(s1, mu_term, vv[l]);
-    s2 = mul_add(s2, mu_term, vw[l]);
-    s3 = s3 + mu_term;
+    // the sums' first terms as they are: adding them to zero costs an instruction each
+    s0 = l ? mul_add(s0, mu_term, vu[l]) : mu_term * vu[l];
+    s1 = l ? mul_add(s1, mu_term, vv[l]) : mu_term * vv[l];
+    s2 = l ? mul_add(s2, mu_term, vw[l]) : mu_term * vw[l];
+    s3 = l ? s3 + mu_term : mu_term;
     mu[l] = mu_term;
   }
   double vstar0 = 0.0, vstar1 = 0.0, vstar2 = 0.0;
@@ -452,9 +452,9 @@ __device__ __forceinline__ void node_update(const NodeArgs& a, const int n) {
 #pragma unroll
     for (int k = 0; k < kNodeGather; ++k)
       if (k < cnt) {
-        f0 = f0 + g[k][0];
-        f1 = f1 + g[k][1];
-        f2 = f2 + g[k][2];
+        f0 = k || base > c0 ? f0 + g[k][0] : g[k][0];
+        f1 = k || base > c0 ? f1 + g[k][1] : g[k][1];
+        f2 = k || base > c0 ? f2 + g[k][2] : g[k][2];
       }
   }
   const double adt = a.rk_alpha * ctrl->dt;
@@ -543,7 +543,8 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
       double power = 0.0;
 #pragma unroll
       for (int l = 0; l < 8; ++l) {
-        power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 0) * ne + e), ld_pl<COH>(a.hx + nid[l]));
+        const double F0 = ld_pl<COH>(a.force + (size_t)(l * 3 + 0) * ne + e), h0 = ld_pl<COH>(a.hx + nid[l]);
+        power = l ? mul_add(power, F0, h0) : F0 * h0;
         power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 1) * ne + e), ld_pl<COH>(a.hy + nid[l]));
         power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 2) * ne + e), ld_pl<COH>(a.hz + nid[l]));
       }

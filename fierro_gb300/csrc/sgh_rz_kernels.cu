@@ -153,17 +153,11 @@ __device__ __forceinline__ void rz_corner_areas(const double (&x)[4], const doub
 // 1e-6 P^2.  Quads too small (P < 1e-13) or large for float fail it.
 // True for all four centroid triangles (and finite coordinates) means the corner
 // areas need not be formed; otherwise they are, as the reference does.
-__device__ __forceinline__ float f32_signed(double d) {
-  const long long b = __double_as_longlong(d);
-  const int e = (int)((b >> 52) & 0x7FF) - 1023 + 127;
-  const unsigned m = (unsigned)((b >> 29) & 0x7FFFFF), s = (unsigned)(b >> 32) & 0x80000000u;
-  return __uint_as_float(s | (e <= 0 ? 0u : e >= 255 ? 0x7F800000u : ((unsigned)e << 23) | m));
-}
 __device__ __forceinline__ bool rz_corner_areas_finite(double x02, double x13, double y02, double y13, double m_x,
                                                        double m_y) {
-  const float ax = 0.5f * f32_signed(-x02), bx = 0.5f * f32_signed(-x13);
-  const float ay = 0.5f * f32_signed(-y02), by = 0.5f * f32_signed(-y13);
-  const float mx = 0.25f * f32_signed(m_x), my = 0.25f * f32_signed(m_y);
+  const float ax = 0.5f * f32_of(-x02), bx = 0.5f * f32_of(-x13);
+  const float ay = 0.5f * f32_of(-y02), by = 0.5f * f32_of(-y13);
+  const float mx = 0.25f * f32_of(m_x), my = 0.25f * f32_of(m_y);
   const float px[4] = {-ax - mx, -bx + mx, ax - mx, bx + mx};
   const float py[4] = {-ay - my, -by + my, ay - my, by + my};
   bool ok = true;
@@ -289,9 +283,9 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
     const double mu_term = rz_impedance(den, q1c, qb, u[l] - vs0, v[l] - vs1) * bn[l & 1];
-    s0 = mul_add(s0, mu_term, u[l]);
-    s1 = mul_add(s1, mu_term, v[l]);
-    s3 = s3 + mu_term;
+    s0 = l ? mul_add(s0, mu_term, u[l]) : mu_term * u[l];
+    s1 = l ? mul_add(s1, mu_term, v[l]) : mu_term * v[l];
+    s3 = l ? s3 + mu_term : mu_term;
     mu[l] = mu_term;
   }
   double vstar0 = 0.0, vstar1 = 0.0;
@@ -398,8 +392,8 @@ __global__ void __launch_bounds__(kRzNodeBlock) k_node_rz(const RzNodeArgs a) {
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (base + k < c1) {
-        f0 = f0 + g[k][0];
-        f1 = f1 + g[k][1];
+        f0 = k || base > c0 ? f0 + g[k][0] : g[k][0];
+        f1 = k || base > c0 ? f1 + g[k][1] : g[k][1];
       }
   }
   const double adt = a.rk_alpha * a.ctrl->dt;
@@ -478,7 +472,8 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
 #pragma unroll
       for (int l = 0; l < 4; ++l) {
         const double r = a.rad[nid[l]];
-        power = mul_add(power, a.force[(size_t)(l * 2 + 0) * ne + e] * r, a.hx[nid[l]]);
+        const double F0 = a.force[(size_t)(l * 2 + 0) * ne + e] * r, h0 = a.hx[nid[l]];
+        power = l ? mul_add(power, F0, h0) : F0 * h0;
         power = mul_add(power, a.force[(size_t)(l * 2 + 1) * ne + e] * r, a.hy[nid[l]]);
       }
       const double adt = a.rk_alpha * ctrl->dt;
@@ -497,7 +492,7 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     const double elem_vel_r = 0.25 * (v[0] + v[1] + v[2] + v[3]);
     const double su = mul_add(mul_add(mul_mul(u[0], B[0][0], u[1], B[1][0]), u[2], B[2][0]), u[3], B[3][0]);
     const double sv = mul_add(mul_add(mul_mul(v[0], B[0][1], v[1], B[1][1]), v[2], B[2][1]), v[3], B[3][1]);
-    double div = mul_add(0.0, su, inverse_area);
+    double div = su * inverse_area;
     div = div + mul_add(newton_div(elem_vel_r, mean_radius), sv, inverse_area);
     a.div[e] = div;
     double sspd;

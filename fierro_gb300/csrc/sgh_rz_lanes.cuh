@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kRzLaneBlock) k_elem_rz_lanes(const RzElemArgs
   const double qt = newton_div(num, dvs);
   __syncwarp();
   const double inverse_area = quad_lane(qt, 0), mean_radius = quad_lane(qt, 1);
-  double div = mul_add(0.0, su, inverse_area);
+  double div = su * inverse_area;
   div = div + mul_add(newton_div(vr, mean_radius), sv, inverse_area);
   __syncwarp();
   double sspd;
