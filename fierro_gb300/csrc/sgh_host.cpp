@@ -89,7 +89,7 @@ uint64_t spread21(uint64_t v) {
 // where clearing and summing 65536 counters would outweigh the items.
 std::vector<int64_t> radix_order(const std::vector<uint64_t>& key) {
   const size_t n = key.size();
-  const int bits = n < (1u << 20) ? 11 : 16;
+  const int bits = n < (1u << 16) ? 11 : 16;
   const uint64_t mask = (1u << bits) - 1;
   std::vector<int64_t> idx(n), tmp(n);
   std::iota(idx.begin(), idx.end(), 0);
