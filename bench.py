@@ -225,11 +225,11 @@ def alg_bytes(kind: str, nn: int, ne: int, nnz: int) -> float:
 DRAM_PER_ELEM = {"k_force": (847900928 + 373555200) / 2097152,
                  "k_elem": (716255232 + 464538624 + 717109760 + 462138624) / 2 / 2097152}
 NCU_PER_ELEM = {"exact": {
-    "k_force": {"fp64_ops": 124518424 / 262144, "dram_bytes": DRAM_PER_ELEM["k_force"]},
-    "k_elem": {"fp64_ops": (157286400 + 169936928) / 2 / 262144, "dram_bytes": DRAM_PER_ELEM["k_elem"]},
+    "k_force": {"fp64_ops": 458.0, "dram_bytes": DRAM_PER_ELEM["k_force"]},
+    "k_elem": {"fp64_ops": (560.0 + 607.3) / 2, "dram_bytes": DRAM_PER_ELEM["k_elem"]},
 }, "fma": {
-    "k_force": {"fp64_ops": 88342528 / 262144, "dram_bytes": DRAM_PER_ELEM["k_force"]},
-    "k_elem": {"fp64_ops": (127926272 + 137425432) / 2 / 262144, "dram_bytes": DRAM_PER_ELEM["k_elem"]},
+    "k_force": {"fp64_ops": 304.0, "dram_bytes": DRAM_PER_ELEM["k_force"]},
+    "k_elem": {"fp64_ops": (426.0 + 462.2) / 2, "dram_bytes": DRAM_PER_ELEM["k_elem"]},
 }}
 
 
