@@ -14,6 +14,7 @@
 #include <cstring>
 #include <exception>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -21,6 +22,7 @@
 #include "fierro_sgh.h"
 #include "sgh_device.h"
 #include "sgh_internal.h"
+#include "sgh_xfer.h"
 
 using namespace fierro;
 
@@ -75,6 +77,12 @@ struct fierro_batch {
   Ctrl* d_ctrl = nullptr;
   unsigned int* d_sync = nullptr;  // fused stage: arrival counter, generation, timeout status
   cudaError_t capture_err = cudaSuccess;
+  // transfers by the GPU (sgh_xfer.cu): the instances' caller -> internal maps one
+  // after the other (elements in their padded ranges) and the check's result; the
+  // staging buffer, made when a transfer first needs it (see by_gpu)
+  bool direct_host = false;
+  int *d_node_ext2int = nullptr, *d_elem_ext2int = nullptr;
+  XferStatus* d_xfer = nullptr;
   double* h_stage = nullptr;
   size_t stage_elems = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -118,10 +126,65 @@ constexpr int64_t kSmallBatch = 1 << 19;
 // Values a host loop over one instance's array shares among the threads from.
 constexpr int64_t kHostParallel = 4096;
 
+// Instance i's part of the device arrays.
+xfer::StateView view_of(fierro_batch* b, int64_t i) {
+  const int64_t no = b->node_off[i], eo = b->elem_off[i];
+  xfer::StateView v{};
+  v.nn = (int)b->topo[i].nn;
+  v.ne = (int)b->topo[i].ne;
+  v.nmat = (int)(b->mat_off[i + 1] - b->mat_off[i]);
+  v.mat_base = (int)b->mat_off[i];
+  v.dims = 3;
+  v.force_stride = b->NE;
+  v.stream = b->stream;
+  v.status = b->d_xfer;
+  v.node_ext2int = b->d_node_ext2int + no;
+  v.elem_ext2int = b->d_elem_ext2int + eo;
+  for (int k = 0; k < 2; ++k) {
+    for (int d = 0; d < 3; ++d) {
+      v.x[k][d] = b->d_x[k][d] + no;
+      v.v[k][d] = b->d_v[k][d] + no;
+    }
+    v.sie[k] = b->d_sie[k] + eo;
+    v.div[k] = b->d_div[k] + eo;
+  }
+  v.node_mass = b->d_node_mass + no;
+  v.den = b->d_den + eo;
+  v.pres = b->d_pres + eo;
+  v.sspd = b->d_sspd + eo;
+  v.vol = b->d_vol + eo;
+  v.elem_mass = b->d_elem_mass + eo;
+  v.gamma = b->d_gamma + eo;
+  v.csmin = b->d_csmin + eo;
+  v.force = b->d_force + eo;
+  v.mat = b->d_mat + eo;
+  return v;
+}
+
+// Whether the GPU moves a state itself: it can dereference host memory and every
+// array lies on an 8-byte boundary (a host loop takes any address, a kernel's load
+// does not).  Twelve decks of 9^3 to 32^3 elements, 148,000 in all, host loops and a
+// copy per row against the transfer kernels: set_state 7.6 and 1.2 ms, get_state
+// 13.1 and 4.5 ms (most of it the first touch of the output's pages).
+bool by_gpu(const fierro_batch* b, const fierro_sgh_state* s) {
+  const void* p[] = {s->node_coords, s->node_vel, s->node_mass, s->elem_den, s->elem_pres, s->elem_stress,
+                     s->elem_sspd, s->elem_sie, s->elem_vol, s->elem_div, s->elem_mass, s->elem_mat_id,
+                     s->elem_statev, s->corner_force};
+  uintptr_t low = 0;
+  for (const void* q : p) low |= reinterpret_cast<uintptr_t>(q) & 7;
+  return b->direct_host && low == 0;
+}
+
+int make_stage(fierro_batch* b) {
+  if (!b->h_stage) CUDA_TRY(cudaHostAlloc((void**)&b->h_stage, sizeof(double) * b->stage_elems, cudaHostAllocDefault));
+  return FIERRO_OK;
+}
+
 // dst[off + k] = src[map[k] * stride + sub] through the pinned staging buffer.
 int gather_up(fierro_batch* b, double* dst, int64_t off, const double* src, const std::vector<int64_t>& map,
               size_t stride, size_t sub) {
   const int64_t n = (int64_t)map.size();
+  TRY(make_stage(b));
 #pragma omp parallel for schedule(static) if (n >= kHostParallel)
   for (int64_t k = 0; k < n; ++k) b->h_stage[k] = src[(size_t)map[k] * stride + sub];
   CUDA_TRY(cudaMemcpyAsync(dst + off, b->h_stage, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, b->stream));
@@ -132,6 +195,7 @@ int gather_up(fierro_batch* b, double* dst, int64_t off, const double* src, cons
 int scatter_down(fierro_batch* b, double* out, const double* src, int64_t off, const std::vector<int64_t>& map,
                  size_t stride, size_t sub) {
   const int64_t n = (int64_t)map.size();
+  TRY(make_stage(b));
   CUDA_TRY(cudaMemcpyAsync(b->h_stage, src + off, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, b->stream));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
 #pragma omp parallel for schedule(static) if (n >= kHostParallel)
@@ -451,6 +515,9 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   std::vector<int32_t> nie((size_t)NE * 8, 0), cin_start((size_t)NN + 1, 0), cin((size_t)cin_off[n]);
   std::vector<int32_t> eie_start((size_t)NE + 1, 0), eie((size_t)eie_off[n]);
   std::vector<int32_t> mat((size_t)NE, 0), inst_e((size_t)NE, 0), inst_n((size_t)NN, 0);
+  const char* env = std::getenv("FIERRO_STAGED_TRANSFERS");
+  b->direct_host = xfer::direct_host_access() && !(env && env[0] == '1');
+  std::vector<int32_t> node_map(b->direct_host ? (size_t)NN : 0), elem_map(b->direct_host ? (size_t)NE : 0, 0);
   std::vector<uint8_t> bc((size_t)NN, 0);
   std::vector<double> qtab((size_t)b->mat_off[n] * 4), dtc((size_t)n);
 #pragma omp parallel for schedule(dynamic, 1) if (NE >= kHostParallel)
@@ -468,6 +535,10 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
     for (int64_t e = eo; e < b->elem_off[i + 1]; ++e)
       eie_start[e + 1] = (int32_t)(eie_off[i] + t.eie_start[std::min(e - eo + 1, t.ne)]);
     for (size_t k = 0; k < t.eie.size(); ++k) eie[(size_t)eie_off[i] + k] = (int32_t)(t.eie[k] + eo);
+    if (b->direct_host) {
+      for (int64_t k = 0; k < t.nn; ++k) node_map[no + k] = (int32_t)t.node_ext2int[k];
+      for (int64_t e = 0; e < t.ne; ++e) elem_map[eo + e] = (int32_t)t.elem_ext2int[e];
+    }
     const fierro_batch_instance& I = inst[i];
     for (int64_t m = 0; m < I.num_materials; ++m) {
       double* q = &qtab[(size_t)(b->mat_off[i] + m) * 4];
@@ -522,6 +593,9 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   TRY(balloc(b, &b->d_cfl, (size_t)(NE / kMinBatchBlock)));  // one partial per tile of the smallest block
   TRY(balloc(b, &b->d_ctrl, (size_t)n));
   TRY(balloc(b, &b->d_sync, 3));
+  TRY(balloc(b, &b->d_node_ext2int, node_map.size()));
+  TRY(balloc(b, &b->d_elem_ext2int, elem_map.size()));
+  TRY(balloc(b, &b->d_xfer, 1));
   CUDA_TRY(cudaMemsetAsync(b->d_sync, 0, 3 * sizeof(unsigned int), b->stream));
   TRY(put(b, b->d_nie, nie));
   TRY(put(b, b->d_cin_start, cin_start));
@@ -533,6 +607,8 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   TRY(put(b, b->d_inst_n, inst_n));
   TRY(put(b, b->d_part_start, b->part_start));
   TRY(put(b, b->d_bc, bc));
+  TRY(put(b, b->d_node_ext2int, node_map));
+  TRY(put(b, b->d_elem_ext2int, elem_map));
   TRY(put(b, b->d_qtab, qtab));
   TRY(put(b, b->d_dt_cfl, dtc));
   TRY(put(b, b->d_lps, b->lps));
@@ -547,12 +623,23 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   for (int64_t i = 0; i < n; ++i)
     stage = std::max<size_t>(stage, (size_t)std::max(inst[i].mesh.num_nodes, inst[i].mesh.num_elems));
   b->stage_elems = stage;
-  CUDA_TRY(cudaHostAlloc((void**)&b->h_stage, sizeof(double) * stage, cudaHostAllocDefault));
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   CUDA_TRY(cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, dev));
   TRY(apply_launch(b, NE < kSmallBatch ? fierro_batch_shape{32, 64, 32, 0, 0} : b->shape));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
+  return FIERRO_OK;
+}
+
+// The control block of an instance whose state is on its way, and the wait for both.
+int start_instance(fierro_batch* b, int64_t i) {
+  Ctrl c{};
+  c.dt = b->dt_start[i];
+  c.time_value = 0.0;
+  c.graphics_time = b->lps[i].graphics_dt_ival;
+  CUDA_TRY(cudaMemcpyAsync(b->d_ctrl + i, &c, sizeof(Ctrl), cudaMemcpyHostToDevice, b->stream));
+  CUDA_TRY(cudaStreamSynchronize(b->stream));
+  b->has_state[i] = 1;
   return FIERRO_OK;
 }
 
@@ -605,14 +692,37 @@ extern "C" int fierro_batch_set_state(fierro_batch* b, int64_t i, const fierro_s
   const HostTopo& t = b->topo[i];
   const int64_t nn = t.nn, ne = t.ne, nsv = s->num_state_vars;
   const int64_t nmat = b->mat_off[i + 1] - b->mat_off[i];
+  auto bad_volume = [&](int64_t e) {
+    return set_error(FIERRO_ENUMERIC, "batch: instance %lld element %lld volume %g", (long long)i, (long long)e,
+                     s->elem_vol[e]);
+  };
+  if (by_gpu(b, s)) {
+    // the checks go first: a refused state leaves the instance as it was
+    xfer::StateView v = view_of(b, i);
+    XferStatus xs{};
+    TRY(xfer::check_state(v, s, &xs));
+    const long long* first = xs.first;
+    const long long fe = std::min({first[XferStatus::MAT_ID], first[XferStatus::VOLUME], first[XferStatus::MASS]});
+    if (xs.flags & (1u << XferStatus::STRESS))
+      return set_error(FIERRO_ENOTSUP, "batch: non-zero stress needs a strength model");
+    if (fe < ne) {
+      if (first[XferStatus::MAT_ID] == fe) return set_error(FIERRO_EINVAL, "batch: material id out of range");
+      if (first[XferStatus::VOLUME] == fe) return bad_volume(fe);
+      return set_error(FIERRO_EINVAL, "batch: element mass <= 0");
+    }
+    if (xs.flags & (1u << XferStatus::NODE_MASS)) return set_error(FIERRO_EINVAL, "batch: node mass <= 0");
+    fierro_sgh_state sg = *s;
+    sg.elem_stress = nullptr;
+    if (!s->elem_div) v.div[1] = nullptr;
+    TRY(xfer::upload_state(v, &sg, &xs, false));
+    return start_instance(b, i);
+  }
   if (s->elem_stress)
     for (int64_t k = 0; k < ne * 18; ++k)
       if (s->elem_stress[k] != 0.0) return set_error(FIERRO_ENOTSUP, "batch: non-zero stress needs a strength model");
   for (int64_t e = 0; e < ne; ++e) {
     if (s->elem_mat_id[e] >= (uint64_t)nmat) return set_error(FIERRO_EINVAL, "batch: material id out of range");
-    if (!(s->elem_vol[e] > 0.0) || !std::isfinite(s->elem_vol[e]))
-      return set_error(FIERRO_ENUMERIC, "batch: instance %lld element %lld volume %g", (long long)i, (long long)e,
-                       s->elem_vol[e]);
+    if (!(s->elem_vol[e] > 0.0) || !std::isfinite(s->elem_vol[e])) return bad_volume(e);
     if (!(s->elem_mass[e] > 0.0)) return set_error(FIERRO_EINVAL, "batch: element mass <= 0");
   }
   for (int64_t k = 0; k < nn; ++k)
@@ -638,14 +748,7 @@ extern "C" int fierro_batch_set_state(fierro_batch* b, int64_t i, const fierro_s
   std::vector<int32_t> mat((size_t)ne);
   for (int64_t e = 0; e < ne; ++e) mat[e] = (int32_t)(s->elem_mat_id[t.elem_int2ext[e]] + (uint64_t)b->mat_off[i]);
   CUDA_TRY(cudaMemcpyAsync(b->d_mat + eo, mat.data(), sizeof(int32_t) * (size_t)ne, cudaMemcpyHostToDevice, b->stream));
-  Ctrl c{};
-  c.dt = b->dt_start[i];
-  c.time_value = 0.0;
-  c.graphics_time = b->lps[i].graphics_dt_ival;
-  CUDA_TRY(cudaMemcpyAsync(b->d_ctrl + i, &c, sizeof(Ctrl), cudaMemcpyHostToDevice, b->stream));
-  CUDA_TRY(cudaStreamSynchronize(b->stream));
-  b->has_state[i] = 1;
-  return FIERRO_OK;
+  return start_instance(b, i);
 }
 
 extern "C" int fierro_batch_run(fierro_batch* b, int64_t cycles) {
@@ -690,6 +793,19 @@ extern "C" int fierro_batch_get_state(fierro_batch* b, int64_t i, fierro_sgh_sta
   const HostTopo& t = b->topo[i];
   const int64_t nn = t.nn, ne = t.ne, no = b->node_off[i], eo = b->elem_off[i];
   const int bins[2] = {b0, b1};
+  const long long stages_done = c.cycle * b->rk_num_stages;
+  const int qb = stages_done == 0 ? 1 : (int)((stages_done - 1) & 1);
+  if (by_gpu(b, s)) {
+    const size_t nb = sizeof(double), n = (size_t)nn, m = (size_t)ne;
+    const std::pair<double*, size_t> out[] = {
+        {s->node_coords, 6 * n}, {s->node_vel, 6 * n}, {s->node_mass, n}, {s->elem_sie, 2 * m}, {s->elem_den, m},
+        {s->elem_pres, m}, {s->elem_sspd, m}, {s->elem_vol, m}, {s->elem_mass, m}, {s->elem_div, m},
+        {s->elem_stress, 18 * m}, {s->corner_force, 24 * m}};
+    for (const auto& a : out) populate(a.first, nb * a.second);
+    TRY(xfer::download_state(view_of(b, i), s, bins, qb, false));
+    CUDA_TRY(cudaStreamSynchronize(b->stream));
+    return FIERRO_OK;
+  }
   for (int rb = 0; rb < 2; ++rb)
     for (int d = 0; d < 3; ++d) {
       if (s->node_coords)
@@ -706,11 +822,7 @@ extern "C" int fierro_batch_get_state(fierro_batch* b, int64_t i, fierro_sgh_sta
   if (s->elem_sspd) TRY(scatter_down(b, s->elem_sspd, b->d_sspd, eo, t.elem_int2ext, 1, 0));
   if (s->elem_vol) TRY(scatter_down(b, s->elem_vol, b->d_vol, eo, t.elem_int2ext, 1, 0));
   if (s->elem_mass) TRY(scatter_down(b, s->elem_mass, b->d_elem_mass, eo, t.elem_int2ext, 1, 0));
-  if (s->elem_div) {
-    const long long stages_done = c.cycle * b->rk_num_stages;
-    const int qb = stages_done == 0 ? 1 : (int)((stages_done - 1) & 1);
-    TRY(scatter_down(b, s->elem_div, b->d_div[qb], eo, t.elem_int2ext, 1, 0));
-  }
+  if (s->elem_div) TRY(scatter_down(b, s->elem_div, b->d_div[qb], eo, t.elem_int2ext, 1, 0));
   if (s->elem_stress) std::memset(s->elem_stress, 0, sizeof(double) * (size_t)ne * 18);
   if (s->corner_force)
     for (int r = 0; r < 24; ++r)

@@ -651,9 +651,9 @@ static int set_state_impl(fierro_sgh* h, const fierro_sgh_state* s, double time_
     const bool host_check = s->elem_stress && !h->strength;
     fierro_sgh_state sg = *s;
     if (host_check) sg.elem_stress = nullptr;
-    TRY(xfer::upload_state(h, &sg, &xs, false));
+    TRY(xfer::upload_state(xfer::view_of(h), &sg, &xs, false));
     const long long nonzero = host_check ? first_nonzero(s->elem_stress, ne * 18) : -1;
-    TRY(xfer::finish_upload(h, &xs));
+    TRY(xfer::finish_upload(xfer::view_of(h), &xs));
     if (nonzero >= 0) {
       xs.flags |= 1u << XferStatus::STRESS;
       xs.first[XferStatus::STRESS] = nonzero;
@@ -735,17 +735,6 @@ extern "C" int fierro_sgh_set_state(fierro_sgh* h, const fierro_sgh_state* s) {
   return set_state_impl(h, s, 0.0, h->lp.graphics_dt_ival, h->dt_start);
 }
 
-// One store per page, in parallel, so that the pages of an output array exist
-// before the GPU writes it (the array is overwritten completely afterwards).
-static void populate(double* p, size_t bytes) {
-  if (!p || bytes == 0) return;
-  static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
-  char* c = reinterpret_cast<char*>(p);
-  const int64_t n = (int64_t)((bytes + page - 1) / page);
-#pragma omp parallel for schedule(static)
-  for (int64_t k = 0; k < n; ++k) *(volatile char*)(c + (size_t)k * page) = 0;
-}
-
 extern "C" int fierro_sgh_get_state(fierro_sgh* h, fierro_sgh_state* s) {
   clear_error();
   NvtxRange nvtx_("fierro_sgh_get_state");
@@ -786,7 +775,7 @@ extern "C" int fierro_sgh_get_state(fierro_sgh* h, fierro_sgh_state* s) {
     if (!host_zero) populate(s->elem_stress, nb * ne * 18);
     fierro_sgh_state sg = *s;
     if (host_zero) sg.elem_stress = nullptr;
-    TRY(xfer::download_state(h, &sg, bins, qb, false));
+    TRY(xfer::download_state(xfer::view_of(h), &sg, bins, qb, false));
     if (host_zero) zero_parallel(s->elem_stress, (size_t)ne * 18);
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return FIERRO_OK;

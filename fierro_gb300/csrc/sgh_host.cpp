@@ -12,6 +12,8 @@
 #include <numeric>
 #include <vector>
 
+#include <unistd.h>
+
 #ifdef _OPENMP
 #include <omp.h>
 #endif
@@ -25,6 +27,15 @@
 namespace fierro {
 
 static thread_local std::string g_err;
+
+void populate(double* p, size_t bytes) {
+  if (!p || bytes == 0) return;
+  static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
+  char* c = reinterpret_cast<char*>(p);
+  const int64_t n = (int64_t)((bytes + page - 1) / page);
+#pragma omp parallel for schedule(static)
+  for (int64_t k = 0; k < n; ++k) *(volatile char*)(c + (size_t)k * page) = 0;
+}
 
 int set_error(int code, const char* fmt, ...) {
   char buf[1024];

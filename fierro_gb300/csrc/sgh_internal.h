@@ -37,6 +37,10 @@ struct NvtxRange {
 int set_error(int code, const char* fmt, ...);
 void clear_error();
 
+// One store per page, in parallel, so that the pages of an output array exist
+// before the GPU writes it (the array is overwritten completely afterwards).
+void populate(double* p, size_t bytes);
+
 // Host-side mesh topology in the device ("internal") numbering.
 //
 // Elements and nodes are renumbered along a Morton curve of their positions, for

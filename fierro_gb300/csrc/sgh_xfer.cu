@@ -29,6 +29,17 @@ __device__ __forceinline__ void flag(XferStatus* st, int which, long long idx) {
   atomicMin(&st->first[which], idx);
 }
 
+__global__ void __launch_bounds__(kBlock) k_check_state(int nn, int ne, int nmat, const double* node_mass,
+                                                        const uint64_t* mat_id, const double* vol,
+                                                        const double* mass, XferStatus* st) {
+  const int k = blockIdx.x * kBlock + threadIdx.x;
+  if (k < nn && !(node_mass[k] > 0.0)) flag(st, XferStatus::NODE_MASS, k);
+  if (k >= ne) return;
+  if (mat_id[k] >= (uint64_t)nmat) flag(st, XferStatus::MAT_ID, k);
+  if (!(vol[k] > 0.0) || !isfinite(vol[k])) flag(st, XferStatus::VOLUME, k);
+  if (!(mass[k] > 0.0)) flag(st, XferStatus::MASS, k);
+}
+
 struct NodeUp {
   int nn, dims;                        // dims: 3 (hex) or 2 (2D-RZ quads)
   const int* ext2int;
@@ -68,7 +79,7 @@ __global__ void __launch_bounds__(kBlock) k_up_nodes(const NodeUp a) {
 }
 
 struct ElemUp {
-  int ne, nmat, nsv;
+  int ne, nmat, nsv, mat_base;
   const int* ext2int;
   const double *sie, *den, *pres, *sspd, *vol, *mass, *statev, *div;
   const uint64_t* mat_id;
@@ -96,9 +107,9 @@ __global__ void __launch_bounds__(kBlock) k_up_elems(const ElemUp a) {
   a.d_mass[e] = mass;
   a.d_gamma[e] = a.statev[(size_t)E * a.nsv];
   a.d_csmin[e] = a.statev[(size_t)E * a.nsv + 1];
-  a.d_div[e] = a.div ? a.div[E] : 0.0;
+  if (a.d_div) a.d_div[e] = a.div ? a.div[E] : 0.0;
   const uint64_t mid = a.mat_id[E];
-  a.d_mat[e] = mid < (uint64_t)a.nmat ? (int)mid : 0;
+  a.d_mat[e] = a.mat_base + (mid < (uint64_t)a.nmat ? (int)mid : 0);
   if (mid >= (uint64_t)a.nmat) flag(a.st, XferStatus::MAT_ID, E);
   if (!(vol > 0.0) || !isfinite(vol)) flag(a.st, XferStatus::VOLUME, E);
   if (!(mass > 0.0)) flag(a.st, XferStatus::MASS, E);
@@ -177,6 +188,7 @@ __global__ void __launch_bounds__(kBlock) k_down_nodes(const NodeDown a) {
 struct ElemDown {
   int ne, nsv;
   int force_rows;  // corner-force values per element: 24 (hex) or 8 (quad)
+  long long force_stride;
   const int* ext2int;
   double *sie, *den, *pres, *sspd, *vol, *div, *mass, *stress, *corner_force, *statev;  // may be null
   const double* d_sie[2];  // reference bin rb
@@ -234,7 +246,7 @@ __global__ void __launch_bounds__(kBlock) k_down_force(const ElemDown a) {
   const int cnt = min(kForceChunk, a.ne - E0);
   for (int k = threadIdx.x; k < cnt * R; k += kBlock) {
     const int E = E0 + k / R, r = k % R;
-    buf[k] = a.d_force[(size_t)r * a.ne + a.ext2int[E]];
+    buf[k] = a.d_force[(size_t)r * a.force_stride + a.ext2int[E]];
   }
   __syncthreads();
   store_run(a.corner_force + (size_t)E0 * R, buf, cnt * R);
@@ -322,34 +334,92 @@ bool direct_host_access() {
   return v != 0;
 }
 
-int upload_state(fierro_sgh* h, const fierro_sgh_state* s, XferStatus* host_status, bool wait) {
-  const int nn = (int)h->nn, ne = (int)h->ne;
-  cudaStream_t stream = h->stream;
+StateView view_of(fierro_sgh* h) {
+  StateView v{};
+  v.nn = (int)h->nn;
+  v.ne = (int)h->ne;
+  v.nmat = h->nmat;
+  v.dims = h->dims;
+  v.nsv = h->nsv;
+  v.strength = h->strength;
+  v.force_stride = h->ne;
+  v.stream = h->stream;
+  v.status = h->d_xfer;
+  v.node_ext2int = h->d_node_ext2int;
+  v.elem_ext2int = h->d_elem_ext2int;
+  for (int b = 0; b < 2; ++b) {
+    for (int d = 0; d < 3; ++d) {
+      v.x[b][d] = h->d_x[b][d];
+      v.v[b][d] = h->d_v[b][d];
+    }
+    v.sie[b] = h->d_sie[b];
+    v.div[b] = h->d_div[b];
+    v.stress[b] = h->d_stress[b];
+  }
+  v.node_mass = h->d_node_mass;
+  v.den = h->d_den;
+  v.pres = h->d_pres;
+  v.sspd = h->d_sspd;
+  v.vol = h->d_vol;
+  v.elem_mass = h->d_elem_mass;
+  v.gamma = h->d_gamma;
+  v.csmin = h->d_csmin;
+  v.force = h->d_force;
+  v.statev = h->d_statev;
+  v.mat = h->d_mat;
+  return v;
+}
+
+static int reset_status(const StateView& h) {
   XferStatus init{};
-  init.flags = 0;
   for (int k = 0; k < XferStatus::COUNT; ++k) init.first[k] = LLONG_MAX;
-  CUDA_TRY(cudaMemcpyAsync(h->d_xfer, &init, sizeof(init), cudaMemcpyHostToDevice, stream));
-  const int D = h->dims == 2 ? 2 : 3;
+  CUDA_TRY(cudaMemcpyAsync(h.status, &init, sizeof(init), cudaMemcpyHostToDevice, h.stream));
+  return FIERRO_OK;
+}
+
+static int check_zero_stress(const StateView& h, const double* stress) {
+  int dev = 0, sms = 0;
+  CUDA_TRY(cudaGetDevice(&dev));
+  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  k_check_zero<<<sms * 8, kBlock, 0, h.stream>>>(stress, (long long)h.ne * 18, h.status);
+  return FIERRO_OK;
+}
+
+int check_state(const StateView& h, const fierro_sgh_state* s, XferStatus* host_status) {
+  TRY(reset_status(h));
+  k_check_state<<<blocks(h.nn > h.ne ? h.nn : h.ne), kBlock, 0, h.stream>>>(
+      h.nn, h.ne, h.nmat, s->node_mass, s->elem_mat_id, s->elem_vol, s->elem_mass, h.status);
+  if (s->elem_stress && !h.strength) TRY(check_zero_stress(h, s->elem_stress));
+  CUDA_TRY(cudaGetLastError());
+  return finish_upload(h, host_status);
+}
+
+int upload_state(const StateView& h, const fierro_sgh_state* s, XferStatus* host_status, bool wait) {
+  const int nn = h.nn, ne = h.ne;
+  cudaStream_t stream = h.stream;
+  TRY(reset_status(h));
+  const int D = h.dims == 2 ? 2 : 3;
   NodeUp nu{};
   nu.nn = nn;
   nu.dims = D;
-  nu.ext2int = h->d_node_ext2int;
+  nu.ext2int = h.node_ext2int;
   nu.coords = s->node_coords;
   nu.vel = s->node_vel;
   nu.mass = s->node_mass;
   for (int b = 0; b < 2; ++b)
     for (int d = 0; d < D; ++d) {
-      nu.x[b][d] = h->d_x[b][d];
-      nu.v[b][d] = h->d_v[b][d];
+      nu.x[b][d] = h.x[b][d];
+      nu.v[b][d] = h.v[b][d];
     }
-  nu.node_mass = h->d_node_mass;
-  nu.st = h->d_xfer;
+  nu.node_mass = h.node_mass;
+  nu.st = h.status;
   k_up_nodes<<<blocks(nn), kBlock, 0, stream>>>(nu);
   ElemUp eu{};
   eu.ne = ne;
-  eu.nmat = h->nmat;
+  eu.nmat = h.nmat;
+  eu.mat_base = h.mat_base;
   eu.nsv = (int)s->num_state_vars;
-  eu.ext2int = h->d_elem_ext2int;
+  eu.ext2int = h.elem_ext2int;
   eu.sie = s->elem_sie;
   eu.den = s->elem_den;
   eu.pres = s->elem_pres;
@@ -359,71 +429,66 @@ int upload_state(fierro_sgh* h, const fierro_sgh_state* s, XferStatus* host_stat
   eu.statev = s->elem_statev;
   eu.div = s->elem_div;
   eu.mat_id = s->elem_mat_id;
-  eu.d_sie[0] = h->d_sie[0];
-  eu.d_sie[1] = h->d_sie[1];
-  eu.d_den = h->d_den;
-  eu.d_pres = h->d_pres;
-  eu.d_sspd = h->d_sspd;
-  eu.d_vol = h->d_vol;
-  eu.d_mass = h->d_elem_mass;
-  eu.d_gamma = h->d_gamma;
-  eu.d_csmin = h->d_csmin;
-  eu.d_div = h->d_div[1];  // the caller's elem_div is what the reference shows before any stage runs
-  eu.d_mat = h->d_mat;
-  eu.st = h->d_xfer;
-  if (h->strength) {
+  eu.d_sie[0] = h.sie[0];
+  eu.d_sie[1] = h.sie[1];
+  eu.d_den = h.den;
+  eu.d_pres = h.pres;
+  eu.d_sspd = h.sspd;
+  eu.d_vol = h.vol;
+  eu.d_mass = h.elem_mass;
+  eu.d_gamma = h.gamma;
+  eu.d_csmin = h.csmin;
+  eu.d_div = h.div[1];  // the caller's elem_div is what the reference shows before any stage runs
+  eu.d_mat = h.mat;
+  eu.st = h.status;
+  if (h.strength) {
     eu.stress = s->elem_stress;
-    eu.d_stress[0] = h->d_stress[0];
-    eu.d_stress[1] = h->d_stress[1];
-    eu.d_statev = h->d_statev;
+    eu.d_stress[0] = h.stress[0];
+    eu.d_stress[1] = h.stress[1];
+    eu.d_statev = h.statev;
     if (!s->elem_stress) {
       int dev = 0, sms = 0;
       CUDA_TRY(cudaGetDevice(&dev));
       CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      for (int b = 0; b < 2; ++b) k_zero<<<sms * 4, kBlock, 0, stream>>>(h->d_stress[b], (long long)ne * 9);
+      for (int b = 0; b < 2; ++b) k_zero<<<sms * 4, kBlock, 0, stream>>>(h.stress[b], (long long)ne * 9);
     }
   }
   k_up_elems<<<blocks(ne), kBlock, 0, stream>>>(eu);
-  if (s->elem_stress && !h->strength) {
-    int dev = 0, sms = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
-    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    k_check_zero<<<sms * 8, kBlock, 0, stream>>>(s->elem_stress, (long long)ne * 18, h->d_xfer);
-  }
+  if (s->elem_stress && !h.strength) TRY(check_zero_stress(h, s->elem_stress));
   CUDA_TRY(cudaGetLastError());
   return wait ? finish_upload(h, host_status) : FIERRO_OK;
 }
 
-int finish_upload(fierro_sgh* h, XferStatus* host_status) {
-  CUDA_TRY(cudaMemcpyAsync(host_status, h->d_xfer, sizeof(XferStatus), cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(cudaStreamSynchronize(h->stream));
+int finish_upload(const StateView& h, XferStatus* host_status) {
+  CUDA_TRY(cudaMemcpyAsync(host_status, h.status, sizeof(XferStatus), cudaMemcpyDeviceToHost, h.stream));
+  CUDA_TRY(cudaStreamSynchronize(h.stream));
   return FIERRO_OK;
 }
 
-int download_state(fierro_sgh* h, fierro_sgh_state* s, const int bins[2], int div_buffer, bool wait) {
-  const int nn = (int)h->nn, ne = (int)h->ne;
-  cudaStream_t stream = h->stream;
-  const int D = h->dims == 2 ? 2 : 3;
+int download_state(const StateView& h, fierro_sgh_state* s, const int bins[2], int div_buffer, bool wait) {
+  const int nn = h.nn, ne = h.ne;
+  cudaStream_t stream = h.stream;
+  const int D = h.dims == 2 ? 2 : 3;
   if (s->node_coords || s->node_vel || s->node_mass) {
     NodeDown nd{};
     nd.nn = nn;
     nd.dims = D;
-    nd.ext2int = h->d_node_ext2int;
+    nd.ext2int = h.node_ext2int;
     nd.coords = s->node_coords;
     nd.vel = s->node_vel;
     nd.mass = s->node_mass;
     for (int rb = 0; rb < 2; ++rb)
       for (int d = 0; d < D; ++d) {
-        nd.x[rb][d] = h->d_x[bins[rb]][d];
-        nd.v[rb][d] = h->d_v[bins[rb]][d];
+        nd.x[rb][d] = h.x[bins[rb]][d];
+        nd.v[rb][d] = h.v[bins[rb]][d];
       }
-    nd.node_mass = h->d_node_mass;
+    nd.node_mass = h.node_mass;
     k_down_nodes<<<blocks(nn), kBlock, 0, stream>>>(nd);
   }
   ElemDown ed{};
   ed.ne = ne;
   ed.force_rows = D == 2 ? 8 : 24;
-  ed.ext2int = h->d_elem_ext2int;
+  ed.ext2int = h.elem_ext2int;
   ed.sie = s->elem_sie;
   ed.den = s->elem_den;
   ed.pres = s->elem_pres;
@@ -433,21 +498,22 @@ int download_state(fierro_sgh* h, fierro_sgh_state* s, const int bins[2], int di
   ed.mass = s->elem_mass;
   ed.stress = s->elem_stress;
   ed.corner_force = s->corner_force;
-  ed.d_sie[0] = h->d_sie[bins[0]];
-  ed.d_sie[1] = h->d_sie[bins[1]];
-  ed.d_den = h->d_den;
-  ed.d_pres = h->d_pres;
-  ed.d_sspd = h->d_sspd;
-  ed.d_vol = h->d_vol;
-  ed.d_div = h->d_div[div_buffer];
-  ed.d_mass = h->d_elem_mass;
-  ed.d_force = h->d_force;
-  if (h->strength) {
-    ed.d_stress[0] = h->d_stress[bins[0]];
-    ed.d_stress[1] = h->d_stress[bins[1]];
+  ed.d_sie[0] = h.sie[bins[0]];
+  ed.d_sie[1] = h.sie[bins[1]];
+  ed.d_den = h.den;
+  ed.d_pres = h.pres;
+  ed.d_sspd = h.sspd;
+  ed.d_vol = h.vol;
+  ed.d_div = h.div[div_buffer];
+  ed.d_mass = h.elem_mass;
+  ed.d_force = h.force;
+  ed.force_stride = h.force_stride;
+  if (h.strength) {
+    ed.d_stress[0] = h.stress[bins[0]];
+    ed.d_stress[1] = h.stress[bins[1]];
     ed.statev = s->elem_statev;
-    ed.nsv = (int)h->nsv;
-    ed.d_statev = h->d_statev;
+    ed.nsv = (int)h.nsv;
+    ed.d_statev = h.statev;
   }
   k_down_elems<<<blocks(ne), kBlock, 0, stream>>>(ed);
   if (s->corner_force) k_down_force<<<(unsigned)((ne + kForceChunk - 1) / kForceChunk), kBlock, 0, stream>>>(ed);

@@ -25,21 +25,40 @@ namespace xfer {
 
 // True when kernels may dereference pageable host pointers on the current device.
 bool direct_host_access();
-// Uploads a state (reference layouts) into the handle's bins and reports the
+// One problem's arrays on the device: a handle's, or one instance's part of a
+// batch's (pointers at its first node or element, forces `force_stride` apart).
+struct StateView {
+  int nn, ne, nmat, dims;
+  int mat_base;  // added to the caller's material ids
+  bool strength;
+  int64_t nsv;   // state variables held (strength)
+  long long force_stride;
+  cudaStream_t stream;
+  XferStatus* status;
+  const int *node_ext2int, *elem_ext2int;
+  double *x[2][3], *v[2][3], *sie[2], *div[2], *stress[2];
+  double *node_mass, *den, *pres, *sspd, *vol, *elem_mass, *gamma, *csmin, *force, *statev;
+  int* mat;
+};
+StateView view_of(fierro_sgh* h);
+// The checks of an upload alone, the zero stress included: writes nothing on the
+// device but the status.
+int check_state(const StateView& h, const fierro_sgh_state* s, XferStatus* status);
+// Uploads a state (reference layouts) into the bins and reports the
 // validation result; the state on the device is the caller's even when a check
-// failed (the caller then discards it).  A strength handle also takes the stress
-// bins and all num_state_vars state variables (h->d_statev sized for them).
-// With wait == false the transfers are only enqueued on the handle's stream and
-// `status` is not written: the caller does host work meanwhile, then calls
+// failed (the caller then discards it).  A view with strength also takes the stress
+// bins and all num_state_vars state variables (statev sized for them); div[1] may be
+// null (left as it is).  With wait == false the transfers are only enqueued on the
+// stream and `status` is not written: the caller does host work meanwhile, then calls
 // finish_upload.
-int upload_state(fierro_sgh* h, const fierro_sgh_state* s, XferStatus* status, bool wait = true);
-int finish_upload(fierro_sgh* h, XferStatus* status);
-// Writes the handle's state into the non-null fields of `s`: reference bin rb
-// from device bin bins[rb]; elem_div from divergence buffer div_buffer.  On a
-// handle with strength materials the stress bins and the state variables come
+int upload_state(const StateView& h, const fierro_sgh_state* s, XferStatus* status, bool wait = true);
+int finish_upload(const StateView& h, XferStatus* status);
+// Writes the state into the non-null fields of `s`: reference bin rb
+// from device bin bins[rb]; elem_div from divergence buffer div_buffer.  With
+// strength the stress bins and the state variables come
 // from the device; otherwise the stress is zero and elem_statev is not written.
-// wait == false: enqueued only; the caller synchronises the handle's stream.
-int download_state(fierro_sgh* h, fierro_sgh_state* s, const int bins[2], int div_buffer, bool wait = true);
+// wait == false: enqueued only; the caller synchronises the stream.
+int download_state(const StateView& h, fierro_sgh_state* s, const int bins[2], int div_buffer, bool wait = true);
 
 // Graphics-dump snapshots (write_outputs, outputs.cpp:10-506): one slot of the
 // device ring holds, in the caller's numbering, node rows x, y, z, u, v, w
