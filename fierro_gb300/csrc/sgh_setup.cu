@@ -275,7 +275,7 @@ int run(const fierro_mesh* mesh, const double* state_vars, int64_t num_state_var
       cudaStreamDestroy(s);
     }
   } guard{st};
-  Scratch sc;
+  Scratch sc((288 + 8 * (size_t)nsv) * (size_t)ne + 68 * (size_t)nn);
   int* nie = nullptr;
   double *xyz = nullptr, *vol = nullptr;
   Status* d_st = nullptr;

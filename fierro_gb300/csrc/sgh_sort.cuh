@@ -144,35 +144,48 @@ __global__ void k_scan_add(long long n, unsigned* __restrict__ out, const unsign
   if (i < n) out[i] += sums[i / kScanChunk];
 }
 
-// Device memory of one set-up call, given back at its end.  Arrays of small meshes
-// share allocations of kChunk bytes: some forty arrays of a 12^3 mesh took as long to
-// allocate and free as its sorts.
+// Device memory of one set-up call, given back at its end: parts of one allocation of
+// the expected size (some forty arrays of a 12^3 mesh took as long to allocate and free
+// as its sorts), what does not fit by itself.
 struct Scratch {
-  static constexpr size_t kChunk = 1 << 20, kAlign = 256;
+  static constexpr size_t kAlign = 256;
   std::vector<void*> p;
-  char* chunk = nullptr;
-  size_t used = 0;
+  char* block = nullptr;
+  size_t size, used = 0;
+  explicit Scratch(size_t expected) : size(expected + (64 << 10)) {}
   ~Scratch() {
+    if (block) cudaFree(block);
     for (void* q : p) cudaFree(q);
+  }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  // Everything allocated so far is free for reuse (whatever used it has finished).
+  void reset() {
+    for (void* q : p) cudaFree(q);
+    p.clear();
+    used = 0;
   }
   template <typename T>
   int alloc(T** out, size_t n) {
     const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + kAlign - 1) / kAlign * kAlign;
-    const bool small = bytes <= kChunk / 4;
-    if (!small || !chunk || used + bytes > kChunk) {
+    if (!block && size) {
       void* q = nullptr;
-      if (cudaMalloc(&q, small ? kChunk : bytes) != cudaSuccess)
-        return set_error(FIERRO_ENOMEM, "topology: cudaMalloc(%zu bytes) failed", small ? kChunk : bytes);
-      p.push_back(q);
-      if (!small) {
-        *out = static_cast<T*>(q);
-        return FIERRO_OK;
+      if (cudaMalloc(&q, size) != cudaSuccess) {
+        cudaGetLastError();
+        size = 0;  // each array by itself
       }
-      chunk = static_cast<char*>(q);
-      used = 0;
+      block = static_cast<char*>(q);
     }
-    *out = reinterpret_cast<T*>(chunk + used);
-    used += bytes;
+    if (used + bytes <= size) {
+      *out = reinterpret_cast<T*>(block + used);
+      used += bytes;
+      return FIERRO_OK;
+    }
+    void* q = nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess)
+      return set_error(FIERRO_ENOMEM, "topology: cudaMalloc(%zu bytes) failed", bytes);
+    p.push_back(q);
+    *out = static_cast<T*>(q);
     return FIERRO_OK;
   }
 };

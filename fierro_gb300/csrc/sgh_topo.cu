@@ -308,10 +308,12 @@ __global__ void k_mask_u8(int nn, const unsigned* __restrict__ in, unsigned char
 
 }  // namespace
 
-int build_device(fierro_sgh* h, const fierro_mesh* mesh, const fierro_boundary* bcs, int64_t num_bcs) {
+// Bytes `build` takes of its scratch memory, to a few percent.
+static size_t build_bytes(size_t nn, size_t ne) { return 300 * ne + 44 * nn; }
+
+static int build(fierro_sgh* h, const fierro_mesh* mesh, const fierro_boundary* bcs, int64_t num_bcs, Scratch& sc) {
   const int nn = (int)mesh->num_nodes, ne = (int)mesh->num_elems;
   cudaStream_t st = h->stream;
-  Scratch sc;
   // ---- caller arrays, read by the GPU; validation
   int* nie_ext = nullptr;
   double* xyz = nullptr;
@@ -432,6 +434,11 @@ int build_device(fierro_sgh* h, const fierro_mesh* mesh, const fierro_boundary* 
   CUDA_TRY(cudaStreamSynchronize(st));
   t.elem_int2ext.assign(tmp.begin(), tmp.begin() + ne);
   return FIERRO_OK;
+}
+
+int build_device(fierro_sgh* h, const fierro_mesh* mesh, const fierro_boundary* bcs, int64_t num_bcs) {
+  Scratch sc(build_bytes((size_t)mesh->num_nodes, (size_t)mesh->num_elems));
+  return build(h, mesh, bcs, num_bcs, sc);
 }
 
 }  // namespace topo
