@@ -18,10 +18,12 @@
 #include <vector>
 
 #include <cuda_runtime.h>
+#include <omp.h>
 
 #include "fierro_sgh.h"
 #include "sgh_device.h"
 #include "sgh_internal.h"
+#include "sgh_topo.h"
 #include "sgh_xfer.h"
 
 using namespace fierro;
@@ -430,17 +432,28 @@ int check_instance(const fierro_batch_instance& I, const fierro_sgh_params& p0, 
   return FIERRO_OK;
 }
 
-// The instances' topologies, inst[0..count): several at a time, one host thread
-// each (build_topology's own loops are too short to fill the threads on an
-// ensemble's meshes: twelve decks of 148,000 elements 56 ms one after the other);
-// instances above an eighth of the ensemble run by themselves over all threads.
+// What an instance's topology takes, ns: on the GPU kGpuTopo + kGpuTopoElem an element
+// (one after the other), on one host thread kHostTopoElem an element (a batch of one
+// 32^3 mesh is made in 3.1 ms with the GPU, 20.5 with one host thread, 6.0 with its
+// loops over sixteen).  Batches, ms, host threads alone against both: twelve decks of
+// 148,000 elements 25.7 / 10.5, 96 decks of 3.9 million 258 / 155, twelve of 20^3 (the
+// host's alone) 6.6 / 7.1.
+constexpr double kGpuTopo = 8e5, kGpuTopoElem = 30, kHostTopoElem = 600;
+
+// The instances' topologies, inst[0..count).  Where the GPU can read the meshes in
+// place it builds the largest, driven by this thread, while the other host threads
+// take the rest, one each; how many go to the GPU is what makes the later of the two
+// end earliest.  What is left (all without the GPU, and any mesh its builder turned
+// down, whose answer is the host builder's) follows on the host: instances above an
+// eighth of the ensemble by themselves over all threads, the others one thread each.
 // Reports the error of the lowest-numbered instance, as one after the other did.
 int build_topologies(fierro_batch* b, const fierro_batch_instance* inst, int64_t count) {
   std::vector<int> rc((size_t)count, FIERRO_OK);
   std::vector<std::string> msg((size_t)count);
-  int64_t total = 0;
-  for (int64_t i = 0; i < count; ++i) total += std::max<int64_t>(inst[i].mesh.num_elems, 0);
+  std::vector<char> done((size_t)count, 0);
   auto one = [&](int64_t i) {
+    if (done[i]) return;
+    done[i] = 1;
     try {
       rc[i] = build_topology(&inst[i].mesh, inst[i].boundaries, inst[i].num_bcs, true, &b->topo[i]);
       if (rc[i]) msg[i] = fierro_last_error();
@@ -448,6 +461,54 @@ int build_topologies(fierro_batch* b, const fierro_batch_instance* inst, int64_t
       rc[i] = FIERRO_ENOMEM;
     }
   };
+  auto elems = [&](int64_t i) { return std::max<int64_t>(inst[i].mesh.num_elems, 0); };
+  int64_t total = 0;
+  for (int64_t i = 0; i < count; ++i) total += elems(i);
+  if (b->direct_host) {
+    std::vector<int64_t> order;  // the meshes the GPU can read, largest first
+    double host = 0.0;
+    for (int64_t i = 0; i < count; ++i) {
+      const fierro_mesh& m = inst[i].mesh;
+      if (((reinterpret_cast<uintptr_t>(m.nodes_in_elem) | reinterpret_cast<uintptr_t>(m.coords)) & 7) == 0) {
+        order.push_back(i);
+        host += kHostTopoElem * (double)elems(i);
+      }
+    }
+    std::sort(order.begin(), order.end(), [&](int64_t p, int64_t q) {
+      return elems(p) != elems(q) ? elems(p) > elems(q) : p < q;
+    });
+    const double threads = std::max(1, omp_get_max_threads());
+    double gpu = 0.0, best = 1e300;
+    size_t take = 0;
+    for (size_t k = 0; k <= order.size(); ++k) {
+      const double longest = k < order.size() ? kHostTopoElem * (double)elems(order[k]) : 0.0;
+      const double rest = std::max(longest, host / threads);
+      const double end = threads > 1 ? std::max(gpu, rest) : gpu + host;
+      if (end < best) best = end, take = k;
+      if (k < order.size()) {
+        gpu += kGpuTopo + kGpuTopoElem * (double)elems(order[k]);
+        host -= longest;
+      }
+    }
+    std::vector<topo::ToHost> list;
+    for (size_t k = 0; k < take; ++k) {
+      const int64_t i = order[k];
+      list.push_back({&inst[i].mesh, inst[i].boundaries, inst[i].num_bcs, &b->topo[i]});
+    }
+    std::vector<char> ok(list.size(), 0);
+    const int64_t left = (int64_t)order.size();
+#pragma omp parallel
+    {
+#pragma omp master
+      topo::build_to_host(list, &ok);
+#pragma omp for schedule(dynamic, 1)
+      for (int64_t k = (int64_t)take; k < left; ++k) one(order[(size_t)k]);
+    }
+    for (size_t k = 0; k < take; ++k) {
+      done[order[k]] = ok[k];
+      if (!ok[k]) b->topo[order[k]] = HostTopo{};
+    }
+  }
   auto alone = [&](int64_t i) { return inst[i].mesh.num_elems > total / 8; };
   for (int64_t i = 0; i < count; ++i)
     if (alone(i)) one(i);
@@ -478,6 +539,8 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   b->lps.resize((size_t)n);
   b->dt_start.resize((size_t)n);
   b->has_state.assign((size_t)n, 0);
+  const char* env = std::getenv("FIERRO_STAGED_TRANSFERS");
+  b->direct_host = xfer::direct_host_access() && !(env && env[0] == '1');
   // the instances' controls in order, up to the first that is refused
   int64_t checked = 0;
   int bad_rc = FIERRO_OK;
@@ -515,8 +578,6 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
   std::vector<int32_t> nie((size_t)NE * 8, 0), cin_start((size_t)NN + 1, 0), cin((size_t)cin_off[n]);
   std::vector<int32_t> eie_start((size_t)NE + 1, 0), eie((size_t)eie_off[n]);
   std::vector<int32_t> mat((size_t)NE, 0), inst_e((size_t)NE, 0), inst_n((size_t)NN, 0);
-  const char* env = std::getenv("FIERRO_STAGED_TRANSFERS");
-  b->direct_host = xfer::direct_host_access() && !(env && env[0] == '1');
   std::vector<int32_t> node_map(b->direct_host ? (size_t)NN : 0), elem_map(b->direct_host ? (size_t)NE : 0, 0);
   std::vector<uint8_t> bc((size_t)NN, 0);
   std::vector<double> qtab((size_t)b->mat_off[n] * 4), dtc((size_t)n);

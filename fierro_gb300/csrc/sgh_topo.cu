@@ -18,6 +18,8 @@
 #include <climits>
 #include <cmath>
 #include <cstdint>
+#include <exception>
+#include <utility>
 #include <vector>
 
 #include "sgh_handle.h"
@@ -439,6 +441,76 @@ static int build(fierro_sgh* h, const fierro_mesh* mesh, const fierro_boundary* 
 int build_device(fierro_sgh* h, const fierro_mesh* mesh, const fierro_boundary* bcs, int64_t num_bcs) {
   Scratch sc(build_bytes((size_t)mesh->num_nodes, (size_t)mesh->num_elems));
   return build(h, mesh, bcs, num_bcs, sc);
+}
+
+namespace {
+template <typename T>
+int fetch(std::vector<T>* out, const T* src, size_t n, cudaStream_t st) {
+  out->resize(n);
+  if (n) CUDA_TRY(cudaMemcpyAsync(out->data(), src, sizeof(T) * n, cudaMemcpyDeviceToHost, st));
+  return FIERRO_OK;
+}
+
+int build_one(cudaStream_t st, const ToHost& in, Scratch& sc) {
+  TRY(check_mesh_header(in.mesh));
+  TRY(validate_bcs(in.bcs, in.num_bcs));
+  const size_t nn = (size_t)in.mesh->num_nodes, ne = (size_t)in.mesh->num_elems;
+  struct Handle : fierro_sgh {
+    ~Handle() {
+      cudaStreamSynchronize(stream);  // the copies to the host under way
+      for (void* p : allocations) cudaFree(p);
+    }
+  } h;
+  h.stream = st;
+  h.nn = (int64_t)nn;
+  h.ne = (int64_t)ne;
+  TRY(sc.alloc(&h.d_nie, ne * 8));
+  TRY(sc.alloc(&h.d_cin_start, nn + 1));
+  TRY(sc.alloc(&h.d_cin, ne * 8));
+  TRY(sc.alloc(&h.d_eie_start, ne + 1));
+  TRY(sc.alloc(&h.d_bc, nn));
+  TRY(sc.alloc(&h.d_node_ext2int, nn));
+  TRY(sc.alloc(&h.d_elem_ext2int, ne));
+  TRY(sc.alloc(&h.d_node_int2ext, nn));
+  TRY(sc.alloc(&h.d_elem_int2ext, ne));
+  TRY(build(&h, in.mesh, in.bcs, in.num_bcs, sc));
+  HostTopo* out = in.out;
+  *out = std::move(h.topo);
+  TRY(fetch(&out->nie, h.d_nie, ne * 8, st));
+  TRY(fetch(&out->cin_start, h.d_cin_start, nn + 1, st));
+  TRY(fetch(&out->cin, h.d_cin, ne * 8, st));
+  TRY(fetch(&out->eie_start, h.d_eie_start, ne + 1, st));
+  TRY(fetch(&out->eie, h.d_eie, (size_t)h.nnz_eie, st));
+  TRY(fetch(&out->bc_mask, h.d_bc, nn, st));
+  out->node_ext2int.resize(nn);
+  out->elem_ext2int.resize(ne);
+  for (size_t i = 0; i < nn; ++i) out->node_ext2int[(size_t)out->node_int2ext[i]] = (int64_t)i;
+  for (size_t i = 0; i < ne; ++i) out->elem_ext2int[(size_t)out->elem_int2ext[i]] = (int64_t)i;
+  CUDA_TRY(cudaStreamSynchronize(st));
+  return FIERRO_OK;
+}
+}  // namespace
+
+void build_to_host(const std::vector<ToHost>& list, std::vector<char>* built) {
+  built->assign(list.size(), 0);
+  size_t most = 0;
+  for (const ToHost& in : list)
+    if (check_mesh_header(in.mesh) == FIERRO_OK)
+      most = std::max(most, build_bytes((size_t)in.mesh->num_nodes, (size_t)in.mesh->num_elems) +
+                                80 * (size_t)in.mesh->num_elems + 16 * (size_t)in.mesh->num_nodes);
+  cudaStream_t st = nullptr;
+  if (most == 0 || cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return;
+  {
+    Scratch sc(most);
+    for (size_t k = 0; k < list.size(); ++k) {
+      try {
+        (*built)[k] = build_one(st, list[k], sc) == FIERRO_OK;
+      } catch (const std::exception&) {  // host memory
+      }
+      sc.reset();
+    }
+  }
+  cudaStreamDestroy(st);
 }
 
 }  // namespace topo
