@@ -586,7 +586,7 @@ int create_impl(fierro_batch* b, const fierro_batch_instance* inst, int64_t n, i
     const HostTopo& t = b->topo[i];
     const int64_t no = b->node_off[i], eo = b->elem_off[i];
     for (int64_t e = 0; e < t.ne * 8; ++e) nie[(size_t)eo * 8 + e] = (int32_t)(t.nie[e] + no);
-    for (int64_t e = eo; e < b->elem_off[i + 1]; ++e) inst_e[e] = (e - eo < t.ne) ? (int32_t)i : (int32_t)(-i - 1);
+    for (int64_t e = eo; e < b->elem_off[i + 1]; ++e) inst_e[e] = (e - eo < t.ne) ? (int32_t)i : padding_code((int)i);
     for (int64_t k = 0; k < t.nn; ++k) {
       cin_start[no + k + 1] = (int32_t)(cin_off[i] + t.cin_start[k + 1]);
       inst_n[no + k] = (int32_t)i;

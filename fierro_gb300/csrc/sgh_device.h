@@ -42,6 +42,15 @@ struct Ctrl {
 #define FIERRO_STATUS_BAD_STATE 2u   // non-finite energy, pressure or velocity
 #define FIERRO_STATUS_DT_FLOOR 4u    // a CFL step fell below dt_min and dt was raised to it (warning)
 
+// A batch's element -> instance codes: instance i's elements hold i, the padding
+// after them -i - 1.  A tile lies inside one instance, but its first element may be
+// padding (blocks smaller than the padding's unit leave tiles of nothing else).
+__host__ __device__ inline int padding_code(int instance) { return -instance - 1; }
+__host__ __device__ inline int tile_instance(const int* inst, int tile, int block) {
+  const int code = inst[(long long)tile * block];
+  return code < 0 ? padding_code(code) : code;
+}
+
 struct LoopParams {
   double time_final, dt_max, dt_min, dt_cfl, graphics_dt_ival, fuzz, small;
   long long graphics_cyc_ival;
@@ -60,7 +69,7 @@ struct ForceArgs {
   const double* div;  // divergence of this stage (written by the previous element pass)
   double* force;
   const Ctrl* ctrl;   // plain: the solver's control block; batch: one per instance
-  const int* inst;    // batch only: instance of each element (negative = padding)
+  const int* inst;    // batch only: instance of each element (padding: padding_code)
   double fuzz, small;
   // adjoint replay only (force_tape launcher): the viscosity intermediates of
   // each element, rows of kForceTapeRows x ne, and the limiter's neighbour
@@ -140,7 +149,7 @@ struct ElemArgs {
   double* bmat;
   long long* cfl_part;  // per-block minimum of the element time steps (order keys)
   Ctrl* ctrl;
-  const int* inst;            // batch only: instance of each element (negative = padding)
+  const int* inst;            // batch only: instance of each element (padding: padding_code)
   const double* dt_cfl_tab;   // batch only: CFL number per instance
   double rk_alpha, dt_cfl, fuzz;
   // hyper strength materials (set when the handle has one): stress rows [9][ne]

@@ -550,12 +550,13 @@ __global__ void __launch_bounds__(kNodeBlock) k_node(const NodeArgs a) {
 // updated state.
 // A tile is one block's worth of elements, with one CFL partial.  In a batch
 // every tile lies inside one instance (instances' element ranges are padded to
-// whole default blocks, padding marked by a negative instance id, and the block
-// divides the default), so the activity test and the CFL partial are per tile.
+// whole default blocks, padding marked by a negative code, and the block divides
+// the default), so the activity test and the CFL partial are per tile; a tile of
+// padding alone leaves the largest key as its partial.
 template <int KIND, bool BATCH, bool STRENGTH, bool COH = false>
 __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
   const int e = tile * blockDim.x + threadIdx.x;
-  const int ib = BATCH ? a.inst[tile * blockDim.x] : 0;
+  const int ib = BATCH ? tile_instance(a.inst, tile, blockDim.x) : 0;
   Ctrl* ctrl = a.ctrl + ib;
   if (KIND != 2 && !ctrl->active) return;
   const bool live = e < a.ne && (!BATCH || a.inst[e] >= 0);
