@@ -268,6 +268,25 @@ void release_run_graphs(fierro_sgh* h) {
   h->graph_cycles = 0;
 }
 
+// Captures what `enqueue` puts on the handle's stream as a graph.  It is captured on
+// a stream of the handle's own: work that the caller's other threads, or other handles,
+// put on a shared stream meanwhile must run, not be recorded.
+template <typename F>
+int capture_graph(fierro_sgh* h, F&& enqueue, cudaGraphExec_t* exec) {
+  const cudaStream_t stream = h->stream;
+  CUDA_TRY(cudaStreamBeginCapture(h->capture, cudaStreamCaptureModeThreadLocal));
+  h->stream = h->capture;
+  const int rc = enqueue();
+  h->stream = stream;
+  cudaGraph_t g = nullptr;
+  cudaError_t err = cudaStreamEndCapture(h->capture, &g);
+  if (err == cudaSuccess && rc == FIERRO_OK) err = cudaGraphInstantiate(exec, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (rc) return rc;
+  if (err != cudaSuccess) return set_error(FIERRO_ECUDA, "cycle graph: %s", cudaGetErrorString(err));
+  return FIERRO_OK;
+}
+
 // Launching a graph leaves the device idle for ~3 us after the one before it: a
 // run on a small mesh launches four cycles at a time (8^3 41.5 -> 38.3 us a cycle,
 // 16^3 45.5 -> 43.0, 32^3 127.9 -> 124.6; eight at a time 38.1, 42.7, 124.2).  The larger
@@ -283,18 +302,13 @@ bool run_graphs_ready(fierro_sgh* h) {
   if (h->run_graph[0]) return true;
   if (h->graph_cycles < kRunAfter) return false;
   for (int c = 0; c < 2; ++c) {
-    cudaGraph_t g = nullptr;
-    cudaError_t err = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
-    if (err == cudaSuccess) {
-      bool ok = true;
-      for (int k = 0; k < kRunCycles && ok; ++k) ok = enqueue_cycle(h, (c + k) & 1) == FIERRO_OK;
-      err = cudaStreamEndCapture(h->stream, &g);
-      if (err == cudaSuccess && !ok) err = cudaErrorUnknown;
-    }
-    if (err == cudaSuccess) err = cudaGraphInstantiate(&h->run_graph[c], g, 0);
-    if (g) cudaGraphDestroy(g);
-    if (err != cudaSuccess) {
+    const int rc = capture_graph(h, [&]() -> int {
+      for (int k = 0; k < kRunCycles; ++k) TRY(enqueue_cycle(h, (c + k) & 1));
+      return FIERRO_OK;
+    }, &h->run_graph[c]);
+    if (rc) {
       cudaGetLastError();
+      clear_error();
       h->run_graph[c] = nullptr;
       release_run_graphs(h);  // tries again after kRunAfter more cycles
       return false;
@@ -306,6 +320,7 @@ bool run_graphs_ready(fierro_sgh* h) {
 int build_graphs(fierro_sgh* h) {
   release_run_graphs(h);
   if (!h->side) CUDA_TRY(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+  if (!h->capture) CUDA_TRY(cudaStreamCreateWithFlags(&h->capture, cudaStreamNonBlocking));
   for (cudaEvent_t& e : h->side_ev)
     if (!e) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (int c = 0; c < 2; ++c) {
@@ -313,17 +328,7 @@ int build_graphs(fierro_sgh* h) {
       cudaGraphExecDestroy(h->graph[c]);
       h->graph[c] = nullptr;
     }
-    cudaGraph_t g = nullptr;
-    CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_cycle(h, c);
-    CUDA_TRY(cudaStreamEndCapture(h->stream, &g));
-    if (rc) {
-      cudaGraphDestroy(g);
-      return rc;
-    }
-    cudaError_t err = cudaGraphInstantiate(&h->graph[c], g, 0);
-    cudaGraphDestroy(g);
-    if (err != cudaSuccess) return set_error(FIERRO_ECUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(err));
+    TRY(capture_graph(h, [&] { return enqueue_cycle(h, c); }, &h->graph[c]));
   }
   return FIERRO_OK;
 }
@@ -359,6 +364,7 @@ extern "C" int fierro_sgh_destroy(fierro_sgh* h) {
     if (h->graph[c]) cudaGraphExecDestroy(h->graph[c]);
   release_run_graphs(h);
   if (h->side) cudaStreamDestroy(h->side);
+  if (h->capture) cudaStreamDestroy(h->capture);
   for (cudaEvent_t e : h->side_ev)
     if (e) cudaEventDestroy(e);
   for (void* p : h->allocations) cudaFree(p);

@@ -50,6 +50,7 @@ struct fierro_sgh {
   // beside the element launch
   cudaStream_t side = nullptr;
   cudaEvent_t side_ev[2] = {};
+  cudaStream_t capture = nullptr;  // graphs are captured here, never on the caller's stream
   std::vector<void*> allocations;
   size_t dev_bytes = 0;
   // mesh
