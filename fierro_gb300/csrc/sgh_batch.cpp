@@ -981,10 +981,11 @@ extern "C" int fierro_batch_autotune(fierro_batch* b, int64_t cycles, fierro_bat
   b->tune_ms.clear();
   int rc = copy_arrays(b, save, arrs, true);
   const fierro_batch_shape start = b->shape, start_launch = b->launch;
-  fierro_batch_shape best = b->shape;
+  fierro_batch_shape best = start_launch;
   double best_ms = 0.0;
   bool have = false;
-  // coordinate descent: force block, node block, element block, persistent grid
+  // coordinate descent from the shape that is launched now, which is timed first: force
+  // block, node block, element block, persistent grid
   auto trial = [&](fierro_batch_shape sh) -> int {
     for (size_t i = 0; i < b->tune_shapes.size(); ++i) {
       const fierro_batch_shape& o = b->tune_shapes[i];
@@ -1007,6 +1008,7 @@ extern "C" int fierro_batch_autotune(fierro_batch* b, int64_t cycles, fierro_bat
   };
   const int force_blocks[] = {128, 64, 32}, node_blocks[] = {256, 128, 512, 64}, elem_blocks[] = {128, 64, 32};
   const int persist[] = {0, 1, 2};
+  if (!rc) rc = trial(start_launch);
   for (int fb : force_blocks) {
     if (rc) break;
     fierro_batch_shape sh = best;

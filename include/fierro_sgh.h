@@ -288,13 +288,16 @@ typedef struct {
   int fused_stage;
 } fierro_batch_shape;
 
-/* Set or read the shape; set only before the first fierro_batch_run. */
+/* Set or read the shape; set only before the first fierro_batch_run.  A shape that
+ * was set or tuned is launched as it is; until then fierro_batch_get_shape gives the
+ * default above, also where smaller blocks are launched. */
 int fierro_batch_set_shape(fierro_batch* b, const fierro_batch_shape* shape);
 int fierro_batch_get_shape(const fierro_batch* b, fierro_batch_shape* shape);
 /* Autotuner: after every instance has its state and before the first run, time
- * `cycles` cycles (after one warm-up cycle) of the captured cycle graphs for each
- * candidate shape of a coordinate descent over the force block {128, 64, 32}, the
- * node block {256, 128, 512, 64}, the element block {128, 64, 32}, the
+ * `cycles` cycles (after one warm-up cycle) of the captured cycle graphs for what
+ * the batch launches now and for each candidate shape of a coordinate descent from
+ * there over the force block {128, 64, 32}, the node block {256, 128, 512, 64},
+ * the element block {128, 64, 32}, the
  * persistent grid {0, 1, 2} and the fused stage at the chosen element block,
  * each from the uploaded state (saved and restored on the device; needs one
  * extra copy of the batch's state), and keep the fastest.  The state afterwards
