@@ -387,10 +387,7 @@ static int create_impl(fierro_sgh* h, const fierro_mesh* mesh, const fierro_mate
   if (num_materials < 1 || !materials) return set_error(FIERRO_EINVAL, "need at least one material");
   TRY(check_mesh_header(mesh));
   h->dims = mesh_dims(mesh);
-  {
-    const char* env = std::getenv("FIERRO_FAIL_ALLOC_AFTER");
-    h->alloc_limit = env ? std::strtoll(env, nullptr, 10) : -1;
-  }
+  h->alloc_limit = alloc_limit();
   for (int64_t m = 0; m < num_materials; ++m) {
     if (materials[m].eos_model != 0) return set_error(FIERRO_ENOTSUP, "material %lld: only the ideal-gas EOS", (long long)m);
     if (materials[m].strength_type < 0 || materials[m].strength_type > 2)

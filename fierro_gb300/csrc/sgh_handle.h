@@ -5,6 +5,8 @@
 #define FIERRO_SGH_HANDLE_H
 
 #include <algorithm>
+#include <cstdint>
+#include <cstdlib>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -122,7 +124,8 @@ struct fierro_sgh {
   int* d_axis_nin = nullptr;
   int naxis = 0;
   // host-side fault injection: FIERRO_FAIL_ALLOC_AFTER=n makes the handle's
-  // device allocations after the first n fail as if the device were full
+  // device allocations after the first n fail as if the device were full (they ask
+  // for more than any device has); so too the one a batch's topology on the GPU makes
   int64_t alloc_limit = -1;
   int64_t alloc_count = 0;
 };
@@ -135,17 +138,26 @@ template <typename T>
 int dalloc(fierro_sgh* h, T** p, size_t count) {
   void* q = nullptr;
   size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-  if (h->alloc_limit >= 0 && h->alloc_count >= h->alloc_limit)
-    return set_error(FIERRO_ENOMEM, "cudaMalloc(%zu bytes): injected failure after %lld allocations", bytes,
-                     (long long)h->alloc_count);
-  h->alloc_count++;
-  cudaError_t err = cudaMalloc(&q, bytes);
-  if (err != cudaSuccess)
+  const bool inject = h->alloc_limit >= 0 && h->alloc_count >= h->alloc_limit;
+  cudaError_t err = cudaMalloc(&q, inject ? SIZE_MAX / 2 : bytes);
+  if (err != cudaSuccess) {
+    cudaGetLastError();  // reported here; not to be met again by the next call's check
+    if (inject)
+      return set_error(FIERRO_ENOMEM, "cudaMalloc(%zu bytes): injected failure after %lld allocations", bytes,
+                       (long long)h->alloc_count);
     return set_error(FIERRO_ENOMEM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(err));
+  }
+  h->alloc_count++;
   h->allocations.push_back(q);
   h->dev_bytes += bytes;
   *p = static_cast<T*>(q);
   return FIERRO_OK;
+}
+
+// The allocations FIERRO_FAIL_ALLOC_AFTER lets succeed; -1 without it.
+inline int64_t alloc_limit() {
+  const char* env = std::getenv("FIERRO_FAIL_ALLOC_AFTER");
+  return env ? std::strtoll(env, nullptr, 10) : -1;
 }
 
 int upload_raw(fierro_sgh* h, void* dst, const void* src, size_t bytes);

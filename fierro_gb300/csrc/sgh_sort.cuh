@@ -182,8 +182,10 @@ struct Scratch {
       return FIERRO_OK;
     }
     void* q = nullptr;
-    if (cudaMalloc(&q, bytes) != cudaSuccess)
+    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+      cudaGetLastError();
       return set_error(FIERRO_ENOMEM, "topology: cudaMalloc(%zu bytes) failed", bytes);
+    }
     p.push_back(q);
     *out = static_cast<T*>(q);
     return FIERRO_OK;

@@ -462,6 +462,7 @@ int build_one(cudaStream_t st, const ToHost& in, Scratch& sc) {
     }
   } h;
   h.stream = st;
+  h.alloc_limit = hd::alloc_limit();
   h.nn = (int64_t)nn;
   h.ne = (int64_t)ne;
   TRY(sc.alloc(&h.d_nie, ne * 8));
@@ -499,13 +500,22 @@ void build_to_host(const std::vector<ToHost>& list, std::vector<char>* built) {
       most = std::max(most, build_bytes((size_t)in.mesh->num_nodes, (size_t)in.mesh->num_elems) +
                                 80 * (size_t)in.mesh->num_elems + 16 * (size_t)in.mesh->num_nodes);
   cudaStream_t st = nullptr;
-  if (most == 0 || cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return;
+  // What is turned down goes to the host builder, and leaves no error behind.
+  if (most == 0 || cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {
+    cudaGetLastError();
+    clear_error();
+    return;
+  }
   {
     Scratch sc(most);
     for (size_t k = 0; k < list.size(); ++k) {
       try {
         (*built)[k] = build_one(st, list[k], sc) == FIERRO_OK;
       } catch (const std::exception&) {  // host memory
+      }
+      if (!(*built)[k]) {
+        cudaGetLastError();
+        clear_error();
       }
       sc.reset();
     }
