@@ -81,6 +81,13 @@ __device__ __forceinline__ double at_most_1(double v) {
   return b > 0x3FF0000000000000LL ? 1.0 : v;  // NaN too, as fmin has it
 }
 
+// A sum that the reference begins from 0.0 and that here begins with its first term
+// (one FP64 operation less): the two differ where all terms are negative zeros, whose
+// sum from 0.0 is +0.0.
+__device__ __forceinline__ double from_zero(double s) {
+  return (__double_as_longlong(s) & kAbsMask) == 0 ? 0.0 : s;
+}
+
 // Single-precision image of a positive double within float range (truncated).
 __device__ __forceinline__ float f32_image(double d) {
   const long long b = __double_as_longlong(d);

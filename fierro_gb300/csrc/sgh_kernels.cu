@@ -4,7 +4,9 @@
 //   FIERRO_FMA=0 with --fmad=false -> fierro::exact_impl: every floating-point
 //       operation is the reference's operation on the reference's operands in
 //       the reference's order (Explicit-Lagrange-Kokkos/SGH_solver), with IEEE
-//       division and square root, so results match its uncontracted evaluation;
+//       division and square root, so results match its uncontracted evaluation
+//       (a corner normal of zero, and through it a corner force of zero, may have
+//       the other sign; sums from 0.0 have the reference's: from_zero);
 //   FIERRO_FMA=1 with --fmad=true  -> fierro::fma_impl: the same schedule, the
 //       compiler free to fuse multiply-adds, the per-node division by mass and
 //       the Riemann velocity's three divisions done through one reciprocal
@@ -186,7 +188,7 @@ __device__ __forceinline__ double divergence(double Sx, double Sy, double Sz, do
   double div = Sx * inverse_vol;
   div = mul_add(div, Sy, inverse_vol);
   div = mul_add(div, Sz, inverse_vol);
-  return div;
+  return from_zero(div);
 }
 // Order key of the element CFL step dt_cfl * min distance / (c + fuzz)
 // (time_integration.cpp:124-131); a NaN bounds nothing.
@@ -300,6 +302,9 @@ __device__ __forceinline__ void force_elem(const ForceArgs& a, const int e) {
     s3 = l ? s3 + mu_term : mu_term;
     mu[l] = mu_term;
   }
+  s0 = from_zero(s0);
+  s1 = from_zero(s1);
+  s2 = from_zero(s2);
   double vstar0 = 0.0, vstar1 = 0.0, vstar2 = 0.0;
   if (BR == 2 ? (br & FIERRO_BR_VSTAR) != 0 : s3 > a.fuzz) {
 #if FIERRO_FMA
@@ -496,6 +501,9 @@ __device__ __forceinline__ void node_update(const NodeArgs& a, const int n) {
         f2 = k || base > c0 ? f2 + g[k][2] : g[k][2];
       }
   }
+  f0 = from_zero(f0);
+  f1 = from_zero(f1);
+  f2 = from_zero(f2);
   const double adt = a.rk_alpha * ctrl->dt;
   const double u0 = a.u0[n], v0 = a.v0[n], w0 = a.w0[n];
 #if FIERRO_FMA
@@ -589,7 +597,7 @@ __device__ __forceinline__ void elem_tile(const ElemArgs& a, const int tile) {
         power = mul_add(power, ld_pl<COH>(a.force + (size_t)(l * 3 + 2) * ne + e), ld_pl<COH>(a.hz + nid[l]));
       }
       const double adt = a.rk_alpha * ctrl->dt;
-      sie1 = a.sie0[e] - FX_MUL(mode_div(adt, a.mass[e]), power);  // not fused: sie1 may cancel sie0
+      sie1 = a.sie0[e] - FX_MUL(mode_div(adt, a.mass[e]), from_zero(power));  // not fused: sie1 may cancel sie0
       a.sie1[e] = sie1;
     };
     // The pass with the CFL step reads what the energy needs after the geometry, the other

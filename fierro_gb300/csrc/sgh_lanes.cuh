@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_force_lanes(const ForceArgs a) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) s = s + sv[r][k];
 #endif
+  s = from_zero(s);  // a fused sum's first product may round to -0.0
   const double s3 = from_lane(s, 3);
   // the element's quotients in different lanes of the same instructions: the
   // Riemann velocity's (0-2), the limiter's (3), the Mach switch's (4 and on)
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_elem_lanes(const ElemArgs a) {
   }
   const double Sx = from_lane(acc, 0), Sy = from_lane(acc, 1), Sz = from_lane(acc, 2);
   const double vol_geo = FX_MUL(from_lane(acc, 3), twelth);
-  const double power = from_lane(acc, 4);
+  const double power = from_zero(from_lane(acc, 4));
   const double vol = (KIND == 2) ? a.vol[e] : vol_geo;
   // three quotients at once: 1 / vol, dt / mass, mass / vol
   const double adt = KIND != 2 ? a.rk_alpha * a.ctrl->dt : 0.0;

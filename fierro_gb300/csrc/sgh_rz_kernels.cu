@@ -3,7 +3,8 @@
 //
 // Compiled twice, like sgh_kernels.cu: FIERRO_FMA=0 with --fmad=false (every
 // operation the reference's, in its order; square roots and shared-divisor
-// quotients by the correctly rounded Newton forms of sgh_common.cuh) and
+// quotients by the correctly rounded Newton forms of sgh_common.cuh; the sign of a
+// zero normal apart) and
 // FIERRO_FMA=1 (contraction and reciprocal reuse allowed; the Newton square
 // roots, quotients and reciprocals).
 //
@@ -212,6 +213,14 @@ __device__ __forceinline__ double rz_limiter_min(const RzForceArgs& a, double di
   }
   return r_min;
 }
+// A corner force without the terms that are zeros (:718-755): the shear stress (+0.0)
+// times the other component of the inward normal and, off the axis, the hoop term.
+// With them a force of -0.0 stays one on the axis alone, beside a negative normal.
+__device__ __forceinline__ double rz_zero_terms(double f, double other_normal, double radius) {
+  if ((__double_as_longlong(f) & kAbsMask) != 0) return f;
+  const bool off_axis = __double_as_longlong(radius) > __double_as_longlong(1e-14);
+  return off_axis || __double_as_longlong(other_normal) >= 0 ? 0.0 : f;
+}
 // Mach-number detector with the characteristic length sqrt(area) (:692-700)
 __device__ __forceinline__ double rz_mach_switch(double area, double div, double sspd, double fuzz) {
   return at_most_1(newton_div(20.0 * (mode_sqrt(area) * fabs(div)), sspd + fuzz));
@@ -288,6 +297,8 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     s3 = l ? s3 + mu_term : mu_term;
     mu[l] = mu_term;
   }
+  s0 = from_zero(s0);
+  s1 = from_zero(s1);
   double vstar0 = 0.0, vstar1 = 0.0;
   if (s3 > a.fuzz) {
 #if FIERRO_FMA
@@ -319,13 +330,9 @@ __global__ void __launch_bounds__(kRzBlock) k_force_rz(const RzForceArgs a) {
     double f[2];
     if (hoop_zero) {
       // finite normals and no shear: the products with tau's zeros are zeros, and so
-      // are the hoop terms; adding those would only turn a -0.0 force into +0.0,
-      // which is done on the bits
-      f[0] = mul_mul(a0, t[0], pm, vs[0] - vl[0]);
-      f[1] = mul_mul(a1, t[4], pm, vs[1] - vl[1]);
-#pragma unroll
-      for (int d = 0; d < 2; ++d)
-        if ((__double_as_longlong(f[d]) & kAbsMask) == 0) f[d] = 0.0;
+      // are the hoop terms; adding those changes no more than the sign of a zero
+      f[0] = rz_zero_terms(mul_mul(a0, t[0], pm, vs[0] - vl[0]), a1, y[l]);
+      f[1] = rz_zero_terms(mul_mul(a1, t[4], pm, vs[1] - vl[1]), a0, y[l]);
     } else {
 #pragma unroll
       for (int d = 0; d < 2; ++d) f[d] = mul_add(mul_mul(a0, t[d], a1, t[3 + d]), pm, vs[d] - vl[d]);
@@ -396,6 +403,8 @@ __global__ void __launch_bounds__(kRzNodeBlock) k_node_rz(const RzNodeArgs a) {
         f1 = k || base > c0 ? f1 + g[k][1] : g[k][1];
       }
   }
+  f0 = from_zero(f0);
+  f1 = from_zero(f1);
   const double adt = a.rk_alpha * a.ctrl->dt;
   const double m = a.node_mass[n];
   const double u0 = a.u0[n], v0 = a.v0[n];
@@ -477,7 +486,7 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
         power = mul_add(power, a.force[(size_t)(l * 2 + 1) * ne + e] * r, a.hy[nid[l]]);
       }
       const double adt = a.rk_alpha * ctrl->dt;
-      sie1 = mul_add(a.sie0[e], -newton_div(adt, a.mass[e]), power);
+      sie1 = mul_add(a.sie0[e], -newton_div(adt, a.mass[e]), from_zero(power));
       a.sie1[e] = sie1;
     }
     const RzDiffs df = rz_diffs(x, y);
@@ -493,7 +502,7 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     const double su = mul_add(mul_add(mul_mul(u[0], B[0][0], u[1], B[1][0]), u[2], B[2][0]), u[3], B[3][0]);
     const double sv = mul_add(mul_add(mul_mul(v[0], B[0][1], v[1], B[1][1]), v[2], B[2][1]), v[3], B[3][1]);
     double div = su * inverse_area;
-    div = div + mul_add(newton_div(elem_vel_r, mean_radius), sv, inverse_area);
+    div = from_zero(div + mul_add(newton_div(elem_vel_r, mean_radius), sv, inverse_area));
     a.div[e] = div;
     double sspd;
     if (KIND != 2) {

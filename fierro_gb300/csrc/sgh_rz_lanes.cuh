@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(kRzLaneBlock) k_force_rz_lanes(const RzForceAr
     s = s + (l == 0 ? p0 : l == 1 ? p1 : p2);
   }
 #endif
+  s = from_zero(s);
   const double s3 = quad_lane(s, 2);
   double vstar = 0.0;
   if (s3 > a.fuzz) {
@@ -117,10 +118,8 @@ __global__ void __launch_bounds__(kRzLaneBlock) k_force_rz_lanes(const RzForceAr
   const double pm = phi * mu, tau = 0.0 - pres;
   double f0, f1;
   if (hoop_zero) {
-    f0 = mul_mul(-g.Bx, tau, pm, vstar0 - ul);
-    f1 = mul_mul(-g.By, tau, pm, vstar1 - vl);
-    if ((__double_as_longlong(f0) & kAbsMask) == 0) f0 = 0.0;
-    if ((__double_as_longlong(f1) & kAbsMask) == 0) f1 = 0.0;
+    f0 = rz_zero_terms(mul_mul(-g.Bx, tau, pm, vstar0 - ul), -g.By, yl);
+    f1 = rz_zero_terms(mul_mul(-g.By, tau, pm, vstar1 - vl), -g.Bx, yl);
   } else {
     double ca[4];
     rz_corner_areas(x, y, ca);
@@ -211,12 +210,12 @@ __global__ void __launch_bounds__(kRzLaneBlock) k_elem_rz_lanes(const RzElemArgs
   __syncwarp();
   const double inverse_area = quad_lane(qt, 0), mean_radius = quad_lane(qt, 1);
   double div = su * inverse_area;
-  div = div + mul_add(newton_div(vr, mean_radius), sv, inverse_area);
+  div = from_zero(div + mul_add(newton_div(vr, mean_radius), sv, inverse_area));
   __syncwarp();
   double sspd;
   const bool writer = live && l == 0;
   if (KIND != 2) {
-    const double sie1 = mul_add(sie0, -quad_lane(qt, 2), pw);
+    const double sie1 = mul_add(sie0, -quad_lane(qt, 2), from_zero(pw));
     const double den = quad_lane(qt, 3);
     const double pres = (gamma - 1.0) * sie1 * den;
     sspd = mode_sqrt(gamma * (gamma - 1.0) * sie1);
