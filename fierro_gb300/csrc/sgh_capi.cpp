@@ -485,9 +485,10 @@ static int create_impl(fierro_sgh* h, const fierro_mesh* mesh, const fierro_mate
   h->blk_elem = small_mesh_block(ne, kElemBlock);
   h->blk_force = small_mesh_block(ne, kForceBlock);
   h->blk_node = small_mesh_block(nn, kNodeBlock);
-  h->lanes_force = (long long)ne <= kLanesForce;
-  h->lanes_node = (long long)nn <= kLanesNode;
-  h->lanes_elem = (long long)ne <= kLanesElem && !h->has_hyper;
+  const bool lanes = lanes_enabled();
+  h->lanes_force = lanes && (long long)ne <= kLanesForce;
+  h->lanes_node = lanes && (long long)nn <= kLanesNode;
+  h->lanes_elem = lanes && (long long)ne <= kLanesElem && !h->has_hyper;
   h->cfl_tile = h->lanes_elem ? kLaneTile : h->blk_elem;
   h->ckpt_tile = checkpoint_tile((long long)ne);
   h->ncfl = (int)((ne + h->cfl_tile - 1) / h->cfl_tile);

@@ -160,6 +160,12 @@ inline int64_t alloc_limit() {
   return env ? std::strtoll(env, nullptr, 10) : -1;
 }
 
+// FIERRO_LANES=0 keeps a handle on the one-thread-per-element passes whatever its size.
+inline bool lanes_enabled() {
+  const char* env = std::getenv("FIERRO_LANES");
+  return !(env && env[0] == '0');
+}
+
 int upload_raw(fierro_sgh* h, void* dst, const void* src, size_t bytes);
 // Permuted upload through the pinned double buffer: dst[i] = src[map[i]*stride + off].
 int upload_gather(fierro_sgh* h, double* dst, const double* src, const std::vector<int64_t>& map,

@@ -351,8 +351,9 @@ int create(fierro_sgh* h, const fierro_mesh* mesh, const fierro_material* materi
   TRY(dalloc(h, &h->d_axis, t.axis_nodes.size()));
   TRY(dalloc(h, &h->d_axis_nin_start, t.axis_nin_start.size()));
   TRY(dalloc(h, &h->d_axis_nin, t.axis_nin.size()));
-  h->lanes_force = (long long)ne <= kRzLanesForce && !h->strength;
-  h->lanes_elem = (long long)ne <= kRzLanesElem;
+  const bool lanes = lanes_enabled();
+  h->lanes_force = lanes && (long long)ne <= kRzLanesForce && !h->strength;
+  h->lanes_elem = lanes && (long long)ne <= kRzLanesElem;
   h->blk_elem = small_mesh_block((long long)ne, kElemBlock);
   h->cfl_tile = h->lanes_elem ? kRzLaneTile : h->blk_elem;
   h->ncfl = (int)((ne + h->cfl_tile - 1) / h->cfl_tile);

@@ -501,8 +501,8 @@ __global__ void __launch_bounds__(kRzBlock) k_elem_rz(const RzElemArgs a) {
     const double elem_vel_r = 0.25 * (v[0] + v[1] + v[2] + v[3]);
     const double su = mul_add(mul_add(mul_mul(u[0], B[0][0], u[1], B[1][0]), u[2], B[2][0]), u[3], B[3][0]);
     const double sv = mul_add(mul_add(mul_mul(v[0], B[0][1], v[1], B[1][1]), v[2], B[2][1]), v[3], B[3][1]);
-    double div = su * inverse_area;
-    div = from_zero(div + mul_add(newton_div(elem_vel_r, mean_radius), sv, inverse_area));
+    const double div =
+        from_zero(mul_add(mul_add(newton_div(elem_vel_r, mean_radius), sv, inverse_area), su, inverse_area));
     a.div[e] = div;
     double sspd;
     if (KIND != 2) {

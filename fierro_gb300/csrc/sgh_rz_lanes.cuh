@@ -209,8 +209,7 @@ __global__ void __launch_bounds__(kRzLaneBlock) k_elem_rz_lanes(const RzElemArgs
   const double qt = newton_div(num, dvs);
   __syncwarp();
   const double inverse_area = quad_lane(qt, 0), mean_radius = quad_lane(qt, 1);
-  double div = su * inverse_area;
-  div = from_zero(div + mul_add(newton_div(vr, mean_radius), sv, inverse_area));
+  const double div = from_zero(mul_add(mul_add(newton_div(vr, mean_radius), sv, inverse_area), su, inverse_area));
   __syncwarp();
   double sspd;
   const bool writer = live && l == 0;
