@@ -18,7 +18,6 @@
 #include <vector>
 
 #include <cuda_runtime.h>
-#include <omp.h>
 
 #include "fierro_sgh.h"
 #include "sgh_device.h"
@@ -477,7 +476,7 @@ int build_topologies(fierro_batch* b, const fierro_batch_instance* inst, int64_t
     std::sort(order.begin(), order.end(), [&](int64_t p, int64_t q) {
       return elems(p) != elems(q) ? elems(p) > elems(q) : p < q;
     });
-    const double threads = std::max(1, omp_get_max_threads());
+    const double threads = std::max(1, max_threads());
     double gpu = 0.0, best = 1e300;
     size_t take = 0;
     for (size_t k = 0; k <= order.size(); ++k) {

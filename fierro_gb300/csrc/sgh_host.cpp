@@ -14,9 +14,6 @@
 
 #include <unistd.h>
 
-#ifdef _OPENMP
-#include <omp.h>
-#endif
 
 #include "fierro_sgh.h"
 #include "sgh_hex.h"
@@ -176,18 +173,10 @@ int boundary_masks(const fierro_mesh* mesh, const fierro_boundary* bcs, int64_t 
   std::vector<int64_t> start, elems;
   node_elem_csr(nn, ne, nie, &start, &elems, nullptr);
   // boundary patches: faces whose four nodes no other element shares (mesh.h:501-515)
-  int nthreads = 1;
-#ifdef _OPENMP
-  nthreads = omp_get_max_threads();
-#endif
-  std::vector<std::vector<int64_t>> found((size_t)nthreads);
+  std::vector<std::vector<int64_t>> found((size_t)max_threads());
 #pragma omp parallel
   {
-    int tid = 0;
-#ifdef _OPENMP
-    tid = omp_get_thread_num();
-#endif
-    auto& out = found[(size_t)tid];
+    auto& out = found[(size_t)thread_number()];
 #pragma omp for schedule(static)
     for (int64_t e = 0; e < ne; ++e) {
       for (int f = 0; f < 6; ++f) {
@@ -339,11 +328,11 @@ int build_topology(const fierro_mesh* mesh, const fierro_boundary* bcs, int64_t 
   // them (at most 256), and copies its lists into place.  The same meetings tell
   // the boundary patches: faces whose four nodes no other element holds.
   t->eie_start.assign((size_t)ne + 1, 0);
-  std::vector<std::vector<int64_t>> patches((size_t)omp_get_max_threads());
+  std::vector<std::vector<int64_t>> patches((size_t)max_threads());
   bool out_of_memory = false;
 #pragma omp parallel
   {
-    const int64_t nth = omp_get_num_threads(), me = omp_get_thread_num();
+    const int64_t nth = region_threads(), me = thread_number();
     const int64_t lo = ne * me / nth, hi = ne * (me + 1) / nth;
     std::vector<int32_t> mine;
     try {

@@ -9,6 +9,10 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#ifdef _OPENMP
+#include <omp.h>
+#endif
+
 #include "fierro_sgh.h"
 
 namespace fierro {
@@ -34,6 +38,30 @@ struct NvtxRange {
 };
 
 // Record an error for fierro_last_error() and return `code`.
+// OpenMP's threads for the next parallel region, a region's threads and the calling
+// one's number; one thread in a build without OpenMP.
+inline int max_threads() {
+#ifdef _OPENMP
+  return omp_get_max_threads();
+#else
+  return 1;
+#endif
+}
+inline int region_threads() {
+#ifdef _OPENMP
+  return omp_get_num_threads();
+#else
+  return 1;
+#endif
+}
+inline int thread_number() {
+#ifdef _OPENMP
+  return omp_get_thread_num();
+#else
+  return 0;
+#endif
+}
+
 int set_error(int code, const char* fmt, ...);
 void clear_error();
 
