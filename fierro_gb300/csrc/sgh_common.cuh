@@ -83,9 +83,13 @@ __device__ __forceinline__ double at_most_1(double v) {
 
 // A sum that the reference begins from 0.0 and that here begins with its first term
 // (one FP64 operation less): the two differ where all terms are negative zeros, whose
-// sum from 0.0 is +0.0.
+// sum from 0.0 is +0.0.  Tested on the halves: the compiler makes an FP64 comparison of
+// the test that all 64 bits but the sign are zero (a cycle at 96^3, exact / FMA: 3,801 /
+// 2,658 us without, 3,801 / 2,659 this way, 3,830 / 2,681 that way; 768^2 FMA 734 / 735 /
+// 751).
 __device__ __forceinline__ double from_zero(double s) {
-  return (__double_as_longlong(s) & kAbsMask) == 0 ? 0.0 : s;
+  const int hi = __double2hiint(s), lo = __double2loint(s);
+  return __hiloint2double((lo | (hi ^ (int)0x80000000)) == 0 ? 0 : hi, lo);
 }
 
 // Single-precision image of a positive double within float range (truncated).
