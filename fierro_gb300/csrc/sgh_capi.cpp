@@ -288,8 +288,8 @@ int capture_graph(fierro_sgh* h, F&& enqueue, cudaGraphExec_t* exec) {
 }
 
 // Launching a graph leaves the device idle for ~3 us after the one before it: a
-// run on a small mesh launches four cycles at a time (8^3 41.5 -> 38.3 us a cycle,
-// 16^3 45.5 -> 43.0, 32^3 127.9 -> 124.6; eight at a time 38.1, 42.7, 124.2).  The larger
+// run on a small mesh launches four cycles at a time (8^3 exact 41.1 -> 37.2 us a cycle,
+// 16^3 FMA 45.2 -> 42.2, 32^3 FMA 124.2 -> 121.2; eight at a time 36.7, 41.9, 120.6).  The larger
 // graphs take ~0.2 ms to make, so they are made when a handle has run kRunAfter
 // cycles; meshes above kRunElems gain under 1 %.
 constexpr int kRunCycles = 4;

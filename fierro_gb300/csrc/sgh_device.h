@@ -264,12 +264,12 @@ inline int checkpoint_tile(long long ne) { return small_mesh_block(ne, kElemBloc
 // it wins until the chip's sub-partitions hold several of its warps each.  Per
 // launch (events, us), one thread per element against eight lanes:
 //                        12^3         18^3         20^3         22^3         23^3
-//   force exact          26.6 / 12.3  26.8 / 16.5  26.7 / 20.4  26.7 / 24.5  26.7 / 28.4
-//   force FMA            20.6 / 10.3               20.7 / 16.3  21.2 / 18.4  20.6 / 20.4
-//   elem exact, CFL step 28.8 / 13.0  28.9 / 20.4  29.9 / 24.7  28.9 / 30.7  29.1 / 36.8
-//   elem FMA, CFL step   23.7 / 12.5               24.6 / 20.5  24.6 / 24.6  24.5 / 28.7
-// and for the nodes, one thread per node against three: 12^3 10.3 / 8.3, 24^3 10.4 /
-// 9.0, 32^3 12.3 / 12.3 (exact).
+//   force exact          24.5 / 12.0  26.5 / 16.4  26.4 / 20.4  26.2 / 22.9  25.8 / 26.7
+//   force FMA            18.5 / 10.3  18.9 / 12.4  19.0 / 16.0  18.9 / 18.4  20.2 / 20.5
+//   elem exact, CFL step 30.7 / 14.3  30.8 / 20.7  30.8 / 26.7  30.9 / 33.0  30.9 / 40.9
+//   elem FMA, CFL step   26.6 / 12.2  26.6 / 16.6  26.6 / 21.9  26.6 / 26.7  26.7 / 30.8
+// and for the nodes, one thread per node against three: 12^3 10.3 / 8.2, 24^3 10.2 /
+// 8.2, 32^3 12.3 / 12.3 (exact).
 constexpr long long kLanesForce = 11500, kLanesElem = 10000, kLanesNode = 30000;
 constexpr int kLaneTile = 4;  // elements per warp of a lane pass
 

@@ -6,11 +6,11 @@
 // Bound: a warp issues one FP64 instruction every ~65 clocks (GB300 has half an
 // FP64 lane per clock and sub-partition, whatever the number of active lanes), so
 // with at most one warp per sub-partition (608) a pass takes as long as one
-// thread's chain: 465 instructions for an element's exact force, 15 us, however
+// thread's chain: 458 instructions for an element's exact force, 15 us, however
 // few elements there are.  Eight lanes cut the chain to the ~95 instructions one
 // corner and the ordered sums take, at twice the total work, which such a mesh
-// does not fill the chip with: a 12^3 cycle 106 -> 50 us exact, 84 -> 43 us FMA,
-// 8^3 105 -> 48 us.  Sums whose order is part of the result run in one
+// does not fill the chip with: a 12^3 cycle 102 -> 40.6 us exact, 78 -> 34.3 us FMA,
+// 8^3 101 -> 37.3 and 78 -> 33.1 us.  Sums whose order is part of the result run in one
 // lane over the corners' products in shared memory (different lanes summing
 // different quantities in the same instructions); everything else is per corner.
 #pragma once

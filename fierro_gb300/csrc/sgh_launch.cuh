@@ -10,7 +10,8 @@
 // loads, never through the read-only path, whose data may not change while a
 // kernel is resident.
 //
-// A cycle at 8^3 47.7 -> 44.0 us, 12^3 49.7 -> 48.7, 32^3 unchanged.  Letting the next
+// A cycle at 8^3 39.5 -> 37.3 us, 12^3 41.7 -> 40.6, 32^3 170.3 -> 169.5 (exact; graphs
+// of four cycles on both sides).  Letting the next
 // launch in any earlier (griddepcontrol.launch_dependents after the wait, or
 // before the stores) was slower: blocks placed while the launch before them still
 // holds its SMs crowd on few of them (12^3: 103 us, 32^3: 241 against 194).

@@ -106,10 +106,10 @@ struct RzEnergyArgs {
 // Quad meshes of at most this many elements run the lane passes of
 // sgh_rz_lanes.cuh.  Per launch (events, us), one thread per element against four
 // lanes:           16^2         64^2         96^2         128^2        160^2
-//   force exact   16.3 / 10.5  16.4 / 12.3  16.4 / 14.5  16.6 / 20.5  18.8 / 28.8
-//   force FMA     14.5 / 10.3  14.2 / 10.3  14.4 / 12.9  14.5 / 16.5  16.6 / 24.4
-//   elem exact    11.6 /  8.8  12.0 / 10.2  11.9 / 12.3  12.1 / 16.5  15.9 / 22.6
-//   elem FMA      10.2 /  8.3  10.4 /  8.2  10.3 / 10.0  10.2 / 13.8  12.5 / 18.4
+//   force exact   17.3 / 11.9  17.5 / 12.1  17.0 / 14.6  18.1 / 21.0  20.4 / 30.4
+//   force FMA     14.1 / 10.0  14.2 / 10.1  14.2 / 12.3  14.1 / 16.2  16.3 / 25.1
+//   elem exact    10.9 / 10.2  10.8 / 10.3  12.0 / 12.3  12.3 / 16.9  14.3 / 23.4
+//   elem FMA       9.7 /  8.2  10.2 /  8.4  10.2 / 10.7  10.2 / 14.2  11.5 / 18.4
 constexpr long long kRzLanesForce = 11500, kRzLanesElem = 9000;
 constexpr int kRzLaneTile = 8;  // elements per warp of a lane pass
 
