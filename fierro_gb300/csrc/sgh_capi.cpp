@@ -270,9 +270,16 @@ void release_run_graphs(fierro_sgh* h) {
 
 // Captures what `enqueue` puts on the handle's stream as a graph.  It is captured on
 // a stream of the handle's own: work that the caller's other threads, or other handles,
-// put on a shared stream meanwhile must run, not be recorded.
+// put on a shared stream meanwhile must run, not be recorded.  The thread is in relaxed
+// mode for it: making a graph would otherwise end a capture that the caller has open on
+// another stream (fierro_sgh_enqueue_cycles alone does nothing that would).
 template <typename F>
 int capture_graph(fierro_sgh* h, F&& enqueue, cudaGraphExec_t* exec) {
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
   const cudaStream_t stream = h->stream;
   CUDA_TRY(cudaStreamBeginCapture(h->capture, cudaStreamCaptureModeThreadLocal));
   h->stream = h->capture;

@@ -26,8 +26,9 @@ def test_foreign_work_on_the_callers_stream(lib_built):
     want, wt = _run(sgh, p, st, None)
     stream = torch.cuda.Stream()
     count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    count.add_(1)  # the kernel is loaded before the thread starts
     torch.cuda.synchronize()
-    done, added, errors = threading.Event(), [0], []
+    done, added, errors = threading.Event(), [1], []
 
     def foreign():
         try:
@@ -41,7 +42,9 @@ def test_foreign_work_on_the_callers_stream(lib_built):
     t = threading.Thread(target=foreign)
     t.start()
     try:
-        runs = [_run(sgh, p, st, stream.cuda_stream) for _ in range(12)]
+        runs = []
+        while len(runs) < 12 or (added[0] < 1000 and len(runs) < 200 and not errors):
+            runs.append(_run(sgh, p, st, stream.cuda_stream))
     finally:
         done.set()
         t.join()
@@ -53,3 +56,32 @@ def test_foreign_work_on_the_callers_stream(lib_built):
         assert gt == wt
         for k in want:
             assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("before", [0, 20, 30])
+def test_cycles_enqueued_while_the_caller_captures_another_stream(lib_built, before):
+    """Enqueueing makes the larger graphs on the way; the caller's open capture goes on."""
+    import torch
+
+    from fierro_gb300 import problems, sgh
+    p = problems.noh(6, jitter=0.1, seed=2, permute=True, cycles=100)
+    st = sgh.setup(p)
+    with sgh.SGHSolver(p) as s:
+        s.set_state(st)
+        s.run_stages(2 * (before + 40))
+        want, wt = s.get_state(), s.time()
+    stream, x, g = torch.cuda.Stream(), torch.zeros(4, device="cuda"), torch.cuda.CUDAGraph()
+    with sgh.SGHSolver(p) as s:
+        s.set_state(st)
+        s.run(before)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=stream):
+            x.add_(1.0)
+            s.enqueue(40)
+        s.synchronize()
+        got, gt = s.get_state(), s.time()
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 4 and gt == wt
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
